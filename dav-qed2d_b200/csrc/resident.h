@@ -1,0 +1,58 @@
+// resident.h -- host interface of the on-chip mixed CG (resident.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <vector>
+
+#include "internal.h"
+
+namespace qed2d {
+
+// One system of a launch: lattice, place in the field arrays, mass, and how the
+// lattice is split over the blocks of a team (see resident.cu).
+struct ResRep {
+    int L1, L2;
+    long long off;      // first site of the lattice in the batch (0: single lattice)
+    double m2;          // 2 + m0
+    int ntx, nty;       // warp tiles along i1 (<= 32 sites wide) and i2 (<= K sites high)
+    int bx, by;         // blocks of the team along i1 and i2
+    int wx, wy;         // most warp tiles of a block along i1 and i2
+    int id, pad;        // index of the system in the caller's order
+};
+
+// outcome of one system
+struct ResOut {
+    int it, conv, nupd, pad;
+    double rr, bb;
+};
+
+// The split of an L1 x L2 lattice over at most `nb` blocks with the least modelled
+// time per iteration, one cluster where that takes at most max_cluster blocks; K = 0
+// where the state does not fit on chip.
+ResPlan res_plan(int L1, int L2, int nb, int max_cluster);
+ResPlan res_plan_single(int L1, int L2, int nb);
+int res_clusters(const ResPlan& p);
+ResRep res_rep(const ResPlan& p, int L1, int L2, long long off, double m2, int id);
+
+struct ResArgs {
+    const ResRep* reps = nullptr;   // device, nrep > 1
+    ResRep rep0{};                  // nrep == 1
+    int nrep = 1;
+    const double2* U = nullptr;
+    const double2* b = nullptr;
+    double2* x = nullptr;
+    double2* t64 = nullptr;         // g5Dw x
+    double2* r64 = nullptr;         // workspace
+    double mu2 = 0.0, eps = 0.0;
+    int maxiter = 0, guess = 0;
+    ResOut* out = nullptr;          // [nrep]
+    void* slots = nullptr;          // res_slot_bytes(plan, nteams)
+    DevCtl* ctl = nullptr;
+    int single = 0;                 // write the context's record of the solve
+};
+size_t res_slot_bytes(const ResPlan& p, int nteams);
+// one launch: nteams teams of plan.blocks() blocks solve the nrep systems
+int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream);
+
+}  // namespace qed2d

@@ -121,7 +121,12 @@ int qed2d_ctx_get_dims(const qed2d_ctx* ctx, int* L1, int* L2);
  * every block's tiles staged once per solve in shared memory; it agrees with
  * the first form to the solver's accuracy, is a candidate of the first solve's
  * timing, and is refused (QED2D_ERR_UNSUPPORTED) where the staged links do not
- * fit beside co-resident blocks (large lattices). */
+ * fit beside co-resident blocks (large lattices).  Where the whole FP32 state of
+ * the mixed CG fits on chip (up to about 530^2) and no schedule is set, the solve
+ * keeps it there (registers and shared memory; only halos and sums leave an SM)
+ * instead of timing candidates; get then reports 6 (one cluster) or 5 (the grid),
+ * the forms whose recurrences it shares; results agree with theirs to the
+ * solver's accuracy.  Setting a schedule selects the form it names. */
 #define QED2D_MULTISHIFT 3   /* schedule selector of the multishift solver (FP64) */
 int qed2d_ctx_set_schedule(qed2d_ctx* ctx, int precision, int schedule);
 int qed2d_ctx_get_schedule(const qed2d_ctx* ctx, int precision, int* schedule);

@@ -1,0 +1,114 @@
+"""The on-chip mixed CG (the mixed solver's default wherever its FP32 state fits in
+registers and shared memory) against the oracle, at the sizes where its split into
+warp tiles, blocks and clusters changes: lattices smaller than a tile, partial
+tiles in both directions, one block, one cluster, a grid of blocks up to the
+largest that fits.
+
+Solutions: the stop rule leaves a relative residual of 1e-12 on both sides and the
+masses are those of the other mixed-solver tests, so the same 5e-12 holds; the
+recurrences and reliable updates are those of the solver's other forms, so iteration
+counts agree with theirs within 2 plus 1% (not with the FP64 oracle's: on the smallest
+lattices an FP64 CG ends exactly after as many steps as there are unknowns)."""
+import numpy as np
+import pytest
+
+from helpers import bound, cgauss, hot_links, rel, to_dev, to_host
+from oracle.oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(2, 2), (3, 5), (31, 2), (33, 7), (32, 32), (64, 64), (65, 31), (100, 37), (128, 128), (40, 250), (257, 66),
+         (256, 256), (330, 97), (512, 512), (544, 400)]
+
+
+@pytest.fixture
+def q():
+    import qed2d
+    qed2d.set_precision("mixed")
+    yield qed2d
+    qed2d.set_precision("f64")
+
+
+def solve(q, prm, U, b, am0, mu=0.0, maxiter=20000, eps=1e-24, x=None):
+    x = q.cfield(*prm.iL) if x is None else x
+    q.set_schedule(prm, -1, "mixed")
+    if mu:
+        it = q.CG(x, U, b, am0, mu, maxiter, eps, q.gamm5Dw_sqr_musq, prm, None, so_as_guess=bool(x.any()))
+    else:
+        it = q.CG(x, U, b, am0, maxiter, eps, q.gamm5Dw_sqr_msq, prm, None)
+    return it, x
+
+
+@pytest.mark.parametrize("L1,L2", SIZES)
+def test_solution_vs_oracle(q, L1, L2):
+    prm = q.LattParm((L1, L2), 4.0)
+    U, b = hot_links(L1, L2, 61), cgauss(L1, L2, 62, 2)
+    am0 = 0.25
+    st, xo, _, _ = Oracle(L1, L2, 4.0).cg(U, b, am0, 20000, 1e-24)
+    assert st == 0
+    Ud, bd = to_dev(U), to_dev(b)
+    q.set_schedule(prm, 1, "mixed")
+    ito = q.CG(q.cfield(L1, L2), Ud, bd, am0, 20000, 1e-24, q.gamm5Dw_sqr_msq, prm, None)
+    it, x = solve(q, prm, Ud, bd, am0)
+    assert q.get_schedule(prm, "mixed") in (5, 6)
+    bound("on-chip mixed CG vs oracle", rel(to_host(x), xo), 5e-12)
+    assert abs(it - ito) <= 2 + ito // 100, (it, ito)
+    _, x2 = solve(q, prm, Ud, bd, am0)   # deterministic
+    assert np.array_equal(to_host(x2), to_host(x))
+
+
+@pytest.mark.parametrize("L1,L2", [(33, 7), (64, 48), (256, 192)])
+def test_shift_guess_cap_and_zero(q, L1, L2):
+    """Method 2 with a shift and with a warm start; a capped solve returns the same
+    iterate as the solver's first form (FP32 rounding of a few iterations: 1e-6, as
+    for the other forms) and reports non-convergence; a zero source gives zero."""
+    prm = q.LattParm((L1, L2), 4.0)
+    U, b = hot_links(L1, L2, 71), cgauss(L1, L2, 72, 2)
+    am0, mu = 0.2, 0.3
+    o = Oracle(L1, L2, 4.0)
+    st, xo, _, _ = o.cg(U, b, am0, 20000, 1e-24, mu=mu)
+    assert st == 0
+    Ud, bd = to_dev(U), to_dev(b)
+    it, x = solve(q, prm, Ud, bd, am0, mu)
+    bound("on-chip mixed CG (shift) vs oracle", rel(to_host(x), xo), 5e-12)
+    guess = x + 1e-3 * to_dev(cgauss(L1, L2, 73, 2))
+    it2, xg = solve(q, prm, Ud, bd, am0, mu, x=guess)
+    assert 0 < it2 <= it
+    # (a warm start stops elsewhere within the stop rule's ball than the oracle's cold start)
+    q.set_schedule(prm, 1, "mixed")
+    x1 = x + 1e-3 * to_dev(cgauss(L1, L2, 73, 2))
+    q.CG(x1, Ud, bd, am0, mu, 20000, 1e-24, q.gamm5Dw_sqr_musq, prm, None, so_as_guess=True)
+    bound("on-chip mixed CG (warm start) vs first form", rel(to_host(xg), to_host(x1)), 5e-12)
+    it3, xs = solve(q, prm, Ud, bd, am0, mu, x=xg.clone())   # already solved
+    assert it3 == 0 and np.array_equal(to_host(xs), to_host(xg))
+    for cap in (1, 7, 8):
+        out = []
+        for sched in (-1, 1):
+            q.set_schedule(prm, sched, "mixed")
+            xc = q.cfield(L1, L2)
+            with pytest.raises(q.Qed2dError):
+                q.CG(xc, Ud, bd, am0, cap, 1e-24, q.gamm5Dw_sqr_msq, prm, None)
+            assert q.last_solve(prm)[0] == cap
+            out.append(to_host(xc))
+        bound("on-chip capped solve vs first form", rel(out[0], out[1]), 1e-6)
+    with pytest.raises(q.Qed2dError):   # no iteration allowed
+        solve(q, prm, Ud, bd, am0, maxiter=0)
+    it, x = solve(q, prm, Ud, to_dev(np.zeros_like(b)), am0)
+    assert it == 0 and not to_host(x).any()
+
+
+def test_non_unitary_links_and_nan_source(q):
+    """Links of any modulus are taken as they are; a NaN source ends unconverged."""
+    L1, L2 = 48, 36
+    prm = q.LattParm((L1, L2), 4.0)
+    U = hot_links(L1, L2, 81) * (1.0 + 0.05 * np.random.default_rng(3).standard_normal((2, L2, L1)))
+    b = cgauss(L1, L2, 82, 2)
+    st, xo, _, _ = Oracle(L1, L2, 4.0).cg(U, b, 0.4, 20000, 1e-24)
+    assert st == 0
+    _, x = solve(q, prm, to_dev(U), to_dev(b), 0.4)
+    bound("on-chip mixed CG (non-unitary links) vs oracle", rel(to_host(x), xo), 5e-12)
+    b[0, 3, 5] = np.nan
+    with pytest.raises(q.Qed2dError):
+        solve(q, prm, to_dev(U), to_dev(b), 0.4, maxiter=30)
+    b[0, 3, 5] = 1.0
+    solve(q, prm, to_dev(U), to_dev(b), 0.4)   # the context stays usable
