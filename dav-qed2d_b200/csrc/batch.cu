@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "graph.h"
+#include "resident.h"
 #include "stencil.cuh"
 
 namespace qed2d {
@@ -764,6 +765,25 @@ __global__ void k_r_finish(const RepState* __restrict__ st, int nrep, int maxite
     if (threadIdx.x == 0 && bad) ctl->status = QED2D_ERR_NOT_CONVERGED;
 }
 
+// the same from the on-chip solver's records
+__global__ void k_r_finish_res(const ResOut* __restrict__ out, int nrep, int* __restrict__ it_out,
+                               int* __restrict__ upd_out, long long* __restrict__ acc, DevCtl* ctl) {
+    if (ctl->status != 0) return;
+    int bad = 0;
+    for (int r = threadIdx.x; r < nrep; r += blockDim.x) {
+        const ResOut s = out[r];
+        it_out[r] = s.it;
+        upd_out[r] = s.nupd;
+        acc[r] += s.it;
+        bad |= !s.conv;
+    }
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) {
+        ctl->last_iters = out[0].it;
+        if (bad) ctl->status = QED2D_ERR_NOT_CONVERGED;
+    }
+}
+
 }  // namespace qed2d
 
 #include "batch_cg_uniform.cuh"
@@ -924,6 +944,21 @@ struct qed2d_batch {
         ws[name] = {p, bytes};
         return p;
     }
+    // The on-chip solver (resident.cu): one class of replicas per size, each a launch.
+    struct ResClass {
+        ResPlan plan;
+        int n, nteams;
+        const ResRep* d_reps;
+        void* slots;
+        cudaStream_t side;   // null: the batch's stream
+        cudaEvent_t done;
+    };
+    std::vector<ResClass> res;
+    int res_fits = -1;              // -1: not planned yet, 0: some replica does not fit on chip
+    bool res_on = false;            // the schedule was chosen by the library and stands for the on-chip form
+    ResOut* d_resout = nullptr;     // [nrep]
+    cudaEvent_t res_fork = nullptr;
+
     double2* field(const char* n) { return (double2*)buf(n, sizeof(double2) * 2 * Vtot); }
     double* real2(const char* n) { return (double*)buf(n, sizeof(double) * 2 * Vtot); }
     float4* field32(const char* n) { return (float4*)buf(n, sizeof(float4) * Vtot); }
@@ -1171,8 +1206,126 @@ int tune_ragged(qed2d_batch* h, const RCGP& P, const CCGP& C, int maxiter, Launc
     return QED2D_OK;
 }
 
+template <class T>
+int upload(T** d, const std::vector<T>& v);
+
+// Plans the on-chip solver: replicas of one size are a class with a split of its
+// own.  Classes run side by side, the one with the most work on the batch's stream
+// and each other on its own: clusters stream through the SMs that the others leave.  Teams
+// larger than a cluster wait for one another over the whole GPU, so their classes
+// share the batch's stream, where two such launches never overlap.
+int res_plan_classes(qed2d_batch* h) {
+    h->res_fits = 0;
+    std::map<std::pair<int, int>, std::vector<int>> by;
+    for (int r = 0; r < h->nrep; r++) by[{h->reps[r].L1, h->reps[r].L2}].push_back(r);
+    std::vector<std::pair<int, int>> sizes;
+    std::vector<int> n;
+    for (const auto& kv : by) {
+        sizes.push_back(kv.first);
+        n.push_back((int)kv.second.size());
+    }
+    const std::vector<ResPlan> plans = res_plan_batch(sizes, n, h->num_sms);
+    if (plans.empty()) return QED2D_OK;
+    std::vector<ResRep> reps;
+    for (size_t i = 0; i < sizes.size(); i++) {
+        qed2d_batch::ResClass c{};
+        c.plan = plans[i];
+        c.n = n[i];
+        c.nteams = c.plan.cl ? c.n : std::min(c.n, h->num_sms / c.plan.blocks());
+        for (int r : by[sizes[i]])
+            reps.push_back(res_rep(c.plan, sizes[i].first, sizes[i].second, h->reps[r].off, 0.0, r));
+        h->res.push_back(c);
+    }
+    ResRep* d = (ResRep*)h->buf("res_reps", sizeof(ResRep) * reps.size());
+    h->d_resout = (ResOut*)h->buf("res_out", sizeof(ResOut) * h->nrep);
+    if (!d || !h->d_resout) return QED2D_ERR_NO_MEMORY;
+    QCHECK(cudaMemcpyAsync(d, reps.data(), sizeof(ResRep) * reps.size(), cudaMemcpyHostToDevice, h->stream));
+    QCHECK(cudaStreamSynchronize(h->stream));
+    size_t at = 0;
+    for (size_t i = 0; i < h->res.size(); i++) {
+        auto& c = h->res[i];
+        c.d_reps = d + at;
+        at += c.n;
+        c.slots = h->buf("res_slots_" + std::to_string(i), res_slot_bytes(c.plan, c.nteams));
+        if (!c.slots) return QED2D_ERR_NO_MEMORY;
+    }
+    // grid teams first, then the longest
+    std::stable_sort(h->res.begin(), h->res.end(), [](const qed2d_batch::ResClass& a, const qed2d_batch::ResClass& b) {
+        if (a.plan.cl != b.plan.cl) return a.plan.cl < b.plan.cl;
+        return a.plan.cost * a.plan.blocks() * a.n > b.plan.cost * b.plan.blocks() * b.n;
+    });
+    const bool grid = !h->res[0].plan.cl;
+    if (h->res.size() > 1) QCHECK(cudaEventCreateWithFlags(&h->res_fork, cudaEventDisableTiming));
+    constexpr size_t kSides = 8;   // streams beside the batch's; further classes follow on them
+    std::vector<cudaStream_t> sides;
+    size_t k = 0;
+    for (size_t i = 0; i < h->res.size(); i++) {
+        auto& c = h->res[i];
+        if (!c.plan.cl || (i == 0 && !grid)) continue;
+        if (sides.size() < kSides) {
+            cudaStream_t s = nullptr;
+            QCHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            sides.push_back(s);
+            c.side = s;
+        } else {
+            c.side = sides[k++ % kSides];
+        }
+        QCHECK(cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming));
+    }
+    h->res_fits = 1;
+    return QED2D_OK;
+}
+
+int res_solve_batch(qed2d_batch* h, const double2* U, const double2* b, double2* x, double2* g5x, int maxiter, double eps) {
+    double2* r64 = h->field("b_r64");
+    if (!r64) return QED2D_ERR_NO_MEMORY;
+    QCHECK(cudaMemsetAsync(&h->ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), h->stream));
+    if (h->res_fork) QCHECK(cudaEventRecord(h->res_fork, h->stream));
+    int st = QED2D_OK;
+    for (auto& c : h->res) {
+        ResArgs a;
+        a.reps = c.d_reps;
+        a.nrep = c.n;
+        a.m2 = h->d_m2;
+        a.U = U;
+        a.b = b;
+        a.x = x;
+        a.t64 = g5x;
+        a.r64 = r64;
+        a.eps = eps;
+        a.maxiter = maxiter;
+        a.out = h->d_resout;
+        a.slots = c.slots;
+        a.ctl = h->ctl;
+        a.reset = false;
+        if (c.side) QCHECK(cudaStreamWaitEvent(c.side, h->res_fork, 0));
+        const int l = res_launch(a, c.plan, c.nteams, c.side ? c.side : h->stream);
+        if (c.side) QCHECK(cudaEventRecord(c.done, c.side));
+        if (st == QED2D_OK) st = l;
+    }
+    for (auto& c : h->res)
+        if (c.side) QCHECK(cudaStreamWaitEvent(h->stream, c.done, 0));
+    if (st != QED2D_OK) return st;
+    k_r_finish_res<<<1, 256, 0, h->stream>>>(h->d_resout, h->nrep, h->d_out, h->d_out + h->nrep, h->d_iters, h->ctl);
+    return r_post("k_r_finish_res");
+}
+
 int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* b, double2* x, double2* g5x,
             int maxiter, double eps) {
+    // No schedule and no tile height set: on chip wherever every replica fits there.
+    if (h->uniform ? (!h->usched_fixed && !h->utile_fixed && (h->usched < 0 || h->utile < 0)) : h->rsched < 0) {
+        if (h->res_fits < 0) QTRY(res_plan_classes(h));
+        if (h->res_fits) {
+            h->res_on = true;
+            if (h->uniform) {
+                h->usched = 9;
+                h->utile = 0;
+            } else {
+                h->rsched = 6;
+            }
+        }
+    }
+    if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
     RCGP P{};
     P.nrep = h->nrep;
     P.reps = h->d_reps;
@@ -1564,6 +1717,13 @@ int qed2d_batch_destroy(qed2d_batch* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     else cudaDeviceSynchronize();
     h->md_graph.release();
+    std::vector<cudaStream_t> sides;
+    for (auto& c : h->res) {
+        if (c.side && std::find(sides.begin(), sides.end(), c.side) == sides.end()) sides.push_back(c.side);
+        if (c.done) cudaEventDestroy(c.done);
+    }
+    for (cudaStream_t s : sides) cudaStreamDestroy(s);
+    if (h->res_fork) cudaEventDestroy(h->res_fork);
     for (auto& kv : h->ws) cudaFree(kv.second.first);
     void* dev[] = {h->d_reps,  h->d_tiles, h->d_seg0,  h->d_segs,  h->d_order, h->d_rep_seg, h->d_dbase_c,
                    h->d_dbase_r, h->d_m2,  h->d_beta,  h->d_seed,  h->d_st,    h->d_flags,   h->d_red,
@@ -1609,6 +1769,7 @@ int qed2d_batch_set_schedule(qed2d_batch* h, int schedule) {
             "qed2d_batch_set_schedule: -1, or 0/1/4/5/7/8/9 (equal sizes, at most 64 replicas), or 2/3/6 (otherwise)");
         return QED2D_ERR_BAD_ARG;
     }
+    h->res_on = false;   // a schedule set by the caller is the form it names
     if (h->uniform) {
         h->usched = schedule;
         h->usched_fixed = schedule >= 0;
@@ -1630,12 +1791,15 @@ int qed2d_batch_set_tile_rows(qed2d_batch* h, int rows) {
         return QED2D_ERR_BAD_ARG;
     }
     if (rows == -1) {
+        h->res_on = false;
         h->utile_fixed = false;
         h->utile = -1;
         return QED2D_OK;
     }
     for (int t = 0; t < h->nuv; t++)
         if (h->uv[t].rows == rows) {
+            if (h->res_on) h->usched = -1;   // tiles are the other forms': tune the schedule at this height
+            h->res_on = false;
             h->utile = t;
             h->utile_fixed = true;
             return QED2D_OK;
@@ -1722,7 +1886,7 @@ int qed2d_batch_hmc_nf2(qed2d_batch* h, double* Ud, const double* am0, double ep
     // graph from the third trajectory with the same arguments on (graph.h)
     GraphKey k;
     k.p(U).p(mom).p(X).p(F).p(G).p(U32).d(eps).i(ns).i(maxiter).d(tol);
-    k.i(h->usched).i(h->utile).i(h->rsched).i(h->rcs).i((long long)h->ws_gen);
+    k.i(h->res_on).i(h->usched).i(h->utile).i(h->rsched).i(h->rcs).i((long long)h->ws_gen);
     for (int r = 0; r < B; r++) k.d(h->m2[r]);
     QTRY(run_graphed(h->md_graph, h->stream, k.s, [&]() -> int {
         QTRY(r_pack(h, U, mom, 0.0, U32));

@@ -56,6 +56,7 @@ typedef unsigned long long u64;
 struct ResP {
     const ResRep* reps;
     ResRep rep0;              // the system when there is only one
+    const double* m2;         // 2 + m0 by system index (null: in the ResRep)
     int nrep, nteams, nb;     // systems, teams, blocks per team
     const double2* U;
     const double2* b;
@@ -905,7 +906,10 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_mixed(const __g
     unsigned seq = 0;
     ulonglong2 base0 = make_ulonglong2(0, 0), base1 = base0;
     for (int next = team; next < P.nrep;) {
-        if (threadIdx.x == 0) B.rep = P.nrep == 1 ? P.rep0 : P.reps[next];
+        if (threadIdx.x == 0) {
+            B.rep = P.reps ? P.reps[next] : P.rep0;
+            if (P.m2) B.rep.m2 = P.m2[B.rep.id];
+        }
         __syncthreads();
         if (threadIdx.x < 32) seq = res_scalar<CL>(P, B, seq, base0, base1);
         else seq = res_worker<K, CL>(P, B, dyn, seq);
@@ -932,18 +936,22 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_mixed(const __g
 // host side
 static int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// The split with the least modelled time per iteration.  An exchange ends when both
-// of its chains have: the workers' (send, stencil, faces; grows with the rows that
-// a scheduler's warps walk) and the sums' (block, team, recurrences, back), and the
-// vector update follows.  The constants are cycles measured on a B200 at 1.92 GHz
-// with one team on the GPU: modelled / measured per iteration 64^2 1.76 / 1.89 us,
-// 128^2 2.2 / 2.6, 256^2 4.0 / 4.3, 512^2 4.3 / 5.2.  Clusters of up to 16 blocks
-// exchange over distributed shared memory, which takes a third of the time through
-// L2, so a small lattice stays in one; beyond, the lattice spreads over as many SMs
-// as there are.
-ResPlan res_plan(int L1, int L2, int nb, int max_cluster) {
-    ResPlan best;
-    best.K = 0;
+// Modelled time of an iteration, us.  An exchange ends when both of its chains have:
+// the workers' (send, stencil, faces; grows with the rows that a scheduler's warps
+// walk, `share` blocks on an SM) and the sums' (block, team, recurrences, back), and
+// the vector update follows.  The constants are cycles measured on a B200 at 1.92
+// GHz: modelled / measured per iteration 64^2 1.76 / 1.89 us, 128^2 2.2 / 2.6, 256^2
+// 3.9 / 4.3, 512^2 4.3 / 5.2.
+static double res_cost(int K, int warps, int blocks, bool cl, int share) {
+    const double rows = (double)ceil_div(warps * share, 4) * K;
+    const double workers = 600 + 150 * rows;
+    const double sums = blocks == 1 ? 900 : cl ? 1250 + 15 * blocks : 2300 + 9 * blocks;
+    return 2 * (std::max(workers, sums) + 150 + 25 * rows) / 1920;
+}
+
+std::vector<ResPlan> res_plans(int L1, int L2, int nb, int max_cluster) {
+    std::vector<ResPlan> best(nb + 1);
+    for (ResPlan& p : best) p.K = 0;
     for (int K : {1, 2, 4}) {
         const int ntx = ceil_div(L1, 32), nty = ceil_div(L2, K);
         if (L2 / nty < K - 1) continue;   // tiles have K or K - 1 rows
@@ -952,13 +960,14 @@ ResPlan res_plan(int L1, int L2, int nb, int max_cluster) {
                 const int wx = ceil_div(ntx, bx), wy = ceil_div(nty, by), n = bx * by;
                 if (wx * wy > kResWarps) continue;
                 const bool cl = n <= max_cluster;
-                const double rows = (double)ceil_div(wx * wy, 4) * K;
-                const double workers = 600 + 150 * rows, sums = n == 1 ? 900 : cl ? 1250 + 15 * n : 3600;
-                const double cost = 2 * (std::max(workers, sums) + 150 + 25 * rows) / 1920;
-                if (!best.K || cost < best.cost) best = ResPlan{K, cl ? 1 : 0, bx, by, wx, wy, ntx, nty, cost};
+                const double cost = res_cost(K, wx * wy, n, cl, 1);
+                if (!best[n].K || cost < best[n].cost) best[n] = ResPlan{K, cl ? 1 : 0, bx, by, wx, wy, ntx, nty, cost};
             }
     }
-    return best;
+    std::vector<ResPlan> out;
+    for (const ResPlan& p : best)
+        if (p.K) out.push_back(p);
+    return out;
 }
 
 ResRep res_rep(const ResPlan& p, int L1, int L2, long long off, double m2, int id) {
@@ -1004,13 +1013,69 @@ int res_clusters(const ResPlan& p) {
     return p.K == 1 ? res_clusters_k<1>(p) : p.K == 2 ? res_clusters_k<2>(p) : res_clusters_k<4>(p);
 }
 
-// the plan of a single lattice: clusters of more than 8 blocks only where the device takes them
+// A single lattice: the split with the least time.  Clusters of up to 16 blocks
+// exchange over distributed shared memory, which takes a third of the time through
+// L2, so a small lattice stays in one; beyond, the lattice spreads over as many SMs
+// as there are.  Clusters of more than 8 blocks only where the device takes them.
 ResPlan res_plan_single(int L1, int L2, int nb) {
-    for (int mc : {kResCluster, 8}) {
-        const ResPlan p = res_plan(L1, L2, nb, mc);
-        if (p.K == 0 || !p.cl || res_clusters(p) > 0) return p;
+    for (int mc : {kResCluster, 8, 0}) {
+        ResPlan best;
+        best.K = 0;
+        for (const ResPlan& p : res_plans(L1, L2, nb, mc))
+            if (!best.K || p.cost < best.cost) best = p;
+        if (best.K == 0 || !best.cl || res_clusters(best) > 0) return best;
     }
-    return res_plan(L1, L2, nb, 0);
+    return ResPlan{};
+}
+
+// Modelled time per iteration of n equal lattices under plan p: rounds of as many
+// teams as run at a time.
+static double res_time(const ResPlan& p, int n, int num_sms) {
+    const int at = p.cl ? res_clusters(p) : num_sms / p.blocks();
+    if (at < 1) return 1e30;
+    const int m = std::min(n, at), share = ceil_div(m * p.blocks(), num_sms);
+    return ceil_div(n, at) * res_cost(p.K, p.wx * p.wy, p.blocks(), p.cl, share);
+}
+
+// A batch of lattices: sizes (L1, L2), counts n.  One size: the split with the least
+// time for all of them.  Several: the one that occupies the least SM time per
+// lattice, unless a single lattice then takes longer than the whole batch needs with
+// every SM busy; such a size gets the least SM time among the splits that do not, or
+// the fastest split.  Empty where a size does not fit.
+std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& sizes, const std::vector<int>& n, int num_sms) {
+    std::vector<ResPlan> out;
+    std::vector<std::vector<ResPlan>> cand;
+    for (const auto& sz : sizes) {
+        cand.push_back({});
+        for (const ResPlan& p : res_plans(sz.first, sz.second, num_sms, kResCluster))
+            if (!p.cl || res_clusters(p) > 0) cand.back().push_back(p);
+        if (cand.back().empty()) return {};
+    }
+    if (sizes.size() == 1) {
+        double tb = 1e30;
+        out.resize(1);
+        for (const ResPlan& p : cand[0]) {
+            const double t = res_time(p, n[0], num_sms);
+            if (t < tb) tb = t, out[0] = p;
+        }
+        return out;
+    }
+    double total = 0;
+    for (size_t i = 0; i < sizes.size(); i++) {
+        double sm = 1e30;
+        for (const ResPlan& p : cand[i]) sm = std::min(sm, p.cost * p.blocks());
+        total += n[i] * sm / num_sms;
+    }
+    for (size_t i = 0; i < sizes.size(); i++) {
+        ResPlan best, fast;
+        best.K = fast.K = 0;
+        for (const ResPlan& p : cand[i]) {
+            if (!fast.K || p.cost < fast.cost) fast = p;
+            if (p.cost <= total && (!best.K || p.cost * p.blocks() < best.cost * best.blocks())) best = p;
+        }
+        out.push_back(best.K ? best : fast);
+    }
+    return out;
 }
 
 template <int K, bool CL>
@@ -1069,10 +1134,11 @@ int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t s
     P.slots = P.psum + (size_t)nteams * 2 * P.nb * P.nb;
     P.acc = (u64*)(P.slots + (size_t)nteams * P.nb * 2 * P.nslots);
     P.queue = (int*)(P.acc + (size_t)nteams * 32);
+    P.m2 = a.m2;
     P.out = a.out;
     P.ctl = a.ctl;
     P.single = a.single;
-    QCHECK(cudaMemsetAsync(&a.ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), stream));
+    if (a.reset) QCHECK(cudaMemsetAsync(&a.ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), stream));
     if (!plan.cl) QCHECK(cudaMemsetAsync(a.slots, 0, res_slot_bytes(plan, nteams), stream));
     switch (plan.K * 2 + plan.cl) {
         case 2: return res_launch_k<1, false>(P, plan, stream);

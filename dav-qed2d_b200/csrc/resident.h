@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -27,17 +28,15 @@ struct ResOut {
     double rr, bb;
 };
 
-// The split of an L1 x L2 lattice over at most `nb` blocks with the least modelled
-// time per iteration, one cluster where that takes at most max_cluster blocks; K = 0
-// where the state does not fit on chip.
-ResPlan res_plan(int L1, int L2, int nb, int max_cluster);
-ResPlan res_plan_single(int L1, int L2, int nb);
+ResPlan res_plan_single(int L1, int L2, int nb);   // K = 0 where the state does not fit on chip
+std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& sizes, const std::vector<int>& n, int num_sms);
 int res_clusters(const ResPlan& p);
 ResRep res_rep(const ResPlan& p, int L1, int L2, long long off, double m2, int id);
 
 struct ResArgs {
-    const ResRep* reps = nullptr;   // device, nrep > 1
-    ResRep rep0{};                  // nrep == 1
+    const ResRep* reps = nullptr;   // device; null: rep0 alone
+    ResRep rep0{};
+    const double* m2 = nullptr;     // device, by system index: masses in the place of the ResReps'
     int nrep = 1;
     const double2* U = nullptr;
     const double2* b = nullptr;
@@ -49,6 +48,7 @@ struct ResArgs {
     ResOut* out = nullptr;          // [nrep]
     void* slots = nullptr;          // res_slot_bytes(plan, nteams)
     DevCtl* ctl = nullptr;
+    bool reset = true;              // clear the control block's error flag first
     int single = 0;                 // write the context's record of the solve
 };
 size_t res_slot_bytes(const ResPlan& p, int nteams);

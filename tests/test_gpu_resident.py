@@ -112,3 +112,59 @@ def test_non_unitary_links_and_nan_source(q):
         solve(q, prm, to_dev(U), to_dev(b), 0.4, maxiter=30)
     b[0, 3, 5] = 1.0
     solve(q, prm, to_dev(U), to_dev(b), 0.4)   # the context stays usable
+
+
+def batch_solve(b, U, src, am0, sched):
+    b.schedule = sched
+    x = b.field()
+    its, upd = b.cg(x, U, src, am0, 20000, 1e-24)
+    return list(its), list(upd), to_host(x)
+
+
+@pytest.mark.parametrize("nrep,L1,L2", [(2, 33, 7), (37, 64, 64), (20, 96, 128), (5, 256, 256), (3, 500, 300)])
+def test_equal_batch_vs_lean_schedule(nrep, L1, L2):
+    """Equal-size batches on chip: one cluster per replica, more clusters than fit at a
+    time, teams of the whole GPU that take the replicas in turn.  Against schedule 5,
+    the same recurrences in the other solver: as schedules 8 and 9 are (1e-11)."""
+    import qed2d
+    b = qed2d.Batch(nrep, L1, L2, 4.0)
+    U, src = b.field(), b.field()
+    for r in range(nrep):
+        U[r] = to_dev(hot_links(L1, L2, 500 + r))
+        src[r] = to_dev(cgauss(L1, L2, 600 + r, 2))
+    src[nrep - 1].zero_()   # one replica with a zero source
+    am0 = [0.2 + 0.1 * (r % 3) for r in range(nrep)]
+    it, upd, x = batch_solve(b, U, src, am0, -1)
+    assert b.schedule == 9 and b.tile_rows in (4, 8, 16)
+    it2, _, x2 = batch_solve(b, U, src, am0, -1)
+    assert it2 == it and np.array_equal(x, x2)   # deterministic
+    it5, _, x5 = batch_solve(b, U, src, am0, 5)
+    assert it[nrep - 1] == 0 and not x[nrep - 1].any()
+    bound("on-chip equal batch vs schedule 5", rel(x, x5), 1e-11)
+    assert all(abs(p - q) <= 2 + q // 100 for p, q in zip(it, it5)), (it, it5)
+
+
+@pytest.mark.parametrize("big", [False, True])
+def test_uneven_batch_vs_grid_solver(big):
+    """Uneven batches on chip: more size classes than side streams, odd sizes, several
+    replicas of a size; with and without sizes whose teams exceed a cluster."""
+    import qed2d
+    sizes = [(32, 32), (48, 48), (64, 64), (33, 20), (100, 37), (17, 90), (128, 128), (2, 3), (64, 48), (31, 31), (96, 96)]
+    sizes = sizes * 2 + ([(256, 256), (300, 200), (256, 256)] if big else [])
+    b = qed2d.Batch.ragged(sizes, [4.0] * len(sizes))
+    U, src = b.field(), b.field()
+    for r, (l1, l2) in enumerate(sizes):
+        b.replica(U, r).copy_(to_dev(hot_links(l1, l2, 700 + r)))
+        b.replica(src, r).copy_(to_dev(cgauss(l1, l2, 800 + r, 2)))
+    am0 = [0.2 + 0.05 * (r % 5) for r in range(len(sizes))]
+    it, upd, x = batch_solve(b, U, src, am0, -1)
+    assert b.schedule == 6
+    assert np.array_equal(batch_solve(b, U, src, am0, -1)[2], x)
+    it2, _, x2 = batch_solve(b, U, src, am0, 2)
+    bound("on-chip uneven batch vs grid solver", rel(x, x2), 1e-11)
+    tiny = [l1 * l2 < 100 for l1, l2 in sizes]   # fewer unknowns than steps: the count is rounding
+    assert all(t or abs(p - q) <= 2 + q // 100 for p, q, t in zip(it, it2, tiny)), (it, it2)
+    with pytest.raises(qed2d.Qed2dError):   # capped
+        b.schedule = -1
+        b.cg(b.field(), U, src, am0, 5, 1e-24)
+    assert np.array_equal(batch_solve(b, U, src, am0, -1)[2], x)
