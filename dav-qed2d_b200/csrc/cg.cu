@@ -1259,25 +1259,27 @@ static int tune_cg(Ctx& c, const CGP& P, int slot) {
     return QED2D_OK;
 }
 
-// The mixed solve with its whole FP32 state on chip (resident.cu): the library's
-// choice wherever the state fits (up to about 530^2 on 148 SMs), a rule on the size
-// without timing.  Per iteration against the fastest of the other forms, B200: 64^2
-// 4.85 -> 1.89 us, 128^2 5.95 -> 2.63, 256^2 7.1 -> 4.3, 512^2 12.3 -> 5.2.
-static int cg_resident(Ctx& c, const SolveArgs& a) {
-    const ResPlan& p = c.res_plan;
+// The solve with its whole state on chip (resident.cuh): the library's choice
+// wherever the state fits (mixed: up to about 530^2 on 148 SMs, FP64: 370^2), a rule
+// on the size without timing.  Per iteration against the fastest of the other forms,
+// B200: mixed 64^2 4.85 -> 1.89 us, 128^2 5.95 -> 2.63, 256^2 7.1 -> 4.3, 512^2 12.3 ->
+// 5.2; FP64 64^2 5.87 -> 2.23, 128^2 6.47 -> 4.0, 256^2 8.3 -> 5.4, 352^2 10.6 -> 5.4.
+static int cg_resident(Ctx& c, const SolveArgs& a, int slot) {
+    const ResPlan& p = c.res_plan[slot];
     ResArgs r;
     r.rep0 = res_rep(p, c.g.L1, c.g.L2, 0, 2.0 + a.am0, 0);
     r.U = a.U;
     r.b = a.b;
     r.x = a.x;
     r.t64 = a.g5x ? a.g5x : c.spinor("cg_t");
+    r.want_g5 = a.g5x ? 1 : 0;
     r.r64 = c.spinor("cg_r");
     r.mu2 = a.mu2;
     r.eps = a.eps;
     r.maxiter = a.maxiter;
     r.guess = a.guess ? 1 : 0;
     r.out = (ResOut*)c.buf("res_out", sizeof(ResOut));
-    r.slots = c.buf("res_slots", res_slot_bytes(p, 1));
+    r.slots = c.buf(slot ? "res_slots" : "res_slots64", res_slot_bytes(p, 1));
     r.ctl = c.ctl;
     r.single = 1;
     if (!r.t64 || !r.r64 || !r.out || !r.slots) return QED2D_ERR_NO_MEMORY;
@@ -1286,6 +1288,16 @@ static int cg_resident(Ctx& c, const SolveArgs& a) {
 
 int cg_solve(Ctx& c, const SolveArgs& a, int precision) {
     if (precision == QED2D_PREC_PLAIN) return solve_plain(c, a);
+    const int slot = precision == QED2D_PREC_F64 ? 0 : 1;
+    if (c.sched[slot] < 0) {   // the choice is the library's: on chip wherever the state fits there
+        ResPlan& p = c.res_plan[slot];
+        if (p.K < 0) p = res_plan_single(c.g.L1, c.g.L2, c.num_sms, slot == 0);
+        if (p.K > 0) {
+            c.res_on[slot] = true;
+            c.sched[slot] = (p.cl ? 2 : 1) + (slot ? 4 : 0);
+        }
+    }
+    if (c.res_on[slot]) return cg_resident(c, a, slot);
     CGP P{};
     P.g = c.g;
     P.U = a.U;
@@ -1309,14 +1321,6 @@ int cg_solve(Ctx& c, const SolveArgs& a, int precision) {
         if (c.sched[0] == 2 && !cluster_possible(c, 0)) c.sched[0] = 1;
         return launch_cg(c, P, 0, c.sched[0]);
     }
-    if (c.sched[1] < 0) {   // the choice is the library's: on chip wherever the state fits there
-        if (c.res_plan.K < 0) c.res_plan = res_plan_single(c.g.L1, c.g.L2, c.num_sms);
-        if (c.res_plan.K > 0) {
-            c.res_on = true;
-            c.sched[1] = c.res_plan.cl ? 6 : 5;
-        }
-    }
-    if (c.res_on) return cg_resident(c, a);
     P.r32 = c.spinor32("cg_r32");
     P.q0 = c.spinor32("cg_q0");
     P.q1 = c.spinor32("cg_q1");

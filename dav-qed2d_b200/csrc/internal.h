@@ -66,6 +66,7 @@ struct GraphCache {
 struct ResPlan {
     int K = -1;         // sites of a thread's column
     int cl = 0;         // a team is one thread-block cluster (exchange over distributed shared memory)
+    int f64 = 0;        // FP64 vectors
     int bx = 0, by = 0, wx = 0, wy = 0, ntx = 0, nty = 0;
     double cost = 0;    // modelled time of one iteration, us
     int blocks() const { return bx * by; }
@@ -87,8 +88,8 @@ struct Ctx {
     double last_relres = 0.0;
     int sched[3] = {-1, -1, -1};   // reduction schedule of the F64 / MIXED / multishift solvers (-1: not tuned yet)
     int ms_layout = -1;            // layout of the multishift kernel (kMsLayouts; -1: tuned with the schedule)
-    ResPlan res_plan;              // split of the on-chip mixed solver (K < 0: not planned, 0: does not fit)
-    bool res_on = false;           // sched[1] was chosen by the library and stands for the on-chip form
+    ResPlan res_plan[2];           // split of the on-chip F64 / MIXED solver (K < 0: not planned, 0: does not fit)
+    bool res_on[2] = {false, false};   // sched[i] was chosen by the library and stands for the on-chip form
     GraphCache md_graph;           // MD integration of the HMC trajectories (graph.h)
     uint64_t ws_gen = 0;           // bumped whenever a workspace buffer is reallocated
 

@@ -1,4 +1,4 @@
-// resident.h -- host interface of the on-chip mixed CG (resident.cu).
+// resident.h -- host interface of the on-chip CG (resident.cu, resident_f64.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -28,7 +28,8 @@ struct ResOut {
     double rr, bb;
 };
 
-ResPlan res_plan_single(int L1, int L2, int nb);   // K = 0 where the state does not fit on chip
+// K = 0 where the state does not fit on chip
+ResPlan res_plan_single(int L1, int L2, int nb, bool f64);
 std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& sizes, const std::vector<int>& n, int num_sms);
 int res_clusters(const ResPlan& p);
 ResRep res_rep(const ResPlan& p, int L1, int L2, long long off, double m2, int id);
@@ -45,6 +46,7 @@ struct ResArgs {
     double2* r64 = nullptr;         // workspace
     double mu2 = 0.0, eps = 0.0;
     int maxiter = 0, guess = 0;
+    int want_g5 = 0;                // FP64: t64 = g5Dw x is wanted (the mixed solver always leaves it)
     ResOut* out = nullptr;          // [nrep]
     void* slots = nullptr;          // res_slot_bytes(plan, nteams)
     DevCtl* ctl = nullptr;

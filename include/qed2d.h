@@ -122,11 +122,11 @@ int qed2d_ctx_get_dims(const qed2d_ctx* ctx, int* L1, int* L2);
  * the first form to the solver's accuracy, is a candidate of the first solve's
  * timing, and is refused (QED2D_ERR_UNSUPPORTED) where the staged links do not
  * fit beside co-resident blocks (large lattices).  Where the whole FP32 state of
- * the mixed CG fits on chip (up to about 530^2) and no schedule is set, the solve
- * keeps it there (registers and shared memory; only halos and sums leave an SM)
- * instead of timing candidates; get then reports 6 (one cluster) or 5 (the grid),
- * the forms whose recurrences it shares; results agree with theirs to the
- * solver's accuracy.  Setting a schedule selects the form it names. */
+ * the mixed CG (up to about 530^2) or the FP64 state of the F64 CG (370^2) fits on
+ * chip and no schedule is set, the solve keeps it there (registers and shared
+ * memory; only halos and sums leave an SM) instead of timing candidates; get then
+ * reports 6 / 2 (one cluster) or 5 / 1 (the grid); results agree with those forms to
+ * the solver's accuracy.  Setting a schedule selects the form it names. */
 #define QED2D_MULTISHIFT 3   /* schedule selector of the multishift solver (FP64) */
 int qed2d_ctx_set_schedule(qed2d_ctx* ctx, int precision, int schedule);
 int qed2d_ctx_get_schedule(const qed2d_ctx* ctx, int precision, int* schedule);

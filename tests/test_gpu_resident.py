@@ -1,5 +1,5 @@
-"""The on-chip mixed CG (the mixed solver's default wherever its FP32 state fits in
-registers and shared memory) against the oracle, at the sizes where its split into
+"""The on-chip CG (the default of the mixed and the FP64 solver wherever the state
+fits in registers and shared memory) against the oracle, at the sizes where its split into
 warp tiles, blocks and clusters changes: lattices smaller than a tile, partial
 tiles in both directions, one block, one cluster, a grid of blocks up to the
 largest that fits.
@@ -18,20 +18,24 @@ from oracle.oracle import Oracle
 pytestmark = pytest.mark.gpu
 
 SIZES = [(2, 2), (3, 5), (31, 2), (33, 7), (32, 32), (64, 64), (65, 31), (100, 37), (128, 128), (40, 250), (257, 66),
-         (256, 256), (330, 97), (512, 512), (544, 400)]
+         (256, 256), (330, 97), (350, 370), (512, 512), (544, 400)]
 
 
-@pytest.fixture
-def q():
+F64_SITES = 148 * 15 * 64   # what FP64 holds; beyond, the solver's other forms run
+
+
+@pytest.fixture(params=["mixed", "f64"])
+def q(request):
     import qed2d
-    qed2d.set_precision("mixed")
+    qed2d.set_precision(request.param)
+    qed2d.prec = request.param
     yield qed2d
     qed2d.set_precision("f64")
 
 
 def solve(q, prm, U, b, am0, mu=0.0, maxiter=20000, eps=1e-24, x=None):
     x = q.cfield(*prm.iL) if x is None else x
-    q.set_schedule(prm, -1, "mixed")
+    q.set_schedule(prm, -1, q.prec)
     if mu:
         it = q.CG(x, U, b, am0, mu, maxiter, eps, q.gamm5Dw_sqr_musq, prm, None, so_as_guess=bool(x.any()))
     else:
@@ -41,17 +45,19 @@ def solve(q, prm, U, b, am0, mu=0.0, maxiter=20000, eps=1e-24, x=None):
 
 @pytest.mark.parametrize("L1,L2", SIZES)
 def test_solution_vs_oracle(q, L1, L2):
+    if q.prec == "f64" and L1 * L2 > F64_SITES:
+        pytest.skip("not on chip in FP64")
     prm = q.LattParm((L1, L2), 4.0)
     U, b = hot_links(L1, L2, 61), cgauss(L1, L2, 62, 2)
     am0 = 0.25
     st, xo, _, _ = Oracle(L1, L2, 4.0).cg(U, b, am0, 20000, 1e-24)
     assert st == 0
     Ud, bd = to_dev(U), to_dev(b)
-    q.set_schedule(prm, 1, "mixed")
+    q.set_schedule(prm, 1, q.prec)
     ito = q.CG(q.cfield(L1, L2), Ud, bd, am0, 20000, 1e-24, q.gamm5Dw_sqr_msq, prm, None)
     it, x = solve(q, prm, Ud, bd, am0)
-    assert q.get_schedule(prm, "mixed") in (5, 6)
-    bound("on-chip mixed CG vs oracle", rel(to_host(x), xo), 5e-12)
+    assert q.get_schedule(prm, q.prec) in ((5, 6) if q.prec == "mixed" else (1, 2))
+    bound("on-chip CG vs oracle", rel(to_host(x), xo), 5e-12)
     assert abs(it - ito) <= 2 + ito // 100, (it, ito)
     _, x2 = solve(q, prm, Ud, bd, am0)   # deterministic
     assert np.array_equal(to_host(x2), to_host(x))
@@ -70,21 +76,21 @@ def test_shift_guess_cap_and_zero(q, L1, L2):
     assert st == 0
     Ud, bd = to_dev(U), to_dev(b)
     it, x = solve(q, prm, Ud, bd, am0, mu)
-    bound("on-chip mixed CG (shift) vs oracle", rel(to_host(x), xo), 5e-12)
+    bound("on-chip CG (shift) vs oracle", rel(to_host(x), xo), 5e-12)
     guess = x + 1e-3 * to_dev(cgauss(L1, L2, 73, 2))
     it2, xg = solve(q, prm, Ud, bd, am0, mu, x=guess)
     assert 0 < it2 <= it
     # (a warm start stops elsewhere within the stop rule's ball than the oracle's cold start)
-    q.set_schedule(prm, 1, "mixed")
+    q.set_schedule(prm, 1, q.prec)
     x1 = x + 1e-3 * to_dev(cgauss(L1, L2, 73, 2))
     q.CG(x1, Ud, bd, am0, mu, 20000, 1e-24, q.gamm5Dw_sqr_musq, prm, None, so_as_guess=True)
-    bound("on-chip mixed CG (warm start) vs first form", rel(to_host(xg), to_host(x1)), 5e-12)
+    bound("on-chip CG (warm start) vs first form", rel(to_host(xg), to_host(x1)), 5e-12)
     it3, xs = solve(q, prm, Ud, bd, am0, mu, x=xg.clone())   # already solved
     assert it3 == 0 and np.array_equal(to_host(xs), to_host(xg))
     for cap in (1, 7, 8):
         out = []
         for sched in (-1, 1):
-            q.set_schedule(prm, sched, "mixed")
+            q.set_schedule(prm, sched, q.prec)
             xc = q.cfield(L1, L2)
             with pytest.raises(q.Qed2dError):
                 q.CG(xc, Ud, bd, am0, cap, 1e-24, q.gamm5Dw_sqr_msq, prm, None)
@@ -106,7 +112,7 @@ def test_non_unitary_links_and_nan_source(q):
     st, xo, _, _ = Oracle(L1, L2, 4.0).cg(U, b, 0.4, 20000, 1e-24)
     assert st == 0
     _, x = solve(q, prm, to_dev(U), to_dev(b), 0.4)
-    bound("on-chip mixed CG (non-unitary links) vs oracle", rel(to_host(x), xo), 5e-12)
+    bound("on-chip CG (non-unitary links) vs oracle", rel(to_host(x), xo), 5e-12)
     b[0, 3, 5] = np.nan
     with pytest.raises(q.Qed2dError):
         solve(q, prm, to_dev(U), to_dev(b), 0.4, maxiter=30)
