@@ -1493,9 +1493,56 @@ static int multishift32_solve(Ctx& c, const double2* U, const double2* b, double
     return QED2D_OK;
 }
 
+// The multishift solve with all its vectors on chip (resident_f64.cu): the library's
+// choice where they fit (about 190^2 with 12 shifts on 148 SMs).
+static int multishift_resident(Ctx& c, const ResPlan& p, const double2* U, const double2* b, double2* const* x,
+                               const double* mu2, int n, double am0, int maxiter, double eps) {
+    ResShifts s{};
+    s.n = n;
+    for (int i = 1; i < n; i++)
+        if (mu2[i] < mu2[s.base]) s.base = i;
+    for (int i = 0; i < n; i++) {
+        s.d[i] = mu2[i] - mu2[s.base];
+        s.x[i] = x[i];
+    }
+    ResArgs r;
+    r.rep0 = res_rep(p, c.g.L1, c.g.L2, 0, 2.0 + am0, 0);
+    r.U = U;
+    r.b = b;
+    r.x = x[s.base];
+    r.t64 = c.spinor("cg_t");
+    r.r64 = r.t64;   // no warm start here
+    r.mu2 = mu2[s.base];
+    r.eps = eps;
+    r.maxiter = maxiter;
+    r.out = (ResOut*)c.buf("res_out", sizeof(ResOut));
+    r.slots = c.buf("res_slots_ms", res_slot_bytes(p, 1));
+    r.ctl = c.ctl;
+    r.single = 1;
+    if (!r.t64 || !r.out || !r.slots) return QED2D_ERR_NO_MEMORY;
+    return res_launch_ms(r, p, s, c.stream);
+}
+
 int multishift_solve(Ctx& c, const double2* U, const double2* b, double2* const* x, const double* mu2, int n,
                      double am0, int maxiter, double eps) {
     if (n < 1 || n > kMaxShifts) return QED2D_ERR_BAD_ARG;
+    if ((c.sched[2] < 0 && c.ms_layout < 0 && c.g.V < kMs32Sites) || c.res_on[2]) {
+        auto it = c.res_ms.find(n);
+        if (it == c.res_ms.end()) {
+            ResPlan p;
+            QTRY(res_plan_ms(c.g.L1, c.g.L2, c.num_sms, n, c.device, &p));
+            it = c.res_ms.emplace(n, p).first;
+        }
+        if (it->second.K > 0) {
+            c.res_on[2] = true;
+            c.sched[2] = 1;
+            return multishift_resident(c, it->second, U, b, x, mu2, n, am0, maxiter, eps);
+        }
+        if (c.res_on[2]) {   // more shifts than fit: the choice is the tuner's after all
+            c.res_on[2] = false;
+            c.sched[2] = -1;
+        }
+    }
     if (c.sched[2] == 3) return multishift32_solve(c, U, b, x, mu2, n, am0, maxiter, eps);
     MSP P{};
     P.g = c.g;

@@ -9,6 +9,9 @@ namespace qed2d {
 // resident_f64.cu
 int res_f64_clusters(const ResPlan& p);
 int res_f64_launch(const ResP& P, const ResPlan& plan, cudaStream_t stream);
+int res_ms_limit(int device, size_t* limit);
+bool res_ms_fits(const ResPlan& p, int n, size_t limit);
+int res_ms_launch(const ResP& P, const ResPlan& plan, const ResMs& m, cudaStream_t stream);
 
 static int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
@@ -73,6 +76,27 @@ ResPlan res_plan_single(int L1, int L2, int nb, bool f64) {
     return ResPlan{};
 }
 
+// A multishift solve with n shifts: the split over a grid of blocks with the least
+// time, where the shifts' vectors fit and their updates (about 36 cycles a row and
+// shift, all in shared memory) hide behind the iteration or bound it.
+int res_plan_ms(int L1, int L2, int nb, int n, int device, ResPlan* best) {
+    size_t limit = 0;
+    QTRY(res_ms_limit(device, &limit));
+    best->K = 0;
+    for (int K : {1, 2}) {
+        const int ntx = ceil_div(L1, 32), nty = ceil_div(L2, K);
+        for (int bx = 1; bx <= std::min(ntx, nb); bx++)
+            for (int by = 1; by <= std::min(nty, nb / bx); by++) {
+                ResPlan p{K, 0, 1, bx, by, ceil_div(ntx, bx), ceil_div(nty, by), ntx, nty, 0.0};
+                if (p.wx * p.wy > kResWarps || !res_ms_fits(p, n, limit)) continue;
+                const double shifts = 36.0 * p.wx * p.wy * K * (n - 1) / 1920;
+                p.cost = std::max(res_cost(K, p.wx * p.wy, bx * by, false, 1, true), shifts);
+                if (!best->K || p.cost < best->cost) *best = p;
+            }
+    }
+    return QED2D_OK;
+}
+
 // Modelled time per iteration of n equal lattices under plan p: rounds of as many
 // teams as run at a time.
 static double res_time(const ResPlan& p, int n, int num_sms) {
@@ -129,8 +153,8 @@ size_t res_slot_bytes(const ResPlan& p, int nteams) {
     return sizeof(ulonglong2) * nteams * (nb * 2 * (nslots + nb) + 16) + 16;
 }
 
-int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream) {
-    ResP P{};
+// the kernel's parameters; clears the slots
+static int res_fill(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream, ResP& P) {
     P.reps = a.reps;
     P.rep0 = a.rep0;
     P.nrep = a.nrep;
@@ -158,6 +182,12 @@ int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t s
     P.single = a.single;
     if (a.reset) QCHECK(cudaMemsetAsync(&a.ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), stream));
     if (!plan.cl) QCHECK(cudaMemsetAsync(a.slots, 0, res_slot_bytes(plan, nteams), stream));
+    return QED2D_OK;
+}
+
+int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream) {
+    ResP P{};
+    QTRY(res_fill(a, plan, nteams, stream, P));
     if (plan.f64) return res_f64_launch(P, plan, stream);
     switch (plan.K * 2 + plan.cl) {
         case 2: return res_launch_k<float, 1, false>(P, plan, stream);
@@ -167,6 +197,19 @@ int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t s
         case 8: return res_launch_k<float, 4, false>(P, plan, stream);
         default: return res_launch_k<float, 4, true>(P, plan, stream);
     }
+}
+
+int res_launch_ms(const ResArgs& a, const ResPlan& plan, const ResShifts& s, cudaStream_t stream) {
+    ResP P{};
+    QTRY(res_fill(a, plan, 1, stream, P));
+    ResMs M{};
+    M.n = s.n;
+    M.base = s.base;
+    for (int i = 0; i < s.n; i++) {
+        M.d[i] = s.d[i];
+        M.x[i] = s.x[i];
+    }
+    return res_ms_launch(P, plan, M, stream);
 }
 
 }  // namespace qed2d

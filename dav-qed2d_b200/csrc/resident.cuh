@@ -499,8 +499,23 @@ __device__ __forceinline__ V4<R> axpy4(R a, const V4<R>& x, const V4<R>& y) {
 }
 
 // ---------------------------------------------------------------------------
+// Multishift solves (MS): the base system as above, and every other shift's x and p
+// in shared memory, updated by warps of their own behind the base system.
+constexpr int kResShifts = QED2D_MAXPOLES;
+struct ResMs {
+    int n, base, nw;             // shifts, the base system's, worker warps of a block
+    double d[kResShifts];        // mu_i^2 - mu_base^2
+    double2* x[kResShifts];
+};
+struct ResMsBlock {              // the shifts' scalars of an iteration
+    double a[kResShifts], b[kResShifts], z[kResShifts];
+    int state[kResShifts];       // 1: x_i += a p_i, 2: p_i = z r + b p_i as well
+    int flag[2];                 // how the round ended, two rounds in turn
+};
+
 // what the threads of a block share
 struct ResBlock {
+    int nwk;                       // worker threads
     double part[32 * kResWarps];   // the threads' partials of an exchange
     ResSc sc;
     int abort;                 // a wait of this block gave up
@@ -514,11 +529,14 @@ struct ResBlock {
 // The scalar warp (warp 0: the scheduler prefers the oldest of its warps, and this
 // one is on the way of all): one step per exchange, in step with the workers.  Returns the
 // exchange it ended at.
-template <bool MIXED, bool CL>
+template <bool MIXED, bool CL, bool MS = false>
 __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsigned seq, ulonglong2& base0,
-                                               ulonglong2& base1) {
+                                               ulonglong2& base1, const ResMs* M = nullptr, ResMsBlock* S = nullptr) {
     enum { X_BEGIN, X_GUESS, X_RR, X_PAP, X_FENCE, X_TRUE };   // what the coming exchange sums
-    const int nth = blockDim.x, nw = (nth >> 5) - 1, lane = threadIdx.x & 31;
+    const int nw = MS ? M->nw : (int)(blockDim.x >> 5) - 1, nth = 32 * (nw + 1), lane = threadIdx.x & 31;
+    double zs = 1.0, zp = 1.0, a_last = 1.0, b_last = 0.0, a_now = 0.0;   // MS: lane i's shift; the recurrences' scalars
+    bool act = MS && lane < M->n && lane != M->base;
+    int round = 0;   // MS: barriers with the shift warps so far
     double rr = 0.0, inv_rr = 0.0, maxrr = 0.0, s = 1.0, beta = 0.0, rr64 = 0.0, bb = 0.0, tol = 0.0;
     double rr_last = 1.0, pap_last = 4.0;   // the last |r|^2 and <p, A p>: the fixed-point scales
     double thr = 0.0;                       // |r|^2 below it: reliable update
@@ -554,9 +572,12 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
             }
             if (!exact && next != X_FENCE && ok) ok = team_sum_slots(B.C, seq, v, tot);
         }
-        double c = 0.0;
+        double c = 0.0, rr_old = rr;
+        const bool all = MS && (next == X_BEGIN || next == X_RR);   // the shift warps join this barrier
+        const bool step = MS && next == X_RR && !fresh;             // and an iteration is behind them
         if (next == X_PAP) {   // <p, (A + mu2) p>
             c = rr / tot;   // alpha
+            if (MS) a_now = c;
             pap_last = tot;
             k++;
             next = X_RR;
@@ -624,7 +645,35 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
             B.sc.flag = flag;
             B.sc.s = s;
         }
-        bar_sync_n(3, nth);
+        if (all) bar_sync_n(5, blockDim.x);
+        else bar_sync_n(3, nth);
+        if constexpr (MS) {
+            const bool give_up = !all && flag == RF_ABORT && next == X_RR;   // in <p, A p>: the shift warps wait for |r|^2
+            if (step) {   // the shifts' recurrences (k_cg_multishift's), lane i shift i
+                const double b_new = tot / rr_old;
+                if (act) {
+                    const double zn = zs * zp * a_last / (a_now * b_last * (zp - zs) + zp * a_last * (1.0 + M->d[lane] * a_now));
+                    const double q = zn / zs;
+                    S->a[lane] = a_now * q;
+                    S->b[lane] = b_new * q * q;
+                    S->z[lane] = zn;
+                    zp = zs;
+                    zs = zn;
+                    act = !(zn * zn * tot < tol);
+                    S->state[lane] = act ? 2 : 1;
+                } else {
+                    S->state[lane] = 0;
+                }
+                a_last = a_now;
+                b_last = b_new;
+            }
+            if (give_up) bar_arrive_n(5, blockDim.x);
+            if (all || give_up) {
+                if (lane == 0) S->flag[round & 1] = flag;
+                round++;
+                bar_arrive_n(4, blockDim.x - 32 * nw);
+            }
+        }
         if (flag >= RF_STOP) break;
         // off the way from one exchange to the next
         inv_rr = 1.0 / rr;
@@ -673,14 +722,15 @@ __device__ __forceinline__ Site col_site(const Column& c, int L1, int L2, int j)
 // workers: the thread's partial of exchange seq
 __device__ __forceinline__ void put_part(ResBlock& B, double s) {
     B.part[threadIdx.x - 32] = s;
-    bar_arrive_n(1, blockDim.x);
+    bar_arrive_n(1, B.nwk + 32);
 }
 // Workers: the end of an exchange.  A warp whose wait for a face gave up (!ok)
 // leaves a note that the scalar warp finds at the next exchange and turns into
 // RF_ABORT for the whole block, so that all its threads leave at the same barrier.
-__device__ __forceinline__ int wait_scalar(ResBlock& B, bool ok) {
+__device__ __forceinline__ int wait_scalar(ResBlock& B, bool ok, bool all = false) {
     if (!ok) *(volatile int*)&B.abort = 1;
-    bar_sync_n(3, blockDim.x);
+    if (all) bar_sync_n(5, blockDim.x);   // MS: with the shift warps
+    else bar_sync_n(3, B.nwk + 32);
     return *(volatile int*)&B.sc.flag;
 }
 
@@ -692,7 +742,7 @@ __device__ __forceinline__ int wait_scalar(ResBlock& B, bool ok) {
 template <bool MIXED>
 __device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x32, unsigned& seq, bool add) {
     const Column c = column_of(B);
-    const int nwk = blockDim.x - 32, L1 = B.rep.L1, L2 = B.rep.L2;
+    const int nwk = B.nwk, L1 = B.rep.L1, L2 = B.rep.L2;
     const long long V = (long long)L1 * L2, o2 = 2 * B.rep.off;
     const double m2 = B.rep.m2, mu2 = P.mu2;
     double2* xs = P.x + o2;
@@ -754,10 +804,10 @@ __device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x3
 
 // Workers: |b|^2 and (mixed) the first FP32 residual, left in x32.  x = 0 without a
 // guess where the solve adds to it or has nothing to do.
-template <bool MIXED>
+template <bool MIXED, bool MS = false>
 __device__ __forceinline__ int res_begin(const ResP& P, ResBlock& B, float4* x32, unsigned& seq) {
     const Column c = column_of(B);
-    const int nwk = blockDim.x - 32, L1 = B.rep.L1;
+    const int nwk = B.nwk, L1 = B.rep.L1;
     const long long V = (long long)L1 * B.rep.L2, o2 = 2 * B.rep.off;
     double acc = 0.0;
 #pragma unroll 1
@@ -767,7 +817,7 @@ __device__ __forceinline__ int res_begin(const ResP& P, ResBlock& B, float4* x32
     }
     put_part(B, acc);
     ++seq;
-    const int flag = wait_scalar(B, true);
+    const int flag = wait_scalar(B, true, MS);
     if (flag == RF_ABORT || flag == RF_UPD) return flag;
     const double2 z = make_double2(0, 0);
     const double s = B.sc.s;
@@ -793,7 +843,7 @@ __device__ __forceinline__ int res_begin(const ResP& P, ResBlock& B, float4* x32
 // Workers, FP64: x (+)= the solve's, and g5Dw x, which reads other blocks' x.
 __device__ __forceinline__ void res_finish(const ResP& P, ResBlock& B, const double4x* xs, unsigned& seq) {
     const Column c = column_of(B);
-    const int nwk = blockDim.x - 32, L1 = B.rep.L1, L2 = B.rep.L2;
+    const int nwk = B.nwk, L1 = B.rep.L1, L2 = B.rep.L2;
     const long long V = (long long)L1 * L2, o2 = 2 * B.rep.off;
     double2* x = P.x + o2;
 #pragma unroll 1
@@ -860,10 +910,11 @@ __device__ __forceinline__ void res_place(ResBlock& B) {
     }
 }
 
-template <class R, int K, bool CL>
-__device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char* dyn, unsigned seq) {
+template <class R, int K, bool CL, bool MS = false>
+__device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char* dyn, unsigned seq,
+                                               V4<R>* rbuf = nullptr) {   // MS: r for the shift warps, two copies in turn
     constexpr bool MIXED = std::is_same<R, float>::value;
-    const int nwk = blockDim.x - 32, lane = threadIdx.x & 31;
+    const int nwk = B.nwk, lane = threadIdx.x & 31;
     V4<R>* xs = reinterpret_cast<V4<R>*>(dyn) + (threadIdx.x - 32);   // x: row j at xs[j * nwk]
     V4<R>* ps = xs + K * nwk;                                         // the search direction likewise
     V4<R>* ts = ps + K * nwk;                                         // mixed: t during an update
@@ -892,7 +943,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
         xs[j * nwk] = ps[j * nwk] = zero;
         if (MIXED) ts[j * nwk] = zero;
     }
-    int flag = res_begin<MIXED>(P, B, reinterpret_cast<float4*>(xs), seq);
+    int flag = res_begin<MIXED, MS>(P, B, reinterpret_cast<float4*>(xs), seq);
     bool first = true;
     V2<R> u1[K], u2[K];
     V4<R> r[K], t[K], w[K];
@@ -944,7 +995,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
 #pragma unroll
                 for (int j = 0; j < K; j++) xs[j * nwk] = axpy4<R>(alpha, ps[j * nwk], xs[j * nwk]);
             });
-            flag = wait_scalar(B, ok);
+            flag = wait_scalar(B, ok, MS);
             if (flag != RF_GO) break;
             const R beta = MIXED ? (R)B.sc.cf : (R)B.sc.c;
             {
@@ -975,12 +1026,16 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
 #pragma unroll
                     for (int j = 0; j < K; j++) ps[j * nwk] = axpy4<R>(beta, ps[j * nwk], r[j]);
             });
-            if (wait_scalar(B, ok) == RF_ABORT) return seq;
+            if (wait_scalar(B, ok) == RF_ABORT) {
+                if (MS) bar_arrive_n(5, blockDim.x);   // the shift warps wait there
+                return seq;
+            }
             alpha = MIXED ? (R)B.sc.cf : (R)B.sc.c;
 #pragma unroll
             for (int j = 0; j < K; j++) {
                 if (mu2 != R(0)) w[j] = axpy4<R>(mu2, ps[j * nwk], w[j]);
                 r[j] = axpy4<R>(-alpha, w[j], r[j]);
+                if constexpr (MS) rbuf[(((seq >> 1) & 1) * K + j) * nwk + threadIdx.x - 32] = r[j];
             }
         }
         alpha = 0;
@@ -1001,6 +1056,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_cg(const __grid
     const int team = blockIdx.x / P.nb;
     if (threadIdx.x == 0) {
         B.abort = 0;
+        B.nwk = blockDim.x - 32;
         B.C.nb = P.nb;
         B.C.rank = blockIdx.x - team * P.nb;
         B.C.nslots = P.nslots;

@@ -53,6 +53,14 @@ struct ResArgs {
     bool reset = true;              // clear the control block's error flag first
     int single = 0;                 // write the context's record of the solve
 };
+// the multishift solve: every shift's solution (the base system's is a.x)
+struct ResShifts {
+    int n, base;
+    double d[QED2D_MAXPOLES];       // mu_i^2 - mu_base^2
+    double2* x[QED2D_MAXPOLES];
+};
+int res_plan_ms(int L1, int L2, int nb, int n, int device, ResPlan* best);   // K = 0 where it does not fit
+int res_launch_ms(const ResArgs& a, const ResPlan& plan, const ResShifts& s, cudaStream_t stream);
 size_t res_slot_bytes(const ResPlan& p, int nteams);
 // one launch: nteams teams of plan.blocks() blocks solve the nrep systems
 int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream);

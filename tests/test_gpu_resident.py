@@ -174,3 +174,41 @@ def test_uneven_batch_vs_grid_solver(big):
         b.schedule = -1
         b.cg(b.field(), U, src, am0, 5, 1e-24)
     assert np.array_equal(batch_solve(b, U, src, am0, -1)[2], x)
+
+
+@pytest.mark.parametrize("L1,L2,n", [(12, 12, 2), (33, 7, 5), (64, 64, 12), (100, 37, 7), (128, 128, 12), (40, 90, 32),
+                                     (180, 200, 12)])
+def test_multishift_vs_grid_solver(L1, L2, n):
+    """The on-chip multishift solve (the default where its vectors fit) against the grid
+    kernel's schedule 1, the same recurrences: the layouts and schedules of that kernel
+    are held to 1e-13 of one another, iteration counts to 1.  The smallest shift is not
+    the first."""
+    import qed2d
+    prm = qed2d.LattParm((L1, L2), 4.0)
+    U, src = to_dev(hot_links(L1, L2, 91)), to_dev(cgauss(L1, L2, 92, 2))
+    mus = [0.05 * 1.3 ** i for i in range(n)]
+    mus = mus[1:] + mus[:1] if n > 2 else mus
+    out = []
+    try:
+        for sched in (-1, -1, 1):
+            qed2d.set_schedule(prm, sched, "multishift")
+            xs = [qed2d.cfield(L1, L2) for _ in mus]
+            it = qed2d.multishift_CG(xs, U, src, 0.2, mus, 20000, 1e-24, prm)
+            out.append((it, np.stack([to_host(x) for x in xs])))
+        assert np.array_equal(out[0][1], out[1][1])   # deterministic
+        assert abs(out[0][0] - out[2][0]) <= 1
+        for i in range(n):
+            bound("on-chip multishift vs grid kernel", rel(out[0][1][i], out[2][1][i]), 1e-13)
+        qed2d.set_schedule(prm, -1, "multishift")
+        xs = [to_dev(cgauss(L1, L2, 93 + i, 2)) for i in range(n)]   # capped: not converged; zero source: zero
+        with pytest.raises(qed2d.Qed2dError):
+            qed2d.multishift_CG(xs, U, src, 0.2, mus, 3, 1e-24, prm)
+        assert qed2d.multishift_CG(xs, U, torch_zeros_like(src), 0.2, mus, 20000, 1e-24, prm) == 0
+        assert not any(bool(x.any()) for x in xs)
+    finally:
+        qed2d.set_schedule(prm, -1, "multishift")
+
+
+def torch_zeros_like(t):
+    import torch
+    return torch.zeros_like(t)
