@@ -13,6 +13,7 @@
 
 #include "graph.h"
 #include "internal.h"
+#include "resident.h"
 
 struct qed2d_ctx {
     qed2d::Ctx c;
@@ -312,6 +313,14 @@ static int md_omf4_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MD
     const double r5 = 0.5 - R1 - R3, r6 = 1.0 - 2.0 * (R2 + R4);
     const double cm[6] = {R1, R3, r5, r5, R3, R1};
     const double cu[5] = {R2, R4, r6, R4, R2};
+    if (ns > 0 && !s.U32 && res_gauge_fits(c)) {
+        ResMd md{cm[0] * eps, {}, {}, cm[5] * eps, 5, ns, 1};
+        for (int k = 0; k < 5; k++) {
+            md.u[k] = eps * cu[k];
+            md.c[k] = cm[k + 1] * eps;
+        }
+        return res_gauge_md(c, mom, U, md);
+    }
     GaugePingPong pp(c, U, mom, s);
     for (int i = 0; i < ns; i++) {
         QTRY(pp.kick(cm[0] * eps));
@@ -321,6 +330,8 @@ static int md_omf4_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MD
 }
 
 static int md_leapfrog_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MDState& s) {
+    if (ns > 0 && !s.U32 && res_gauge_fits(c))
+        return res_gauge_md(c, mom, U, ResMd{0.5 * eps, {eps}, {eps}, 0.5 * eps, 1, ns, 0});
     GaugePingPong pp(c, U, mom, s);
     QTRY(pp.kick(0.5 * eps));
     for (int i = 0; i < ns - 1; i++) QTRY(pp.links_then_kick(eps, eps, s));

@@ -871,10 +871,10 @@ __device__ __forceinline__ void res_finish(const ResP& P, ResBlock& B, const dou
 
 // Lane 0 of a worker warp: the warp's tile and where its faces go.
 template <class R, int K, bool CL>
-__device__ __forceinline__ void res_place(ResBlock& B) {
+__device__ __forceinline__ void res_place(ResBlock& B, int warp) {
     constexpr int N = Num<R>::SLOTS;
     const ResRep& L = B.rep;
-    const int warp = (threadIdx.x >> 5) - 1, rank = B.C.rank, nslots = B.C.nslots;
+    const int rank = B.C.rank, nslots = B.C.nslots;
     const int bi = rank % L.bx, bj = rank / L.bx;
     const int c0 = bi * L.ntx / L.bx, c1 = (bi + 1) * L.ntx / L.bx;
     const int r0 = bj * L.nty / L.by, r1 = (bj + 1) * L.nty / L.by;
@@ -919,7 +919,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
     V4<R>* ps = xs + K * nwk;                                         // the search direction likewise
     V4<R>* ts = ps + K * nwk;                                         // mixed: t during an update
     V2<R>* box = reinterpret_cast<V2<R>*>(dyn + (size_t)nwk * ResSm<R, K>::ARRAYS * K * sizeof(V4<R>));
-    if (lane == 0) res_place<R, K, CL>(B);
+    if (lane == 0) res_place<R, K, CL>(B, (threadIdx.x >> 5) - 1);
     __syncwarp();
     Tile T;
     {

@@ -61,6 +61,15 @@ struct ResShifts {
 };
 int res_plan_ms(int L1, int L2, int nb, int n, int device, ResPlan* best);   // K = 0 where it does not fit
 int res_launch_ms(const ResArgs& a, const ResPlan& plan, const ResShifts& s, cudaStream_t stream);
+// Pure-gauge molecular dynamics on chip (resident_gauge.cu): kick first; ns times
+// { m times: links by u[k], then kick c[k]; kick first again, if each and not the last
+// step }, the very last kick `last`.
+struct ResMd {
+    double first, u[5], c[5], last;
+    int m, ns, each;
+};
+bool res_gauge_fits(Ctx& c);
+int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s);
 size_t res_slot_bytes(const ResPlan& p, int nteams);
 // one launch: nteams teams of plan.blocks() blocks solve the nrep systems
 int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream);

@@ -212,3 +212,35 @@ def test_multishift_vs_grid_solver(L1, L2, n):
 def torch_zeros_like(t):
     import torch
     return torch.zeros_like(t)
+
+
+@pytest.mark.parametrize("L1,L2", [(2, 2), (3, 5), (33, 7), (32, 32), (64, 64), (100, 37), (128, 128), (350, 370), (512, 512),
+                                   (544, 400)])
+def test_gauge_md_vs_separate_kernels(L1, L2):
+    """Pure-gauge OMF4 integration on chip (the default where links and momenta fit)
+    against the same kicks and link updates made one by one with the library's
+    kernels: the same operations, contracted differently by the compiler, so links and
+    momenta agree to rounding over the 22 updates (1e-13)."""
+    import torch
+    import qed2d
+    beta, eps, ns = 5.0, 0.2, 2
+    prm = qed2d.LattParm((L1, L2), beta)
+    U = to_dev(hot_links(L1, L2, 31))
+    mom = torch.from_numpy(np.random.default_rng(5).standard_normal((2, L2, L1))).cuda()
+    U1, m1 = U.clone(), mom.clone()
+    qed2d.OMF4_(m1, U1, eps, ns, prm, None)
+    r1, r2, r3, r4 = 0.08398315262876693, 0.2539785108410595, 0.6822365335719091, -0.03230286765269967
+    r5, r6 = 0.5 - r1 - r3, 1.0 - 2.0 * (r2 + r4)
+    f1, f2 = torch.empty_like(mom), torch.empty_like(mom)
+    for _ in range(ns):
+        for k, c in enumerate((r1, r3, r5, r5, r3, r1)):
+            qed2d.krnl_force_(f1, f2, U, prm)
+            mom += c * eps * (f1 + f2)
+            if k < 5:
+                qed2d.updt_fld_(U, mom, eps * (r2, r4, r6, r4, r2)[k])
+    bound("on-chip gauge MD links vs separate kernels", rel(to_host(U1), to_host(U)), 1e-13)
+    bound("on-chip gauge MD momenta vs separate kernels", rel(to_host(m1), to_host(mom)), 1e-13)
+    U2 = to_dev(hot_links(L1, L2, 31))   # deterministic
+    m2 = torch.from_numpy(np.random.default_rng(5).standard_normal((2, L2, L1))).cuda()
+    qed2d.OMF4_(m2, U2, eps, ns, prm, None)
+    assert torch.equal(U1, U2) and torch.equal(m1, m2)
