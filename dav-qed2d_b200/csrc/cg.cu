@@ -1262,8 +1262,9 @@ static int tune_cg(Ctx& c, const CGP& P, int slot) {
 // The solve with its whole state on chip (resident.cuh): the library's choice
 // wherever the state fits (mixed: up to about 530^2 on 148 SMs, FP64: 370^2), a rule
 // on the size without timing.  Per iteration against the fastest of the other forms,
-// B200: mixed 64^2 4.85 -> 1.89 us, 128^2 5.95 -> 2.63, 256^2 7.1 -> 4.3, 512^2 12.3 ->
-// 5.2; FP64 64^2 5.87 -> 2.23, 128^2 6.47 -> 4.0, 256^2 8.3 -> 5.4, 352^2 10.6 -> 5.4.
+// B200: mixed 64^2 4.85 -> 1.95 us, 128^2 5.95 -> 2.7, 256^2 7.1 -> 3.5, 512^2 12.3 ->
+// 4.3; FP64 64^2 5.13 -> 2.2, 128^2 6.4 -> 3.0, 256^2
+// 8.05 -> 4.2, 350x370 11.1 -> 6.6.
 static int cg_resident(Ctx& c, const SolveArgs& a, int slot) {
     const ResPlan& p = c.res_plan[slot];
     ResArgs r;

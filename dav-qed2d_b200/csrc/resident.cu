@@ -15,17 +15,15 @@ int res_ms_launch(const ResP& P, const ResPlan& plan, const ResMs& m, cudaStream
 
 static int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Modelled time of an iteration, us.  An exchange ends when both of its chains have:
-// the workers' (send, stencil, faces; grows with the rows that a scheduler's warps
-// walk, `share` blocks on an SM) and the sums' (block, team, recurrences, back), and
-// the vector update follows.  The constants are cycles measured on a B200 at 1.92
-// GHz: modelled / measured per iteration 64^2 1.76 / 1.89 us, 128^2 2.2 / 2.6, 256^2
-// 3.9 / 4.3, 512^2 4.3 / 5.2.
-static double res_cost(int K, int warps, int blocks, bool cl, int share, bool f64) {
-    const double rows = (double)ceil_div(warps * share, 4) * K * (f64 ? 2 : 1);
-    const double workers = 600 + 150 * rows;
-    const double sums = blocks == 1 ? 900 : cl ? 1250 + 15 * blocks : 2300 + 9 * blocks;
-    return 2 * (std::max(workers, sums) + 150 + 25 * rows) / 1920;
+// Modelled time of an iteration, us: waiting for exchanges, the depth of a thread's
+// column, a scheduler's warps and the rows they walk (`share` blocks on an SM), the blocks
+// whose sums arrive, and in a cluster columns of faces between blocks (bx > 1).  Fitted to
+// cycles measured on a B200 at 1.92 GHz; within 8% of 60 splits of lattices from 16^2 to 512^2.
+static double res_cost(int K, int warps, int bx, int by, bool cl, int share, bool f64) {
+    const int wps = ceil_div(warps * share, 4), rows = wps * K, n = bx * by;
+    if (f64) return ((n == 1 ? 3000 : cl ? 3390 : 5600) + 340 * K * K + 400 * rows) / 1920.0;
+    if (cl || n == 1) return (3060 + (bx > 1 ? 40 : 20) * K * K + 100 * wps + 170 * rows + 14 * n) / 1920.0;
+    return (5700 + 110 * rows + 3 * n) / 1920.0;
 }
 
 static std::vector<ResPlan> res_plans(int L1, int L2, int nb, int max_cluster, bool f64) {
@@ -40,7 +38,7 @@ static std::vector<ResPlan> res_plans(int L1, int L2, int nb, int max_cluster, b
                 const int wx = ceil_div(ntx, bx), wy = ceil_div(nty, by), n = bx * by;
                 if (wx * wy > kResWarps) continue;
                 const bool cl = n <= max_cluster;
-                const double cost = res_cost(K, wx * wy, n, cl, 1, f64);
+                const double cost = res_cost(K, wx * wy, bx, by, cl, 1, f64);
                 if (!best[n].K || cost < best[n].cost)
                     best[n] = ResPlan{K, cl ? 1 : 0, f64 ? 1 : 0, bx, by, wx, wy, ntx, nty, cost};
             }
@@ -90,7 +88,7 @@ int res_plan_ms(int L1, int L2, int nb, int n, int device, ResPlan* best) {
                 ResPlan p{K, 0, 1, bx, by, ceil_div(ntx, bx), ceil_div(nty, by), ntx, nty, 0.0};
                 if (p.wx * p.wy > kResWarps || !res_ms_fits(p, n, limit)) continue;
                 const double shifts = 36.0 * p.wx * p.wy * K * (n - 1) / 1920;
-                p.cost = std::max(res_cost(K, p.wx * p.wy, bx * by, false, 1, true), shifts);
+                p.cost = std::max(res_cost(K, p.wx * p.wy, bx, by, false, 1, true), shifts);
                 if (!best->K || p.cost < best->cost) *best = p;
             }
     }
@@ -103,7 +101,7 @@ static double res_time(const ResPlan& p, int n, int num_sms) {
     const int at = p.cl ? res_clusters(p) : num_sms / p.blocks();
     if (at < 1) return 1e30;
     const int m = std::min(n, at), share = ceil_div(m * p.blocks(), num_sms);
-    return ceil_div(n, at) * res_cost(p.K, p.wx * p.wy, p.blocks(), p.cl, share, p.f64);
+    return ceil_div(n, at) * res_cost(p.K, p.wx * p.wy, p.bx, p.by, p.cl, share, p.f64);
 }
 
 // A batch of lattices: sizes (L1, L2), counts n.  One size: the split with the least
@@ -150,7 +148,7 @@ std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& size
 size_t res_slot_bytes(const ResPlan& p, int nteams) {
     const size_t nslots = res_slots(p, p.f64 ? 2 : 1), nb = p.blocks();
     if (p.cl) return 16;
-    return sizeof(ulonglong2) * nteams * (nb * 2 * (nslots + nb) + 16) + 16;
+    return sizeof(ulonglong2) * nteams * (nb * (2 * nslots + 4) + kResAcc / 2) + 16;
 }
 
 // the kernel's parameters; clears the slots
@@ -173,9 +171,9 @@ static int res_fill(const ResArgs& a, const ResPlan& plan, int nteams, cudaStrea
     P.want_g5 = a.want_g5;
     P.nslots = res_slots(plan, plan.f64 ? 2 : 1);
     P.psum = (ulonglong2*)a.slots;
-    P.slots = P.psum + (size_t)nteams * 2 * P.nb * P.nb;
+    P.slots = P.psum + (size_t)nteams * 4 * P.nb;
     P.acc = (u64*)(P.slots + (size_t)nteams * P.nb * 2 * P.nslots);
-    P.queue = (int*)(P.acc + (size_t)nteams * 32);
+    P.queue = (int*)(P.acc + (size_t)nteams * kResAcc);
     P.m2 = a.m2;
     P.out = a.out;
     P.ctl = a.ctl;

@@ -1,6 +1,7 @@
-// resident.cuh -- the on-chip CG: the whole state of a solve (links, r, p, t, x; in
-// FP32 for the mixed solver, resident.cu, in FP64 for the other, resident_f64.cu) lives in registers and shared memory for the length of the solve, and
-// only halos and partial sums leave an SM.
+// resident.cuh -- the on-chip CG: the whole state of a solve (links, r, p, q, x; in
+// FP32 for the mixed solver, resident.cu, in FP64 for the other, resident_f64.cu) lives
+// in registers and shared memory for the length of the solve, and only halos and
+// partial sums leave an SM.
 //
 // A *team* of blocks solves one system.  The lattice is cut into warp tiles of at
 // most 32 x K sites: lane = i1, a thread holds a column of K sites, so neighbours
@@ -18,26 +19,36 @@
 // 16 bytes, (value, sequence number) twice, each half a single 64-bit store: the
 // receiver polls the slot itself, so there is no fence, no flag and no barrier on
 // the way.  A team that is one thread-block cluster has its slots in the receivers'
-// shared memory, a larger one in global memory.  A slot of exchange n is overwritten
-// by exchange n + 2, which its sender starts only after every block has published
-// its partial of n + 1, i.e. after the slot has been read.
+// shared memory, a larger one in global memory.  There are two buffers of them, for
+// the two stencils of an iteration.  The first's slots are sent to again after the sum
+// that followed, to which a block adds when its warps have read them; the second's after
+// the first exchange of the next iteration, whose face from the same neighbouring warp
+// says that that warp has read them.
 //
-// One iteration has two exchanges, each halo + sum: r with |r|^2, t with |t|^2.
-// Both stencils run while the sum of their exchange is on its way, and so do the
-// updates of p and x (in shared memory), which nothing waits for:
-//   w = g5Dw r,  x += alpha p    ; beta      ; t = w + beta t
-//   w = g5Dw t,  p = r + beta p  ; alpha     ; r -= alpha w
-// (g5Dw is linear, so t = g5Dw p; the recurrences, the reliable updates and the
-// FP64 stop rule are those of k_cg_mixed's second form).  One extra warp per block
-// does the block's sum, the team's sum and the scalar recurrences.
+// Mixed: the iteration of the solver's other forms, with a sum behind each stencil,
+//   w = g5Dw r          halo of r, |r|^2 summed meanwhile; x += alpha p while faces arrive
+//   beta;  t = w + beta t (= g5Dw p)
+//   w = g5Dw t          halo of t, <p, A p> = |t|^2 + mu^2 |p|^2 meanwhile; p = r + beta p
+//   alpha; r -= alpha (w + mu^2 p)
+// FP64: Chronopoulos and Gear's recurrences (J. Comput. Appl. Math. 25 (1989) 153),
+// which need |r|^2 and <r, A r> = |g5Dw r|^2 + mu^2 |r|^2 only, so one sum:
+//   t = g5Dw r          halo of r
+//   w = g5Dw t + mu^2 r halo of t; the sum of both meanwhile, and p, x of the last iteration
+//   beta = |r|^2 / |r_old|^2,  alpha = |r|^2 / (<r, A r> - beta |r|^2 / alpha_old)
+//   q = w + beta q (= A p),  r -= alpha q;  later p = r_old + beta p, x += alpha p
+// Iteration counts and residuals are those of the other forms (64^2, 128^2, masses down
+// to 0.02 and -0.05, residuals to 1e-14), and 128^2 takes 3.0 us an iteration instead of
+// 4.4.  The mixed solver does not use them, although 256^2 would take 2.9 us instead of
+// 3.5: FP32 rounding and the jumps of r at reliable updates break the identity behind
+// alpha near the critical mass, where solves that converge otherwise did not.  One extra
+// warp per block does the block's sum, the team's sum and the scalar recurrences.
 //
-// What bounds it (B200, 1.92 GHz): the exchanges.  64^2 (one cluster of 16 blocks):
-// 3700 cycles an iteration, of which 2 x 1500 are sum, exchange and recurrences; 512^2
-// (144 blocks): 9000, where both chains take about 4000 an exchange, the workers'
-// stencil (355 instructions per site row and iteration, issue slots 44% used) and the
-// sums (2600 from partial to total).  Against the grid solver with its state in L2:
-// 64^2 4.85 -> 1.89 us per iteration, 128^2 5.95 -> 2.63, 256^2 7.1 -> 4.3,
-// 512^2 12.3 -> 5.2 (reliable updates included).
+// What bounds it (B200): exchanges, until about 8 rows a scheduler's warps walk, then
+// issue.  A sum over a grid takes 1.15 us from the last block's contribution until it is
+// seen, plus 0.25 us of skew between the blocks, 0.2 us for the block's own sum and 0.25
+// us for the recurrences, whatever the split; in a cluster about half of that, which the
+// stencil's own chain (0.8 us) hides.  us an iteration, mixed: 64^2 1.95, 128^2 2.7, 256^2
+// 3.5, 512^2 4.3; FP64: 64^2 2.2, 128^2 3.0, 256^2 4.2, 350x370 6.6.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -51,6 +62,7 @@ namespace qed2d {
 
 constexpr int kResWarps = 15;      // most worker warps of a block (with the scalar warp: 128 registers a thread)
 constexpr int kResCluster = 16;    // most blocks of a cluster
+constexpr int kResAcc = 32;        // words of a team's fixed-point sums: two sets of four, 128 bytes apart
 
 typedef unsigned long long u64;
 
@@ -83,7 +95,7 @@ struct ResP {
     int* queue;               // next system (more systems than teams)
     ulonglong2* slots;        // halo slots: [team][block][2][slots]
     ulonglong2* psum;         // partial slots: [team][2][nb]
-    u64* acc;                 // fixed-point sums: [team][32] words
+    u64* acc;                 // fixed-point sums: [team][kResAcc] words
     int nslots;               // slots of one buffer of a block
     ResOut* out;
     DevCtl* ctl;
@@ -94,10 +106,10 @@ enum { RF_GO, RF_UPD, RF_FIN, RF_STOP, RF_ZERO, RF_ABORT };   // the last three 
 
 // what the scalar warp hands to the workers after an exchange
 struct ResSc {
-    double c;       // alpha or beta
-    float cf;
-    int flag;
-    double s;       // scale of the FP32 vectors
+    double alpha, beta;   // FP64 solver
+    int flag;             // FP64 solver
+    float2 cf;            // mixed solver: alpha or beta, and the flag's bits
+    double s;             // scale of the FP32 vectors
 };
 
 // named barriers: 1 the workers' partials are in (scalar warp waits), 2 the faces
@@ -187,22 +199,21 @@ struct SpDcg {
     __device__ __forceinline__ Pair<double> ld(long long x) const { return {__ldcg(p + x), __ldcg(p + x + V)}; }
 };
 
-// dynamic shared memory of a block: per worker warp x, p and (mixed, during updates)
-// t of its sites and the inbox of faces from other warps of the block
+// dynamic shared memory of a block: per worker warp x, p and q of its sites and two
+// inboxes (one per exchange of an iteration) of faces from other warps of the block
 template <class R, int K>
 struct ResSm {
     static constexpr int BOX = 2 * K + 64;   // left, right columns [K], lower, upper rows [32]
-    static constexpr int ARRAYS = std::is_same<R, float>::value ? 3 : 2;
     static __host__ __device__ size_t bytes(int nw) {
-        return (size_t)nw * (ARRAYS * K * 32 * sizeof(V4<R>) + BOX * sizeof(V2<R>));
+        return (size_t)nw * (3 * K * 32 * sizeof(V4<R>) + 2 * BOX * sizeof(V2<R>));
     }
 };
 
 // a block's place in its team
 struct TeamComm {
     u64 slots;           // global halo slots of the team, or this block's in shared memory (CL)
-    u64 psum;            // the team's partials, [2][receiving block][sending block], or this block's row pair (CL)
-    u64* acc;            // the team's fixed-point sums: two pairs of words (not CL)
+    u64 psum;            // the team's partials, [2][value][block], or this block's rows of them (CL)
+    u64* acc;            // the team's fixed-point sums: two sets of words (not CL)
     int nb, rank, nslots;
     int* err;
 };
@@ -220,109 +231,123 @@ struct Patience {
     }
 };
 
-// warp-wide: publishes this block's partial of exchange seq to every block of the
-// team and returns the team's sum (same additions in the same order in every block)
-__device__ __forceinline__ bool team_sum_slots(const TeamComm& C, unsigned seq, double v, double& tot) {
+// The sums of an exchange: g, and in the FP64 solver (NV = 2) d.
+struct Sums {
+    double g, d;
+};
+
+// warp-wide: publishes this block's partials of sum `seq` in its slots of rows that
+// the whole team polls, and returns the team's sums (same additions in the same order
+// in every block).  For the few sums whose size is not known beforehand.
+template <int NV>
+__device__ __forceinline__ bool team_sum_slots(const TeamComm& C, unsigned seq, Sums v, Sums& tot) {
     const int nb = C.nb, lane = threadIdx.x & 31;
-    const u64 w = (u64)__double_as_longlong(v);
-    const u64 w0 = tag((unsigned)w, seq), w1 = tag((unsigned)(w >> 32), seq);
     bool ok = true;
-    double s = 0.0;
     Patience pt;
-    const u64 rows = C.psum + (u64)(seq & 1u) * nb * nb * 16;
-#pragma unroll 1
-    for (int i = lane; i < nb; i += 32) st_slot<false>(rows + ((u64)i * nb + C.rank) * 16, w0, w1);
-#pragma unroll 1
-    for (int i = 0; i < nb && ok; i += 32) {
-        ulonglong2 q;
-        for (;;) {
-            q = ld_slot<false>(rows + ((u64)C.rank * nb + min(i + lane, nb - 1)) * 16);
-            if (__all_sync(0xffffffffu, tagged(q, seq))) break;
-            if (!(ok = pt.more(C.err))) break;
-        }
-        if (i + lane < nb) s += slot_double(q);
+    const u64 rows = C.psum + (u64)(seq & 1u) * 2 * nb * 16;
+    if (lane < NV) {
+        const u64 w = (u64)__double_as_longlong(lane ? v.d : v.g);
+        st_slot<false>(rows + ((u64)lane * nb + C.rank) * 16, tag((unsigned)w, seq), tag((unsigned)(w >> 32), seq));
     }
-    tot = warp_sum(s);
+    double s[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < NV; k++)
+#pragma unroll 1
+        for (int i = 0; i < nb && ok; i += 32) {
+            ulonglong2 q;
+            for (;;) {
+                q = ld_slot<false>(rows + ((u64)k * nb + min(i + lane, nb - 1)) * 16);
+                if (__all_sync(0xffffffffu, tagged(q, seq))) break;
+                if (!(ok = pt.more(C.err))) break;
+            }
+            if (i + lane < nb) s[k] += slot_double(q);
+        }
+    tot.g = warp_sum(s[0]);
+    if (NV > 1) tot.d = warp_sum(s[1]);
     return ok;
 }
 
-// The same in a cluster: every block's partial goes to a slot in every block's
-// shared memory.  (Every warp's partial to every block, without the block's own sum
-// first, measured slower: 64^2 over 16 blocks 1970 cycles from partial to sum against 1400.)
-__device__ __forceinline__ bool cluster_sum_slots(const TeamComm& C, unsigned seq, double v, double& tot) {
+// The same in a cluster: every block's partials go to slots in every block's shared
+// memory, lanes 0-15 for the first, 16-31 for the second.  (Every warp's partial to
+// every block, without the block's own sum first, measured slower: 64^2 over 16 blocks
+// 1970 cycles from partial to sum against 1400.)
+template <int NV>
+__device__ __forceinline__ bool cluster_sum_slots(const TeamComm& C, unsigned seq, Sums v, Sums& tot) {
     const int nb = C.nb, lane = threadIdx.x & 31;
-    const unsigned row = (unsigned)C.psum + 16 * (seq & 1u) * kResCluster;
-    const u64 w = (u64)__double_as_longlong(v);
-    if (lane < nb) st_slot<true>(map_rank(row + 16 * C.rank, lane), tag((unsigned)w, seq), tag((unsigned)(w >> 32), seq));
+    const int n2 = NV > 1 || nb > 8 ? kResCluster : nb > 4 ? 8 : nb > 2 ? 4 : 2;   // nb up to a power of two
+    const int from = lane & (n2 - 1), k = NV > 1 ? lane / kResCluster : 0;
+    const unsigned row = (unsigned)C.psum + 16 * ((seq & 1u) * 2 + k) * kResCluster;
+    const u64 w = (u64)__double_as_longlong(k ? v.d : v.g);
+    if ((NV > 1 ? from : lane) < nb)
+        st_slot<true>(map_rank(row + 16 * C.rank, from), tag((unsigned)w, seq), tag((unsigned)(w >> 32), seq));
     ulonglong2 q;
     Patience pt;
     bool ok = true;
     for (;;) {
-        q = ld_slot<true>(row + 16 * min(lane, nb - 1));
+        q = ld_slot<true>(row + 16 * min(from, nb - 1));
         if (__all_sync(0xffffffffu, tagged(q, seq))) break;
         if (!(ok = pt.more(C.err))) break;
     }
-    double s = lane < nb ? slot_double(q) : 0.0;
+    // every group of n2 lanes adds the same values in the same tree
+    double s = from < nb ? slot_double(q) : 0.0;
 #pragma unroll
-    for (int o = kResCluster / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    tot = __shfl_sync(0xffffffffu, s, 0);
+    for (int o = kResCluster / 2; o > 0; o >>= 1)
+        if (o < n2) s += __shfl_xor_sync(0xffffffffu, s, o);
+    tot.g = NV > 1 ? __shfl_sync(0xffffffffu, s, 0) : s;
+    if (NV > 1) tot.d = __shfl_sync(0xffffffffu, s, kResCluster);
     return ok;
 }
 
-// The same through one pair of atomic words (large teams over global memory): the
-// partial in 80-bit fixed point, 40 bits a word, scaled by a power of two that every
-// block derives from an earlier sum, with a count of the blocks in the top byte of
-// each word.  Integer additions commute, so the sum does not depend on the order; it
-// is exact to 2^-76 of that earlier sum `est` (and repeated through the slots when
-// that leaves less than 52 bits of it).  The words only grow (modulo 2^64), two pairs
-// in turn, so nothing is cleared; `base` is the pair's value before the exchange.
-// A partial out of range (or NaN) is counted in the next byte instead, and then every
-// block falls back to team_sum_slots.  Measured with 144 blocks: 1430 cycles an
-// exchange, against 2970 through the slots (whose polls grow with the square of the
-// team) and 2440 with an arrival counter and partials behind it.
-__device__ __forceinline__ bool team_sum_fixed(const TeamComm& C, unsigned seq, double v, double est, ulonglong2& base,
-                                               double& tot, bool& exact) {
+// The same through atomic words (teams over global memory): a partial in 80-bit fixed
+// point, 40 bits a word, scaled by a power of two that every block derives from an
+// earlier sum, with a count of the blocks in the top byte of each word.  Integer
+// additions commute, so the sum does not depend on the order; it is exact to 2^-76 of
+// that earlier sum `est` (and repeated through the slots when that leaves less than 52
+// bits of it).  The words only grow (modulo 2^64), two sets in turn, so nothing is
+// cleared; `base` is the set's value before the exchange.  A partial out of range (or
+// NaN) is counted in the next byte instead, and then every block falls back to
+// team_sum_slots.  A lane per word, side by side, so that a block's atomics are one
+// request and its poll another: with a line for each word 128^2 and 256^2 in FP64 took
+// 2% more, with two polls in flight 13%.  Measured with 144
+// blocks: 1610 cycles an exchange, against 2970 with a row of slots per block (whose
+// polls grow with the square of the team), 4660 with one row, 2440 with an arrival
+// counter and partials behind it, and 2740 through 7 clusters of 16 blocks (distributed
+// shared memory, then L2 between the clusters' first blocks).
+template <int NV>
+__device__ __forceinline__ bool team_sum_fixed(const TeamComm& C, unsigned seq, Sums v, Sums est, u64& base, Sums& tot,
+                                               bool need_d, bool& exact) {
     const int lane = threadIdx.x & 31;
-    u64* acc = C.acc + 16 * (seq & 1u);
-    const int ex = min(max((int)((u64)__double_as_longlong(est) >> 52 & 0x7ff) - 1023, -900), 900);
-    ulonglong2 d = make_ulonglong2(0, 0);
-    int ok = 1;
-    if (lane == 0) {
-        const double up = __longlong_as_double((long long)(1023 + 36 - ex) << 52);
-        const double y = v * up;   // exact
+    u64* acc = C.acc + 16 * (seq & 1u) + (lane & 3);
+    const double e = (lane & 2) ? est.d : est.g, x = (lane & 2) ? v.d : v.g;
+    const int ex = min(max((int)((u64)__double_as_longlong(e) >> 52 & 0x7ff) - 1023, -900), 900);
+    if (lane < 2 * NV) {
+        const double y = x * __longlong_as_double((long long)(1023 + 36 - ex) << 52);   // exact
         const bool fits = y < 1099511627776.0;   // 2^40; false for NaN
         const double hi = floor(y);
-        const u64 h = fits ? (u64)hi : 1ull << 48, l = fits ? (u64)((y - hi) * 1099511627776.0) : 0ull;
-        const u64 one = 1ull << 56;
-        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(acc), "l"(h + one) : "memory");
-        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(acc + 1), "l"(l + one) : "memory");
-        unsigned n = 0;
-        for (;;) {
-            const ulonglong2 q = ld_slot<false>((u64)acc);
-            d.x = q.x - base.x;
-            d.y = q.y - base.y;
-            if ((int)(d.x >> 56) == C.nb && (int)(d.y >> 56) == C.nb) {
-                base = q;
-                break;
-            }
-            if ((++n & 255u) == 0) {
-                if (ld_volatile_int(C.err) != 0) ok = 0;
-                else if (n > (1u << 22)) {
-                    atomicExch(C.err, 2 /* QED2D_ERR_TIMEOUT */);
-                    ok = 0;
-                }
-                if (!ok) break;
-            }
-        }
-        const double down = __longlong_as_double((long long)(1023 - 36 + ex) << 52);
-        tot = ((double)(long long)(d.x & ((1ull << 48) - 1)) +
-               (double)(long long)(d.y & ((1ull << 56) - 1)) * 0x1p-40) * down;
-        // no block out of range, and 52 bits left of the sum
-        exact = ((d.x >> 48) & 0xff) == 0 && tot >= __longlong_as_double((long long)(1023 - 24 + ex) << 52);
+        const u64 part = fits ? (u64)((lane & 1) ? (y - hi) * 1099511627776.0 : hi) : (lane & 1) ? 0ull : 1ull << 48;
+        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(acc), "l"(part + (1ull << 56)) : "memory");
     }
-    tot = __shfl_sync(0xffffffffu, tot, 0);
-    exact = __shfl_sync(0xffffffffu, (int)exact, 0);
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    u64 d = 0;
+    bool ok = true;
+    Patience pt;
+    for (;;) {
+        u64 q = base;
+        if (lane < 2 * NV) asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(q) : "l"(acc) : "memory");
+        d = q - base;
+        if (__all_sync(0xffffffffu, lane >= 2 * NV || (int)(d >> 56) == C.nb)) {
+            base = q;
+            break;
+        }
+        if (!(ok = pt.more(C.err))) break;
+    }
+    const double w = (double)(long long)(d & ((lane & 1) ? (1ull << 56) - 1 : (1ull << 48) - 1));
+    const double s = (w + __shfl_xor_sync(0xffffffffu, w, 1) * 0x1p-40) * __longlong_as_double((long long)(1023 - 36 + ex) << 52);
+    tot.g = __shfl_sync(0xffffffffu, s, 0);
+    if (NV > 1) tot.d = __shfl_sync(0xffffffffu, s, 2);
+    // no block out of range, and 52 bits left of the sum
+    const bool good = ((d >> 48) & 0xff) == 0 && s >= __longlong_as_double((long long)(1023 - 24 + ex) << 52);
+    exact = __all_sync(0xffffffffu, good || !(lane == 0 || (NV > 1 && lane == 2 && need_d)));
+    return ok;
 }
 
 // ---------------------------------------------------------------------------
@@ -338,135 +363,195 @@ struct Tile {
     int w, h;            // the warp's sites: w lanes, h rows (0: no tile)
     int srcL, srcR;      // lanes of the neighbours along i1
     bool el, er;         // this lane is the tile's first / last column
-    // where this thread's faces go in the block's inboxes, -1: another block
-    int xto;             // the column's (el, er lanes)
-    int dto, uto;        // the lower and the upper row's
+    // where this thread's faces go in the block's inboxes (column: el, er lanes; lower and
+    // upper row), -1: to another block
+    int xto, dto, uto;
+    bool rx, rd, ru;     // this thread reads slots of a column, the lower, the upper row
+    const WarpFace* W;
+    unsigned sx, sd, su, fx, fd, fu;   // its slots to send to and to read
+};
+// The slots' addresses are worked out once where registers are left for them (512^2 mixed
+// 4.35 -> 4.29 us an iteration, 128^2 in FP64 3.17 -> 2.98), not for FP64 columns of two
+// sites, which spill (350x370 6.5 -> 8.4).
+template <class R, int K, bool CL>
+struct Slots {
+    static constexpr bool REGS = K * sizeof(R) < 16 || std::is_same<R, float>::value;
+    static constexpr bool PRE = REGS && !CL;   // read the block's own inbox before the slots have arrived (a cluster's do at once)
+    static constexpr int E = 16 * Num<R>::SLOTS;   // bytes of a face entry
+    static __device__ __forceinline__ int lane() { return threadIdx.x & 31; }
+    static __device__ __forceinline__ int side() { return lane() >= K ? 1 : 0; }   // the first 2K lanes read a row each of the left and right columns
+    static __device__ __forceinline__ void init(Tile& T) {
+        if (!REGS) return;
+        T.sx = T.W->to[T.el ? 0 : 1];
+        T.sd = T.W->to[2] + E * lane();
+        T.su = T.W->to[3] + E * lane();
+        T.fx = T.W->from[side()] + E * (lane() - side() * K);
+        T.fd = T.W->from[2] + E * lane();
+        T.fu = T.W->from[3] + E * lane();
+    }
+    static __device__ __forceinline__ unsigned sx(const Tile& T) { return REGS ? T.sx : T.W->to[T.el ? 0 : 1]; }
+    static __device__ __forceinline__ unsigned sd(const Tile& T) { return REGS ? T.sd : T.W->to[2] + E * lane(); }
+    static __device__ __forceinline__ unsigned su(const Tile& T) { return REGS ? T.su : T.W->to[3] + E * lane(); }
+    static __device__ __forceinline__ unsigned fx(const Tile& T) { return REGS ? T.fx : T.W->from[side()] + E * (lane() - side() * K); }
+    static __device__ __forceinline__ unsigned fd(const Tile& T) { return REGS ? T.fd : T.W->from[2] + E * lane(); }
+    static __device__ __forceinline__ unsigned fu(const Tile& T) { return REGS ? T.fu : T.W->from[3] + E * lane(); }
 };
 
 template <class R>
 __device__ __forceinline__ V4<R> mk4(R a, R b, R c, R d) { return V4<R>{a, b, c, d}; }
+// A complex number's two parts in one instruction (PK; float: f32x2, the same rounding as
+// two scalar operations at half the issue slots).  A cluster's warps with columns of four
+// are too few to issue at all times, and the pairs' register moves only lengthen their
+// chains: 64^2 over 4 blocks 2.83 us an iteration with it, 2.69 without; over a grid 512^2
+// 4.29 with it, 4.60 without.
+template <int K, bool CL> constexpr bool kPacked = !(CL && K == 4);
+__device__ __forceinline__ u64 bits2(float2 a) { return *reinterpret_cast<u64*>(&a); }
+template <bool PK>
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    if constexpr (!PK) return make_float2(a.x + b.x, a.y + b.y);
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)));
+    return *reinterpret_cast<float2*>(&r);
+}
+template <bool PK>
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    if constexpr (!PK) return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+    return *reinterpret_cast<float2*>(&r);
+}
+template <bool PK>
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    if constexpr (!PK) return make_float2(a.x - b.x, a.y - b.y);
+    return fma2<PK>(b, make_float2(-1.f, -1.f), a);
+}
+template <bool PK>
+__device__ __forceinline__ double2 add2(double2 a, double2 b) { return a + b; }
+template <bool PK>
+__device__ __forceinline__ double2 sub2(double2 a, double2 b) { return a - b; }
+template <bool PK>
+__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
+    return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
 template <class R>
-__device__ __forceinline__ V2<R> half1(const V4<R>& s) { return mk(s.x - s.z, s.y - s.w); }
+__device__ __forceinline__ V2<R> up(const V4<R>& s) { return mk(s.x, s.y); }   // the two spin components
 template <class R>
-__device__ __forceinline__ V2<R> half2(const V4<R>& s, V2<R> u1) { return cjmul(u1, mk(s.x + s.z, s.y + s.w)); }
+__device__ __forceinline__ V2<R> dn(const V4<R>& s) { return mk(s.z, s.w); }
+template <class R>
+__device__ __forceinline__ V4<R> join(V2<R> a, V2<R> b) { return mk4<R>(a.x, a.y, b.x, b.y); }
+
+template <class R, bool PK>
+__device__ __forceinline__ V2<R> half1(const V4<R>& s) { return sub2<PK>(up<R>(s), dn<R>(s)); }
+template <class R, bool PK>
+__device__ __forceinline__ V2<R> half2(const V4<R>& s, V2<R> u1) { return cjmul(u1, add2<PK>(up<R>(s), dn<R>(s))); }
 template <class R>
 __device__ __forceinline__ V2<R> half3(const V4<R>& s) { return mk(s.x - s.w, s.y + s.z); }
 template <class R>
 __device__ __forceinline__ V2<R> half4(const V4<R>& s, V2<R> u2) { return cjmul(u2, mk(s.x + s.w, s.y - s.z)); }
 
+// w += the hopping terms f2 (from above) and b2 (from below): (f + b, i (f - b))
+template <class R, bool PK>
+__device__ __forceinline__ void hop2(V4<R>& w, V2<R> f, V2<R> b) {
+    const V2<R> s = add2<PK>(add2<PK>(up<R>(w), f), b);
+    w.x = s.x;
+    w.y = s.y;
+    w.z += b.y - f.y;
+    w.w += f.x - b.x;
+}
+
 // The first half of w = g5Dw S: sends the tile's faces, then everything that
 // does not come through one.  The links carry the factor -1/2.
 template <class R, int K, bool CL>
-__device__ __forceinline__ void stencil_inner(const Tile& T, const WarpFace& W, const V4<R> (&S)[K],
+__device__ __forceinline__ void stencil_inner(const Tile& T, const V4<R> (&S)[K],
                                               const V2<R> (&u1)[K], const V2<R> (&u2)[K], R m2, V2<R>* box,
-                                              const TeamComm& C, unsigned seq, V4<R> (&w)[K]) {
-    const int lane = threadIdx.x & 31;
-    constexpr int E = 16 * Num<R>::SLOTS;   // bytes of a face entry
-    V2<R> h1[K], h2[K];
+                                              u64 to, unsigned seq, V4<R> (&w)[K]) {
+    constexpr int E = Slots<R, K, CL>::E;
+    constexpr bool PK = kPacked<K, CL>;
     if (T.h == 0) return;
-#pragma unroll
-    for (int j = 0; j < K; j++) {
-        h1[j] = half1<R>(S[j]);
-        h2[j] = half2<R>(S[j], u1[j]);
-    }
-    const u64 slots = (CL ? 0 : C.slots) + (u64)(seq & 1u) * C.nslots * 16;   // W.to holds addresses in a cluster
+    V2<R> h1[K], h2[K], h4[K];
     {   // rows
         const V2<R> lo = half3<R>(S[0]);
         if (T.dto >= 0) box[T.dto] = lo;
-        else send2<CL>(slots + W.to[2] + E * lane, lo, seq);
+        else send2<CL>(to + Slots<R, K, CL>::sd(T), lo, seq);
         constexpr int J = K > 1 ? K - 2 : 0;   // tiles have K or K - 1 rows (res_plan)
         const bool full = T.h == K;
-        const V2<R> h4a = half4<R>(S[K - 1], u2[K - 1]), h4b = half4<R>(S[J], u2[J]);
-        const V2<R> hi = mk(full ? h4a.x : h4b.x, full ? h4a.y : h4b.y);
+        h4[K - 1] = half4<R>(S[K - 1], u2[K - 1]);
+        h4[J] = half4<R>(S[J], u2[J]);
+        const V2<R> hi = mk(full ? h4[K - 1].x : h4[J].x, full ? h4[K - 1].y : h4[J].y);
         if (T.uto >= 0) box[T.uto] = hi;
-        else send2<CL>(slots + W.to[3] + E * lane, hi, seq);
+        else send2<CL>(to + Slots<R, K, CL>::su(T), hi, seq);
+    }
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        h1[j] = half1<R, PK>(S[j]);
+        h2[j] = half2<R, PK>(S[j], u1[j]);
+        if (j + 2 < K) h4[j] = half4<R>(S[j], u2[j]);
     }
     if (T.el || T.er) {   // columns
         if (T.xto >= 0) {
 #pragma unroll
             for (int j = 0; j < K; j++) box[T.xto + j] = T.el ? h1[j] : h2[j];
         } else {
-            const u64 sl = slots + W.to[T.el ? 0 : 1];
 #pragma unroll
-            for (int j = 0; j < K; j++) send2<CL>(sl + E * j, T.el ? h1[j] : h2[j], seq);
+            for (int j = 0; j < K; j++) send2<CL>(to + Slots<R, K, CL>::sx(T) + E * j, T.el ? h1[j] : h2[j], seq);
         }
     }
+    const V2<R> mm = mk(m2, m2), mn = mk(-m2, -m2), zero = mk(R(0), R(0));
 #pragma unroll
     for (int j = 0; j < K; j++) {
         V2<R> fh = mk(__shfl_sync(0xffffffffu, h1[j].x, T.srcR), __shfl_sync(0xffffffffu, h1[j].y, T.srcR));
         V2<R> b1 = mk(__shfl_sync(0xffffffffu, h2[j].x, T.srcL), __shfl_sync(0xffffffffu, h2[j].y, T.srcL));
-        if (T.er) fh = mk(R(0), R(0));
-        if (T.el) b1 = mk(R(0), R(0));
-        const V4<R> s = S[j];
+        if (T.er) fh = zero;
+        if (T.el) b1 = zero;
         const V2<R> f1 = cmul(u1[j], fh);
-        w[j].x = m2 * s.x + (f1.x + b1.x);
-        w[j].y = m2 * s.y + (f1.y + b1.y);
-        w[j].z = -m2 * s.z + (f1.x - b1.x);
-        w[j].w = -m2 * s.w + (f1.y - b1.y);
+        w[j] = join<R>(fma2<PK>(mm, up<R>(S[j]), add2<PK>(f1, b1)), fma2<PK>(mn, dn<R>(S[j]), sub2<PK>(f1, b1)));
+        // along i2 inside the tile; the bond to a missing highest row carries zeros from above only
+        V2<R> f2 = zero, b2 = zero;
+        if (j + 1 < K) f2 = cmul(u2[j], half3<R>(S[j + 1 < K ? j + 1 : j]));
+        if (j > 0) b2 = h4[j > 0 ? j - 1 : 0];
+        if (j == K - 1 && T.h < K) b2 = zero;
+        hop2<R, PK>(w[j], f2, b2);
     }
-#pragma unroll
-    for (int j = 0; j + 1 < K; j++)
-        if (j + 1 < T.h) {   // the bond between rows j and j + 1
-            const V2<R> f2 = cmul(u2[j], half3<R>(S[j + 1])), b2 = half4<R>(S[j], u2[j]);
-            w[j].x += f2.x;
-            w[j].y += f2.y;
-            w[j].z -= f2.y;
-            w[j].w += f2.x;
-            w[j + 1].x += b2.x;
-            w[j + 1].y += b2.y;
-            w[j + 1].z += b2.y;
-            w[j + 1].w -= b2.x;
-        }
 }
 
 // The second half: the faces of other tiles.  Those of other blocks are asked for
 // first, `meanwhile` runs while the answers are on their way, and what has not
 // arrived by then is polled.  False when a wait gave up.
 template <class R, int K, bool CL, class F>
-__device__ __forceinline__ bool stencil_faces(const Tile& T, const WarpFace& W, const V2<R> (&u1)[K],
-                                              const V2<R> (&u2)[K], V2<R>* box, const TeamComm& C, unsigned seq,
-                                              V4<R> (&w)[K], F meanwhile) {
-    constexpr int BOX = ResSm<R, K>::BOX, E = 16 * Num<R>::SLOTS;
+__device__ __forceinline__ bool stencil_faces(const Tile& T, const V2<R> (&u1)[K], const V2<R> (&u2)[K], V2<R>* box,
+                                              u64 from, int* err, unsigned seq, V4<R> (&w)[K], F meanwhile) {
+    constexpr int BOX = ResSm<R, K>::BOX;
+    constexpr bool PK = kPacked<K, CL>;
     const int lane = threadIdx.x & 31;
     V2<R>* mine = box + ((threadIdx.x >> 5) - 1) * BOX;
-    const u64 slots = C.slots + (u64)(seq & 1u) * C.nslots * 16;
-    const bool on = T.h > 0;
-    const int side = lane >= K ? 1 : 0;   // the first 2K lanes ask for a row each of the left and right columns
-    const bool rx = on && lane < 2 * K && W.warp[side] < 0 && lane - side * K < T.h;
-    const bool rd = on && T.dto < 0, ru = on && T.uto < 0;
     Arrival<R> qx, qd, qu;
     auto ask = [&]() {
-        if (rd) qd.template ask<CL>(slots + W.from[2] + E * lane);
-        if (ru) qu.template ask<CL>(slots + W.from[3] + E * lane);
-        if (rx) qx.template ask<CL>(slots + W.from[side] + E * (lane - side * K));
+        if (T.rd) qd.template ask<CL>(from + Slots<R, K, CL>::fd(T));
+        if (T.ru) qu.template ask<CL>(from + Slots<R, K, CL>::fu(T));
+        if (T.rx) qx.template ask<CL>(from + Slots<R, K, CL>::fx(T));
     };
     ask();
+    V2<R> lo, hi;
+    if (Slots<R, K, CL>::PRE) lo = mine[2 * K + lane], hi = mine[2 * K + 32 + lane];
     meanwhile();
-    if (!on) return true;
+    if (T.h == 0) return true;
     Patience pt;
     bool ok = true;
     for (;;) {
-        const bool ready = (!rd || qd.here(seq)) && (!ru || qu.here(seq)) && (!rx || qx.here(seq));
+        const bool ready = (!T.rd || qd.here(seq)) && (!T.ru || qu.here(seq)) && (!T.rx || qx.here(seq));
         if (__all_sync(0xffffffffu, ready)) break;
-        if (!(ok = pt.more(C.err))) break;
+        if (!(ok = pt.more(err))) break;
         ask();
     }
-    if (rx) mine[lane] = qx.val();
+    if (T.rx) mine[lane] = qx.val();
     __syncwarp();
-    if (T.el || T.er) {
-        const R sg = T.er ? R(1) : R(-1);
+    V2<R> e[K];
+    if (Slots<R, K, CL>::PRE)
 #pragma unroll
-        for (int j = 0; j < K; j++) {
-            if (j == K - 1 && T.h < K) break;   // no such row: its inbox entry is never written
-            V2<R> e = mine[(T.er ? K : 0) + j];
-            if (T.er) e = cmul(u1[j], e);
-            w[j].x += e.x;
-            w[j].y += e.y;
-            w[j].z += sg * e.x;
-            w[j].w += sg * e.y;
-        }
-    }
-    const V2<R> lo = rd ? qd.val() : mine[2 * K + lane], hi = ru ? qu.val() : mine[2 * K + 32 + lane];
+        for (int j = 0; j < K; j++) e[j] = mine[(T.er ? K : 0) + j];
+    if (!Slots<R, K, CL>::PRE) lo = mine[2 * K + lane], hi = mine[2 * K + 32 + lane];
+    if (T.rd) lo = qd.val();
+    if (T.ru) hi = qu.val();
     w[0].x += lo.x;
     w[0].y += lo.y;
     w[0].z += lo.y;
@@ -488,14 +573,28 @@ __device__ __forceinline__ bool stencil_faces(const Tile& T, const WarpFace& W, 
             w[J].w += fb.x;
         }
     }
+    if (T.el || T.er) {
+        const V2<R> sg = T.er ? mk(R(1), R(1)) : mk(R(-1), R(-1));
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+            if (j == K - 1 && T.h < K) break;   // no such row: its inbox entry is never written
+            if (!Slots<R, K, CL>::PRE) e[j] = mine[(T.er ? K : 0) + j];
+            if (T.er) e[j] = cmul(u1[j], e[j]);
+            w[j] = join<R>(add2<PK>(up<R>(w[j]), e[j]), fma2<PK>(sg, e[j], dn<R>(w[j])));
+        }
+    }
     return ok;
 }
 
-template <class R>
-__device__ __forceinline__ R norm4(const V4<R>& a) { return a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w; }
-template <class R>
+template <class R, bool PK = true>
+__device__ __forceinline__ R norm4(const V4<R>& a) {
+    const V2<R> n = fma2<PK>(up<R>(a), up<R>(a), fma2<PK>(dn<R>(a), dn<R>(a), mk(R(0), R(0))));
+    return n.x + n.y;
+}
+template <class R, bool PK = true>
 __device__ __forceinline__ V4<R> axpy4(R a, const V4<R>& x, const V4<R>& y) {
-    return mk4<R>(y.x + a * x.x, y.y + a * x.y, y.z + a * x.z, y.w + a * x.w);
+    const V2<R> aa = mk(a, a);
+    return join<R>(fma2<PK>(aa, up<R>(x), up<R>(y)), fma2<PK>(aa, dn<R>(x), dn<R>(y)));
 }
 
 // ---------------------------------------------------------------------------
@@ -516,7 +615,7 @@ struct ResMsBlock {              // the shifts' scalars of an iteration
 // what the threads of a block share
 struct ResBlock {
     int nwk;                       // worker threads
-    double part[32 * kResWarps];   // the threads' partials of an exchange
+    double part[2][32 * kResWarps];   // the threads' partials of the two sums
     ResSc sc;
     int abort;                 // a wait of this block gave up
     double next;
@@ -527,89 +626,100 @@ struct ResBlock {
 };
 
 // The scalar warp (warp 0: the scheduler prefers the oldest of its warps, and this
-// one is on the way of all): one step per exchange, in step with the workers.  Returns the
-// exchange it ended at.
+// one is on the way of all): one step per sum, in step with the workers.  Returns the
+// number of sums so far.
 template <bool MIXED, bool CL, bool MS = false>
-__device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsigned seq, ulonglong2& base0,
-                                               ulonglong2& base1, const ResMs* M = nullptr, ResMsBlock* S = nullptr) {
-    enum { X_BEGIN, X_GUESS, X_RR, X_PAP, X_FENCE, X_TRUE };   // what the coming exchange sums
+__device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsigned seq, u64& base0, u64& base1,
+                                               const ResMs* M = nullptr, ResMsBlock* S = nullptr) {
+    enum { X_BEGIN, X_RR, X_PAP, X_FENCE, X_TRUE };   // what the coming exchange sums (X_PAP: mixed only)
+    constexpr int NV = MIXED ? 1 : 2;
     const int nw = MS ? M->nw : (int)(blockDim.x >> 5) - 1, nth = 32 * (nw + 1), lane = threadIdx.x & 31;
-    double zs = 1.0, zp = 1.0, a_last = 1.0, b_last = 0.0, a_now = 0.0;   // MS: lane i's shift; the recurrences' scalars
-    bool act = MS && lane < M->n && lane != M->base;
-    int round = 0;   // MS: barriers with the shift warps so far
-    double rr = 0.0, inv_rr = 0.0, maxrr = 0.0, s = 1.0, beta = 0.0, rr64 = 0.0, bb = 0.0, tol = 0.0;
-    double rr_last = 1.0, pap_last = 4.0;   // the last |r|^2 and <p, A p>: the fixed-point scales
-    double thr = 0.0;                       // |r|^2 below it: reliable update
+    // |r|^2, its inverse, the inverse of the last alpha
+    double rr = 0.0, inv_rr = 0.0, inv_a = 0.0, beta = 0.0;
+    double maxrr = 0.0, thr = 0.0;   // the largest |r|^2 since the last update; below thr: update
+    double s = 1.0, rr64 = 0.0, bb = 0.0, tol = 0.0;
+    double rr_last = 1.0, pap_last = 4.0;   // the last sums: the fixed-point scales
     int k = 0, nupd = 0, fences = 0, flag = RF_GO, next = X_BEGIN;
     bool conv = false, fresh = true;
+    // MS: lane i's shift; the base system's last alpha and the alpha and beta before
+    double zs = 1.0, zp = 1.0, a_now = 0.0, a_last = 1.0, b_now = 0.0;
+    bool act = MS && lane < M->n && lane != M->base;
+    int round = 0;                  // barriers with the shift warps so far
 #pragma unroll 1
     for (;;) {
         ++seq;
-        const bool dead = ld_volatile_int(&B.abort) != 0;   // noted by a worker before the last barrier
-        double tot = 0.0;
+        const bool dead = ld_volatile_int(&B.abort) != 0;   // noted by a worker
+        Sums tot{0.0, 0.0}, v;
         bool ok = true;
         bar_sync_n(1, nth);   // the workers' partials are in
-        double v = 0.0, v1 = 0.0;
+        {
+            double a[4] = {0.0, 0.0, 0.0, 0.0}, c[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-        for (int i = 0; i < kResWarps; i++) {
-            const double a = i < nw ? B.part[32 * i + lane] : 0.0;
-            if (i & 1) v1 += a;
-            else v += a;
+            for (int i = 0; i < kResWarps; i++)
+                if (i < nw) {
+                    a[i & 3] += B.part[0][32 * i + lane];
+                    if (NV > 1) c[i & 3] += B.part[1][32 * i + lane];
+                }
+            v.g = (a[0] + a[1]) + (a[2] + a[3]);
+            v.d = (c[0] + c[1]) + (c[2] + c[3]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                v.g += __shfl_xor_sync(0xffffffffu, v.g, o);
+                if (NV > 1) v.d += __shfl_xor_sync(0xffffffffu, v.d, o);
+            }
         }
-        v = warp_sum(v + v1);
         if (B.C.nb == 1) {
             tot = v;
         } else if constexpr (CL) {
-            ok = cluster_sum_slots(B.C, seq, v, tot);
+            ok = cluster_sum_slots<NV>(B.C, seq, v, tot);
         } else {
             bool exact = false;
             if (next != X_BEGIN) {
-                const double est = next == X_RR ? rr_last : next == X_PAP ? pap_last : next == X_TRUE ? rr64 : 1.0;
-                ulonglong2 bs = (seq & 1u) ? base1 : base0;
-                ok = team_sum_fixed(B.C, seq, v, est, bs, tot, exact);
+                const Sums e{next == X_RR ? rr_last : next == X_PAP ? pap_last : next == X_TRUE ? rr64 : 1.0, pap_last};
+                u64 bs = (seq & 1u) ? base1 : base0;
+                ok = team_sum_fixed<NV>(B.C, seq, v, e, bs, tot, next == X_RR, exact);
                 if (seq & 1u) base1 = bs;
                 else base0 = bs;
             }
-            if (!exact && next != X_FENCE && ok) ok = team_sum_slots(B.C, seq, v, tot);
+            if (!exact && next != X_FENCE && ok) ok = team_sum_slots<NV>(B.C, seq, v, tot);
         }
-        double c = 0.0, rr_old = rr;
+        double alpha = 0.0;
+        const double inv_old = inv_rr;
         const bool all = MS && (next == X_BEGIN || next == X_RR);   // the shift warps join this barrier
         const bool step = MS && next == X_RR && !fresh;             // and an iteration is behind them
-        if (next == X_PAP) {   // <p, (A + mu2) p>
-            c = rr / tot;   // alpha
-            if (MS) a_now = c;
-            pap_last = tot;
+        if (MIXED && next == X_PAP) {   // <p, (A + mu2) p>
+            alpha = rr / tot.g;
+            pap_last = tot.g;
             k++;
             next = X_RR;
-        } else if (next == X_RR) {   // |r|^2
-            next = X_PAP;
-            rr_last = tot;
-            if (fresh) {
-                rr = maxrr = tot;
-                fresh = false;
-            } else if (!MIXED && (tot < tol || k == P.maxiter)) {
-                conv = tot < tol;
-                rr64 = tot;
-                flag = RF_FIN;
+        } else if (next == X_RR) {   // |r|^2; FP64: and |g5Dw r|^2
+            rr_last = tot.g;
+            if (!fresh && ((MIXED ? tot.g < thr : tot.g < tol) || k == P.maxiter)) {
+                flag = MIXED ? RF_UPD : RF_FIN;
                 next = X_FENCE;
-                fences = 1;
-            } else if (MIXED && (tot < thr || k == P.maxiter)) {
-                flag = RF_UPD;
-                nupd++;
-                next = X_FENCE;
-                fences = 2;
-                rr64 = tot / (s * s);
+                fences = MIXED ? 2 : 1;
+                nupd += MIXED;
+                conv = !MIXED && tot.g < tol;
+                rr64 = MIXED ? tot.g / (s * s) : tot.g;
             } else {
-                beta = tot * inv_rr;
-                rr = tot;
+                if (!fresh) beta = tot.g * inv_rr;
+                if (MIXED) {
+                    next = X_PAP;
+                } else {
+                    pap_last = tot.d;
+                    alpha = tot.g / (tot.d + P.mu2 * tot.g - beta * (tot.g * inv_a));   // beta = inv_a = 0 at first
+                    k++;
+                }
+                if (fresh) maxrr = tot.g;
+                fresh = false;
+                rr = tot.g;
             }
-            c = beta;
         } else if (next == X_FENCE) {   // orders the blocks' FP64 stores
             __threadfence();
             if (flag == RF_FIN) flag = RF_STOP;
             if (--fences == 0) next = X_TRUE;
         } else if (next == X_BEGIN) {   // |b|^2
-            bb = rr64 = tot;
+            bb = rr64 = tot.g;
             tol = P.eps * bb;
             conv = bb == 0.0;
             if (MIXED && !conv) s = 1.0 / sqrt(bb);
@@ -618,57 +728,60 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
             next = P.guess ? X_FENCE : X_RR;
             fences = 1;
         } else {   // |b - (A + mu2) x|^2
-            rr64 = tot;
-            conv = tot < tol;
+            rr64 = tot.g;
+            conv = tot.g < tol;
             if (conv || k == P.maxiter) {
                 flag = RF_STOP;
-            } else if (!MIXED) {   // a warm start
-                flag = RF_GO;
-                next = X_RR;
-                rr_last = tot;
-                pap_last = 4.0 * tot;
             } else {
-                const double sn = 1.0 / sqrt(tot);
-                if (nupd) beta = (tot * s * s * inv_rr) * (sn / s);
-                s = sn;
-                fresh = true;
                 flag = RF_GO;
                 next = X_RR;
-                rr_last = 1.0;
-                pap_last = 4.0;
+                if (MIXED) {
+                    const double sn = 1.0 / sqrt(tot.g);
+                    if (nupd) beta = (tot.g * s * s * inv_rr) * (sn / s);
+                    s = sn;
+                    fresh = true;
+                    rr_last = 1.0;
+                    pap_last = 4.0;
+                } else {   // a warm start
+                    rr_last = tot.g;
+                    pap_last = 4.0 * tot.g;
+                }
             }
         }
         if (!ok || dead) flag = RF_ABORT;
         if (lane == 0) {
-            if (MIXED) B.sc.cf = (float)c;
-            else B.sc.c = c;
-            B.sc.flag = flag;
+            if (MIXED) {
+                B.sc.cf = make_float2((float)(next == X_PAP ? beta : alpha), __int_as_float(flag));
+            } else {
+                B.sc.alpha = alpha;
+                B.sc.beta = beta;
+                B.sc.flag = flag;
+            }
             B.sc.s = s;
         }
         if (all) bar_sync_n(5, blockDim.x);
         else bar_sync_n(3, nth);
         if constexpr (MS) {
-            const bool give_up = !all && flag == RF_ABORT && next == X_RR;   // in <p, A p>: the shift warps wait for |r|^2
             if (step) {   // the shifts' recurrences (k_cg_multishift's), lane i shift i
-                const double b_new = tot / rr_old;
+                const double b_new = tot.g * inv_old;
                 if (act) {
-                    const double zn = zs * zp * a_last / (a_now * b_last * (zp - zs) + zp * a_last * (1.0 + M->d[lane] * a_now));
+                    const double zn = zs * zp * a_last / (a_now * b_now * (zp - zs) + zp * a_last * (1.0 + M->d[lane] * a_now));
                     const double q = zn / zs;
                     S->a[lane] = a_now * q;
                     S->b[lane] = b_new * q * q;
                     S->z[lane] = zn;
                     zp = zs;
                     zs = zn;
-                    act = !(zn * zn * tot < tol);
+                    act = !(zn * zn * tot.g < tol);
                     S->state[lane] = act ? 2 : 1;
                 } else {
                     S->state[lane] = 0;
                 }
                 a_last = a_now;
-                b_last = b_new;
+                b_now = b_new;
             }
-            if (give_up) bar_arrive_n(5, blockDim.x);
-            if (all || give_up) {
+            if (all) {
+                a_now = alpha;
                 if (lane == 0) S->flag[round & 1] = flag;
                 round++;
                 bar_arrive_n(4, blockDim.x - 32 * nw);
@@ -677,6 +790,7 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
         if (flag >= RF_STOP) break;
         // off the way from one exchange to the next
         inv_rr = 1.0 / rr;
+        if (!MIXED && alpha != 0.0) inv_a = 1.0 / alpha;
         maxrr = fmax(maxrr, rr);
         thr = fmax(P.delta2 * maxrr, tol * s * s);
     }
@@ -719,28 +833,37 @@ __device__ __forceinline__ Site col_site(const Column& c, int L1, int L2, int j)
     q.xm2 = q.i2 == 0 ? q.x + (V - L1) : q.x - L1;
     return q;
 }
-// workers: the thread's partial of exchange seq
-__device__ __forceinline__ void put_part(ResBlock& B, double s) {
-    B.part[threadIdx.x - 32] = s;
+// workers: the thread's partials of the coming exchange
+__device__ __forceinline__ void put_part(ResBlock& B, double g) {
+    B.part[0][threadIdx.x - 32] = g;
     bar_arrive_n(1, B.nwk + 32);
 }
-// Workers: the end of an exchange.  A warp whose wait for a face gave up (!ok)
-// leaves a note that the scalar warp finds at the next exchange and turns into
-// RF_ABORT for the whole block, so that all its threads leave at the same barrier.
-__device__ __forceinline__ int wait_scalar(ResBlock& B, bool ok, bool all = false) {
+__device__ __forceinline__ void put_part(ResBlock& B, double g, double d) {
+    B.part[1][threadIdx.x - 32] = d;
+    put_part(B, g);
+}
+// A warp whose wait for a face gave up leaves a note that the scalar warp finds at a
+// later sum and turns into RF_ABORT for the whole block, so that all its threads leave at
+// the same barrier.
+__device__ __forceinline__ void note(ResBlock& B, bool ok) {
     if (!ok) *(volatile int*)&B.abort = 1;
+}
+// workers: the end of a sum
+template <bool MIXED>
+__device__ __forceinline__ int wait_scalar(ResBlock& B, bool all = false) {
     if (all) bar_sync_n(5, blockDim.x);   // MS: with the shift warps
     else bar_sync_n(3, B.nwk + 32);
-    return *(volatile int*)&B.sc.flag;
+    if constexpr (MIXED) return __float_as_int(B.sc.cf.y);
+    else return B.sc.flag;
 }
 
 // Workers: the FP64 true residual b - (A + mu2) x, after x += x32 / s (add), and,
 // where the solve goes on, the FP32 residual for the next iteration, left in x32
 // (the caller takes it and clears x32).  The stencils read other blocks' x and
-// t64, so an exchange follows each of them.  Runs a few times per solve, with
-// the iteration's registers put away in shared memory (t) or read again (links).
+// t64, so an exchange follows each of them.  Runs a few times per solve, between
+// iterations, when only shared memory holds anything.
 template <bool MIXED>
-__device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x32, unsigned& seq, bool add) {
+__device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x32, bool add) {
     const Column c = column_of(B);
     const int nwk = B.nwk, L1 = B.rep.L1, L2 = B.rep.L2;
     const long long V = (long long)L1 * L2, o2 = 2 * B.rep.off;
@@ -763,9 +886,8 @@ __device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x3
         }
         __threadfence();
         __syncwarp();
-        put_part(B, 0.0);
-        ++seq;
-        if (wait_scalar(B, true) == RF_ABORT) return RF_ABORT;
+        put_part(B, 0.0, 0.0);
+        if (wait_scalar<MIXED>(B) == RF_ABORT) return RF_ABORT;
     }
 #pragma unroll 1
     for (int j = 0; j < c.h; j++) {
@@ -774,9 +896,8 @@ __device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x3
     }
     __threadfence();
     __syncwarp();
-    put_part(B, 0.0);
-    ++seq;
-    if (wait_scalar(B, true) == RF_ABORT) return RF_ABORT;
+    put_part(B, 0.0, 0.0);
+    if (wait_scalar<MIXED>(B) == RF_ABORT) return RF_ABORT;
     double n = 0.0;
 #pragma unroll 1
     for (int j = 0; j < c.h; j++) {
@@ -788,9 +909,8 @@ __device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x3
         st_d(r64, V, q.x, rv);
         n += norm2(rv.a) + norm2(rv.b);
     }
-    put_part(B, n);
-    ++seq;
-    const int flag = wait_scalar(B, true);
+    put_part(B, n, 0.0);
+    const int flag = wait_scalar<MIXED>(B);
     if (flag != RF_GO || !MIXED) return flag;
     const double s = B.sc.s;
 #pragma unroll 1
@@ -805,7 +925,7 @@ __device__ __forceinline__ int res_update(const ResP& P, ResBlock& B, float4* x3
 // Workers: |b|^2 and (mixed) the first FP32 residual, left in x32.  x = 0 without a
 // guess where the solve adds to it or has nothing to do.
 template <bool MIXED, bool MS = false>
-__device__ __forceinline__ int res_begin(const ResP& P, ResBlock& B, float4* x32, unsigned& seq) {
+__device__ __forceinline__ int res_begin(const ResP& P, ResBlock& B, float4* x32) {
     const Column c = column_of(B);
     const int nwk = B.nwk, L1 = B.rep.L1;
     const long long V = (long long)L1 * B.rep.L2, o2 = 2 * B.rep.off;
@@ -815,9 +935,8 @@ __device__ __forceinline__ int res_begin(const ResP& P, ResBlock& B, float4* x32
         const long long g = o2 + c.g0 + (long long)j * L1;
         acc += norm2(__ldg(P.b + g)) + norm2(__ldg(P.b + V + g));
     }
-    put_part(B, acc);
-    ++seq;
-    const int flag = wait_scalar(B, true, MS);
+    put_part(B, acc, 0.0);
+    const int flag = wait_scalar<MIXED>(B, MS);
     if (flag == RF_ABORT || flag == RF_UPD) return flag;
     const double2 z = make_double2(0, 0);
     const double s = B.sc.s;
@@ -841,7 +960,7 @@ __device__ __forceinline__ int res_begin(const ResP& P, ResBlock& B, float4* x32
 }
 
 // Workers, FP64: x (+)= the solve's, and g5Dw x, which reads other blocks' x.
-__device__ __forceinline__ void res_finish(const ResP& P, ResBlock& B, const double4x* xs, unsigned& seq) {
+__device__ __forceinline__ void res_finish(const ResP& P, ResBlock& B, const double4x* xs) {
     const Column c = column_of(B);
     const int nwk = B.nwk, L1 = B.rep.L1, L2 = B.rep.L2;
     const long long V = (long long)L1 * L2, o2 = 2 * B.rep.off;
@@ -859,9 +978,8 @@ __device__ __forceinline__ void res_finish(const ResP& P, ResBlock& B, const dou
     }
     __threadfence();
     __syncwarp();
-    put_part(B, 0.0);
-    ++seq;
-    if (wait_scalar(B, true) == RF_ABORT || !P.want_g5) return;
+    put_part(B, 0.0, 0.0);
+    if (wait_scalar<false>(B) == RF_ABORT || !P.want_g5) return;
 #pragma unroll 1
     for (int j = 0; j < c.h; j++) {
         const Site q = col_site(c, L1, L2, j);
@@ -910,15 +1028,20 @@ __device__ __forceinline__ void res_place(ResBlock& B, int warp) {
     }
 }
 
+// Returns the number of halo exchanges so far.
 template <class R, int K, bool CL, bool MS = false>
 __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char* dyn, unsigned seq,
                                                V4<R>* rbuf = nullptr) {   // MS: r for the shift warps, two copies in turn
     constexpr bool MIXED = std::is_same<R, float>::value;
+    constexpr int BOX = ResSm<R, K>::BOX;
+    constexpr bool PK = kPacked<K, CL>;
+    constexpr bool OLD = K * sizeof(R) <= 8;   // registers for r before the last update, so that p can wait
     const int nwk = B.nwk, lane = threadIdx.x & 31;
     V4<R>* xs = reinterpret_cast<V4<R>*>(dyn) + (threadIdx.x - 32);   // x: row j at xs[j * nwk]
-    V4<R>* ps = xs + K * nwk;                                         // the search direction likewise
-    V4<R>* ts = ps + K * nwk;                                         // mixed: t during an update
-    V2<R>* box = reinterpret_cast<V2<R>*>(dyn + (size_t)nwk * ResSm<R, K>::ARRAYS * K * sizeof(V4<R>));
+    V4<R>* ps = xs + K * nwk;                                         // p and q likewise: A p (FP64), or t between updates (mixed)
+    V4<R>* qs = ps + K * nwk;
+    V2<R>* box0 = reinterpret_cast<V2<R>*>(dyn + (size_t)nwk * 3 * K * sizeof(V4<R>));
+    V2<R>* box1 = box0 + (nwk >> 5) * BOX;
     if (lane == 0) res_place<R, K, CL>(B, (threadIdx.x >> 5) - 1);
     __syncwarp();
     Tile T;
@@ -930,30 +1053,36 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
         T.er = lane == T.w - 1;
         T.srcR = min(lane + 1, 31);
         T.srcL = lane < T.w ? max(lane - 1, 0) : 31;   // lanes past the tile take lane 31's zero
-        constexpr int BOX = ResSm<R, K>::BOX;
         const WarpFace& F = B.face[(threadIdx.x >> 5) - 1];
         T.xto = F.warp[T.el ? 0 : 1] < 0 ? -1 : F.warp[T.el ? 0 : 1] * BOX + (T.el ? K : 0);
         T.dto = F.warp[2] < 0 ? -1 : F.warp[2] * BOX + 2 * K + 32 + lane;
         T.uto = F.warp[3] < 0 ? -1 : F.warp[3] * BOX + 2 * K + lane;
+        T.W = &F;
+        Slots<R, K, CL>::init(T);
+        const int side = Slots<R, K, CL>::side();
+        T.rx = T.h > 0 && lane < 2 * K && F.warp[side] < 0 && lane - side * K < T.h;
+        T.rd = T.h > 0 && T.dto < 0;
+        T.ru = T.h > 0 && T.uto < 0;
     }
-    const WarpFace& W = B.face[(threadIdx.x >> 5) - 1];
+    // the slots of the two exchanges of an iteration (in a cluster WarpFace::to holds addresses)
+    const u64 from1 = B.C.slots, from0 = from1 + (u64)B.C.nslots * 16, to1 = CL ? 0 : from1, to0 = to1 + (u64)B.C.nslots * 16;
+    int* const err = B.C.err;
     const V4<R> zero = mk4<R>(0, 0, 0, 0);
 #pragma unroll
-    for (int j = 0; j < K; j++) {
-        xs[j * nwk] = ps[j * nwk] = zero;
-        if (MIXED) ts[j * nwk] = zero;
-    }
-    int flag = res_begin<MIXED, MS>(P, B, reinterpret_cast<float4*>(xs), seq);
+    for (int j = 0; j < K; j++) xs[j * nwk] = ps[j * nwk] = qs[j * nwk] = zero;
+    int flag = res_begin<MIXED, MS>(P, B, reinterpret_cast<float4*>(xs));
     bool first = true;
     V2<R> u1[K], u2[K];
     V4<R> r[K], t[K], w[K];
-    R alpha = 0;
+    V4<R> ro[K];   // FP64: r before the last update
+    R alpha = 0, beta = 0;
     const R m2 = (R)B.rep.m2, mu2 = (R)P.mu2;
+    int m = 0;   // MS: iterations
     for (;;) {
         const double2* src = P.b;
         if (flag != RF_GO) {
             if (flag != RF_UPD) return seq;
-            flag = res_update<MIXED>(P, B, reinterpret_cast<float4*>(xs), seq, !first);
+            flag = res_update<MIXED>(P, B, reinterpret_cast<float4*>(xs), !first);
             if (flag != RF_GO) return seq;
             src = P.r64;
         }
@@ -962,9 +1091,9 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
 #pragma unroll
         for (int j = 0; j < K; j++) {
             u1[j] = u2[j] = mk(R(0), R(0));
-            w[j] = zero;
+            w[j] = ro[j] = zero;
             if constexpr (MIXED) {
-                t[j] = ts[j * nwk];
+                t[j] = qs[j * nwk];
                 r[j] = xs[j * nwk];
                 xs[j * nwk] = zero;
             } else {
@@ -981,69 +1110,112 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
                 }
             }
         }
-        for (;;) {
-            {
-                R f = 0;
+        alpha = beta = 0;
+        if constexpr (MIXED) {
+            for (;;) {
+                {
+                    R f = 0;
 #pragma unroll
-                for (int j = 0; j < K; j++) f += norm4<R>(r[j]);
-                put_part(B, (double)f);
-                ++seq;
-            }
-            stencil_inner<R, K, CL>(T, W, r, u1, u2, m2, box, B.C, seq, w);
-            bar_sync_n(2, nwk);
-            bool ok = stencil_faces<R, K, CL>(T, W, u1, u2, box, B.C, seq, w, [&]() {   // x += alpha p of the last iteration
-#pragma unroll
-                for (int j = 0; j < K; j++) xs[j * nwk] = axpy4<R>(alpha, ps[j * nwk], xs[j * nwk]);
-            });
-            flag = wait_scalar(B, ok, MS);
-            if (flag != RF_GO) break;
-            const R beta = MIXED ? (R)B.sc.cf : (R)B.sc.c;
-            {
-                R f = 0;
-#pragma unroll
-                for (int j = 0; j < K; j++) {
-                    t[j] = axpy4<R>(beta, t[j], w[j]);
-                    f += norm4<R>(t[j]);
+                    for (int j = 0; j < K; j++) f += norm4<R, PK>(r[j]);
+                    put_part(B, (double)f);
                 }
-                double d = (double)f;
-                if (mu2 != R(0)) {   // with a shift <p, A p> needs p now, else it is formed during the exchange
-                    f = 0;
+                ++seq;   // w = g5Dw r
+                stencil_inner<R, K, CL>(T, r, u1, u2, m2, box0, to0, seq, w);
+                bar_sync_n(2, nwk);
+                note(B, stencil_faces<R, K, CL>(T, u1, u2, box0, from0, err, seq, w, [&]() {   // x += alpha p of the last iteration
+#pragma unroll
+                    for (int j = 0; j < K; j++) xs[j * nwk] = axpy4<R, PK>(alpha, ps[j * nwk], xs[j * nwk]);
+                }));
+                flag = wait_scalar<MIXED>(B);
+                if (flag != RF_GO) break;
+                beta = B.sc.cf.x;
+                {
+                    R f = 0;
 #pragma unroll
                     for (int j = 0; j < K; j++) {
-                        const V4<R> pn = axpy4<R>(beta, ps[j * nwk], r[j]);
-                        ps[j * nwk] = pn;
-                        f += norm4<R>(pn);
+                        t[j] = axpy4<R, PK>(beta, t[j], w[j]);
+                        f += norm4<R, PK>(t[j]);
                     }
-                    d += P.mu2 * (double)f;
+                    double d = (double)f;
+                    if (mu2 != R(0)) {   // with a shift <p, A p> needs p now, else it is formed during the exchange
+                        f = 0;
+#pragma unroll
+                        for (int j = 0; j < K; j++) {
+                            const V4<R> pn = axpy4<R, PK>(beta, ps[j * nwk], r[j]);
+                            ps[j * nwk] = pn;
+                            f += norm4<R, PK>(pn);
+                        }
+                        d += P.mu2 * (double)f;
+                    }
+                    put_part(B, d);
                 }
-                put_part(B, d);
-                ++seq;
-            }
-            stencil_inner<R, K, CL>(T, W, t, u1, u2, m2, box, B.C, seq, w);
-            bar_sync_n(2, nwk);
-            ok = stencil_faces<R, K, CL>(T, W, u1, u2, box, B.C, seq, w, [&]() {
-                if (mu2 == R(0))
+                ++seq;   // w = g5Dw t
+                stencil_inner<R, K, CL>(T, t, u1, u2, m2, box1, to1, seq, w);
+                bar_sync_n(2, nwk);
+                note(B, stencil_faces<R, K, CL>(T, u1, u2, box1, from1, err, seq, w, [&]() {
+                    if (mu2 == R(0))
 #pragma unroll
-                    for (int j = 0; j < K; j++) ps[j * nwk] = axpy4<R>(beta, ps[j * nwk], r[j]);
-            });
-            if (wait_scalar(B, ok) == RF_ABORT) {
-                if (MS) bar_arrive_n(5, blockDim.x);   // the shift warps wait there
-                return seq;
-            }
-            alpha = MIXED ? (R)B.sc.cf : (R)B.sc.c;
+                        for (int j = 0; j < K; j++) ps[j * nwk] = axpy4<R, PK>(beta, ps[j * nwk], r[j]);
+                }));
+                if (wait_scalar<MIXED>(B) == RF_ABORT) return seq;
+                alpha = B.sc.cf.x;
 #pragma unroll
-            for (int j = 0; j < K; j++) {
-                if (mu2 != R(0)) w[j] = axpy4<R>(mu2, ps[j * nwk], w[j]);
-                r[j] = axpy4<R>(-alpha, w[j], r[j]);
-                if constexpr (MS) rbuf[(((seq >> 1) & 1) * K + j) * nwk + threadIdx.x - 32] = r[j];
+                for (int j = 0; j < K; j++) {
+                    if (mu2 != R(0)) w[j] = axpy4<R, PK>(mu2, ps[j * nwk], w[j]);
+                    r[j] = axpy4<R, PK>(-alpha, w[j], r[j]);
+                }
             }
-        }
-        alpha = 0;
-        if constexpr (MIXED) {
 #pragma unroll
-            for (int j = 0; j < K; j++) ts[j * nwk] = t[j];
+            for (int j = 0; j < K; j++) qs[j * nwk] = t[j];
         } else {
-            if (flag == RF_FIN) res_finish(P, B, xs, seq);
+            bool adv = false;   // an iteration's p and x are still to be formed
+            for (;;) {
+                ++seq;   // t = g5Dw r
+                stencil_inner<R, K, CL>(T, r, u1, u2, m2, box0, to0, seq, t);
+                bar_sync_n(2, nwk);
+                R g = 0, d = 0;
+                bool ok = stencil_faces<R, K, CL>(T, u1, u2, box0, from0, err, seq, t, [&]() {
+#pragma unroll
+                    for (int j = 0; j < K; j++) g += norm4<R, PK>(r[j]);
+                });
+#pragma unroll
+                for (int j = 0; j < K; j++) d += norm4<R, PK>(t[j]);
+                put_part(B, (double)g, (double)d);
+                ++seq;   // w = g5Dw t
+                stencil_inner<R, K, CL>(T, t, u1, u2, m2, box1, to1, seq, w);
+                bar_sync_n(2, nwk);
+                ok &= stencil_faces<R, K, CL>(T, u1, u2, box1, from1, err, seq, w, []() {});
+                note(B, ok);
+                if (adv) {   // p = r_old + beta p, x += alpha p
+#pragma unroll
+                    for (int j = 0; j < K; j++) {
+                        V4<R> pn = ps[j * nwk];
+                        if constexpr (OLD) ps[j * nwk] = pn = axpy4<R, PK>(beta, pn, ro[j]);
+                        xs[j * nwk] = axpy4<R, PK>(alpha, pn, xs[j * nwk]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < K; j++) {
+                    if (mu2 != R(0)) w[j] = axpy4<R, PK>(mu2, r[j], w[j]);
+                    if constexpr (OLD) ro[j] = r[j];
+                    t[j] = qs[j * nwk];
+                }
+                flag = wait_scalar<MIXED>(B, MS);
+                if (flag != RF_GO) break;
+                alpha = (R)B.sc.alpha;
+                beta = (R)B.sc.beta;
+                adv = true;
+                m++;
+#pragma unroll
+                for (int j = 0; j < K; j++) {   // q = A r + beta q, r -= alpha q
+                    const V4<R> q = axpy4<R, PK>(beta, t[j], w[j]);
+                    qs[j * nwk] = q;
+                    if constexpr (!OLD) ps[j * nwk] = axpy4<R, PK>(beta, ps[j * nwk], r[j]);
+                    r[j] = axpy4<R, PK>(-alpha, q, r[j]);
+                    if constexpr (MS) rbuf[((m & 1) * K + j) * nwk + threadIdx.x - 32] = r[j];
+                }
+            }
+            if (flag == RF_FIN) res_finish(P, B, xs);
             return seq;
         }
     }
@@ -1063,20 +1235,20 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_cg(const __grid
         B.C.err = &P.ctl->err;
         if constexpr (CL) {
             B.C.psum = smem_u32(dyn + ResSm<R, K>::bytes((blockDim.x >> 5) - 1));
-            B.C.slots = B.C.psum + 2 * kResCluster * 16;
+            B.C.slots = B.C.psum + 4 * kResCluster * 16;
         } else {
             B.C.slots = (u64)(P.slots + (size_t)team * P.nb * 2 * P.nslots);
-            B.C.psum = (u64)(P.psum + (size_t)team * 2 * P.nb * P.nb);
-            B.C.acc = P.acc + 32 * team;
+            B.C.psum = (u64)(P.psum + (size_t)team * 4 * P.nb);
+            B.C.acc = P.acc + kResAcc * team;
         }
     }
     if constexpr (CL) {   // no slot carries a tag yet
         ulonglong2* sl = reinterpret_cast<ulonglong2*>(dyn + ResSm<R, K>::bytes((blockDim.x >> 5) - 1));
-        for (int i = threadIdx.x; i < 2 * (kResCluster + P.nslots); i += blockDim.x) sl[i] = make_ulonglong2(0, 0);
+        for (int i = threadIdx.x; i < 4 * kResCluster + 2 * P.nslots; i += blockDim.x) sl[i] = make_ulonglong2(0, 0);
         cooperative_groups::this_cluster().sync();
     }
     unsigned seq = 0;
-    ulonglong2 base0 = make_ulonglong2(0, 0), base1 = base0;
+    u64 base0 = 0, base1 = 0;
     for (int next = team; next < P.nrep;) {
         if (threadIdx.x == 0) {
             B.rep = P.reps ? P.reps[next] : P.rep0;
@@ -1087,14 +1259,14 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_cg(const __grid
         else seq = res_worker<R, K, CL>(P, B, dyn, seq);
         if (CL || P.nteams >= P.nrep) break;
         __syncthreads();
-        if (B.sc.flag == RF_ABORT) break;
-        ++seq;   // the team's first block takes the next system for the team
-        if (threadIdx.x < 32) {
+        if ((std::is_same<R, float>::value ? __float_as_int(B.sc.cf.y) : B.sc.flag) == RF_ABORT) break;
+        if (threadIdx.x < 32) {   // the team's first block takes the next system for the team
+            ++seq;
             int n = 0;
             if (B.C.rank == 0 && threadIdx.x == 0) n = atomicAdd(P.queue, 1);
-            double tot = (double)__shfl_sync(0xffffffffu, n, 0);
-            if (P.nb > 1 && !team_sum_slots(B.C, seq, tot, tot)) tot = (double)P.nrep;
-            if (threadIdx.x == 0) B.next = tot;
+            Sums tot{(double)__shfl_sync(0xffffffffu, n, 0), 0.0};
+            if (P.nb > 1 && !team_sum_slots<1>(B.C, seq, tot, tot)) tot.g = (double)P.nrep;
+            if (threadIdx.x == 0) B.next = tot.g;
         }
         __syncthreads();
         next = P.nteams + (int)B.next;
@@ -1111,7 +1283,7 @@ inline int res_slots(const ResPlan& p, int per) { return per * (2 * p.wy * p.K +
 template <class R, int K>
 static size_t res_smem(const ResPlan& p) {
     return ResSm<R, K>::bytes(p.wx * p.wy) +
-           (p.cl ? sizeof(ulonglong2) * 2 * (kResCluster + res_slots(p, Num<R>::SLOTS)) : 0);
+           (p.cl ? sizeof(ulonglong2) * (4 * kResCluster + 2 * res_slots(p, Num<R>::SLOTS)) : 0);
 }
 
 template <class R, int K>

@@ -23,7 +23,7 @@ int res_f64_launch(const ResP& P, const ResPlan& plan, cudaStream_t stream) {
 // and the block's remaining warps update them,
 //   x_i += a_i p_i,  p_i = z_i r + b_i p_i,
 // one iteration behind the residual they read.  Nothing in the base system waits for
-// them except at the next |r|^2: they join that barrier, which keeps the two copies of r
+// them except at the next sum: they join that barrier, which keeps the two copies of r
 // apart.  Shared memory holds about 3000 site-shifts a block, so a lattice is spread
 // over at least that many blocks: 128^2 with 12 shifts over 128 of them.
 template <int K>
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1)
     __syncthreads();
     double4x* rbuf = reinterpret_cast<double4x*>(dyn + ResSm<double, K>::bytes(M.nw));
     double4x* sx = rbuf + 2 * K * 32 * M.nw;
-    ulonglong2 base0 = make_ulonglong2(0, 0), base1 = base0;
+    u64 base0 = 0, base1 = 0;
     if (threadIdx.x < 32) res_scalar<false, false, true>(P, B, 0, base0, base1, &M, &S);
     else if ((int)threadIdx.x < 32 * (M.nw + 1)) res_worker<double, K, false, true>(P, B, dyn, 0, rbuf);
     else res_shifts<K>(P, M, B, S, rbuf, sx);
