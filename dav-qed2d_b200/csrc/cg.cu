@@ -203,6 +203,7 @@ __device__ __forceinline__ void finish_solve(const CGP& P, int iters, bool conv,
 }
 
 #define FOR_TILES(q) FOR_RANGE(q, P.g, TR)
+#define FOR_TILES_BACK(q) FOR_RANGE_BACK(q, P.g, TR)
 
 // ---------------------------------------------------------------------------
 // FP64 persistent CG
@@ -472,9 +473,12 @@ __global__ void __launch_bounds__(TILE, 4) k_cg_mixed(const CGP P) {
             double v[1] = {(double)ft + mu2 * (double)fc};
             if (!reduce_sync<1, RS>(gs, v, P.part, P.ctl->red, smem)) goto done;
             const float alpha = (float)(rr / v[0]);
+            // The second phase runs from the block's last tile to its first: it starts
+            // with what the first phase left in L2, and the next first phase with what
+            // it leaves.  Per iteration 1500^2 78.4 -> 72.4 us, 2048^2 142 -> 137.
             float fr = 0.f;
             if (!kPair) {
-                FOR_TILES(q) {
+                FOR_TILES_BACK(q) {
                     const Pair<float> pc = SpF{qn}.ld(q.x);
                     const Pair<float> a = sten(SpF{P.t32}, SpF{P.t32}.ld(q.x), q, tt_ - TR.lo);
                     Pair<float> xv = SpF{P.x32}.ld(q.x), r = SpF{P.r32}.ld(q.x);
@@ -487,7 +491,7 @@ __global__ void __launch_bounds__(TILE, 4) k_cg_mixed(const CGP P) {
                     fr += norm2(r.a) + norm2(r.b);
                 }
             } else if (pend) {
-                FOR_TILES(q) {   // x += apend p_old, then x += alpha p
+                FOR_TILES_BACK(q) {   // x += apend p_old, then x += alpha p
                     const Pair<float> po = SpF{qo}.ld(q.x), pc = SpF{qn}.ld(q.x);
                     const Pair<float> a = sten(SpF{P.t32}, SpF{P.t32}.ld(q.x), q, tt_ - TR.lo);
                     Pair<float> xv = SpF{P.x32}.ld(q.x), r = SpF{P.r32}.ld(q.x);
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(TILE, 4) k_cg_mixed(const CGP P) {
                     fr += norm2(r.a) + norm2(r.b);
                 }
             } else if (shifted) {
-                FOR_TILES(q) {   // x's update waits for the next iteration
+                FOR_TILES_BACK(q) {   // x's update waits for the next iteration
                     const Pair<float> pc = SpF{qn}.ld(q.x);
                     const Pair<float> a = sten(SpF{P.t32}, SpF{P.t32}.ld(q.x), q, tt_ - TR.lo);
                     Pair<float> r = SpF{P.r32}.ld(q.x);
@@ -512,7 +516,7 @@ __global__ void __launch_bounds__(TILE, 4) k_cg_mixed(const CGP P) {
                     fr += norm2(r.a) + norm2(r.b);
                 }
             } else {
-                FOR_TILES(q) {   // the same without a shift (a + 0 p = a exactly)
+                FOR_TILES_BACK(q) {   // the same without a shift (a + 0 p = a exactly)
                     const Pair<float> a = sten(SpF{P.t32}, SpF{P.t32}.ld(q.x), q, tt_ - TR.lo);
                     Pair<float> r = SpF{P.r32}.ld(q.x);
                     r.a = r.a - alpha * a.a;

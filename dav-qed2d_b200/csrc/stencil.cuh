@@ -74,6 +74,7 @@ __device__ __forceinline__ Site site_at(const Lat& g, int t1, int t2, int t) {
 // the block's contiguous tile range [lo, hi) and the coordinates of tile lo
 struct TileRange {
     int lo, hi, s1, s2, nt1;
+    int e1, e2;   // the last tile's
 };
 __device__ __forceinline__ TileRange tile_range(long long ntiles, int nt1, int per_block, int b) {
     TileRange r;
@@ -82,11 +83,19 @@ __device__ __forceinline__ TileRange tile_range(long long ntiles, int nt1, int p
     r.s2 = r.lo / nt1;
     r.s1 = r.lo - r.s2 * nt1;
     r.nt1 = nt1;
+    r.e2 = (r.hi - 1) / nt1;
+    r.e1 = r.hi - 1 - r.e2 * nt1;
     return r;
 }
 #define FOR_RANGE(q, G, R)                                                                                    \
     for (int tt_ = (R).lo, t1_ = (R).s1, t2_ = (R).s2; tt_ < (R).hi;                                        \
          ++tt_, (++t1_ == (R).nt1 ? (t1_ = 0, ++t2_) : 0))                                                    \
+        if (const Site q = site_at((G), t1_, t2_, threadIdx.x); q.ok)
+
+// the same from the last tile to the first
+#define FOR_RANGE_BACK(q, G, R)                                                                               \
+    for (int tt_ = (R).hi - 1, t1_ = (R).e1, t2_ = (R).e2; tt_ >= (R).lo;                                   \
+         --tt_, (t1_-- == 0 ? (t1_ = (R).nt1 - 1, --t2_) : 0))                                                \
         if (const Site q = site_at((G), t1_, t2_, threadIdx.x); q.ok)
 
 // the same for a BX x BY tile visited by BX*BY threads (thread t -> (t % BX, t / BX))
