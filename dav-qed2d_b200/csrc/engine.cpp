@@ -268,12 +268,9 @@ static int md_kick_rhmc(Ctx& c, double* mom, const double2* U, double2* X, const
 // order as separate updates and kicks; the compiler contracts them into FMAs
 // differently in the fused kernel, so results agree to rounding (1e-14 on links
 // after OMF4 trajectories), not bit for bit.  Lattices of whole 32 x 8 tiles
-// (kernel requirement) without an FP32 link copy to refresh.  Measured per
-// OMF4 step: up to 256^2 44.5 -> 34.9 us (fewer launches), 512^2 67.1 -> 49.5,
-// 2048^2 555 -> 516, 4096^2 2082 -> 1942, 8192^2 8274 -> 8179; but 1024^2
-// 112.8 -> 143.4 us, where the separate kernels' links and momenta (48 B/site)
-// stay in the 126 MB L2 and the two buffer pairs (96 B/site) do not -- so not
-// for 2^19 < V <= 2^21 sites.
+// (kernel requirement) without an FP32 link copy to refresh, beyond what the on-chip
+// integration holds.  Two OMF4 steps against the separate kernels: 768^2 185 -> 125 us,
+// 1024^2 231 -> 200, 1440^2 538 -> 379.
 struct GaugePingPong {
     Ctx& c;
     double2* U[2];
@@ -285,7 +282,7 @@ struct GaugePingPong {
         mom[0] = m0;
         U[1] = nullptr;
         mom[1] = nullptr;
-        if (s.U32 || !updt_kick_fits(c) || (c.g.V > (1LL << 19) && c.g.V <= (1LL << 21))) return;
+        if (s.U32 || !updt_kick_fits(c)) return;
         U[1] = c.spinor("md_u_alt");
         mom[1] = c.real2("md_mom_alt");
         on = U[1] && mom[1];
@@ -296,7 +293,7 @@ struct GaugePingPong {
             QTRY(md_links(c, U[cur], mom[cur], eu, s));
             return md_kick_gauge(c, mom[cur], U[cur], ek);
         }
-        QTRY(launch_updt_kick(c, U[cur ^ 1], U[cur], mom[cur ^ 1], mom[cur], eu, ek));
+        QTRY(launch_updt_kick(c, U[cur ^ 1], U[cur], mom[cur ^ 1], mom[cur], eu, ek, cur != 0));
         cur ^= 1;
         return QED2D_OK;
     }

@@ -279,73 +279,117 @@ __global__ void __launch_bounds__(TILE, FERM ? 4 : 6) k_mom_kick(double* __restr
 
 // updt_fld! followed by the pure-gauge kick, in one pass (OMF4! and leapfrog
 // pure gauge alternate the two, src/QED2dHMC.jl:248-305): Uout = e^{i eu mom_in} Uin,
-// mom_out = mom_in + ek F(Uout).  The tile's updated links and the halo the force
-// needs (U1 on rows -1..TY of columns -1..31, U2 on rows -1..TY-1 of columns
-// -1..32) are computed into shared memory, each with the operations of
-// updt_fld!; then the plaquettes of the tile, of the row below and of the
-// column to its left; then the kick with those of k_mom_kick.  Reads Uin and mom_in,
-// writes Uout and mom_out (distinct buffers: neighbours read the old momenta).  Lattices
-// of whole 32 x TY tiles only.  Per site: links in 32 + out 32, momenta in 16 +
-// out 16 (96 B) instead of 80 + 64 B for the two kernels.
-__global__ void __launch_bounds__(TILE) k_updt_kick(double2* __restrict__ Uout, const double2* __restrict__ Uin,
-                                                    double* __restrict__ mom_out, const double* __restrict__ mom_in, Lat g,
-                                                    double beta, double eu, double ek) {
-    constexpr int R1 = TY + 2, C1 = TX + 1;   // U1: rows -1..TY, columns -1..31
-    constexpr int R2 = TY + 1, C2 = TX + 2;   // U2: rows -1..TY-1, columns -1..32
-    __shared__ double2 s1[R1 * C1], s2[R2 * C2];
-    __shared__ double sv[(TY + 1) * (TX + 1)];   // v on rows -1..TY-1, columns -1..31
-    int t1, t2;
-    if (gridDim.y > 1 || g.L2 <= TY) {
-        t1 = blockIdx.x;
-        t2 = blockIdx.y;
-    } else {
-        const int nt1 = g.L1 / TX;
-        t2 = blockIdx.x / nt1;
-        t1 = blockIdx.x - t2 * nt1;
+// mom_out = mom_in + ek F(Uout), each with the operations of updt_fld! and k_mom_kick.
+// Reads Uin and mom_in, writes Uout and mom_out (distinct buffers: neighbours read the
+// old momenta).  Lattices of whole tiles only.  Per site: links in 32 + out 32, momenta
+// in 16 + out 16 (96 B) instead of 80 + 64 B for the two kernels.
+//
+// A tile is 32 x 8K sites, a thread a column of K: its links and momenta stay in registers
+// from the update to the kick.  What the tile's plaquettes need beyond it (U1 of the rows
+// above and below, U2 of the row below, U2 of the column to the right, both links of the
+// column to the left) is updated again by the warps that `halo` names, a lane a link;
+// neighbouring columns come by shuffle, neighbouring warps' rows through shared memory.
+//
+// Bound by memory: with 16 rows a tile (K = 2) 1/8 more links are updated than the lattice
+// has.  With tiles of 8 rows staged in shared memory by a loop over their links (index
+// divisions, wrapping and 64-bit addresses for each) it was bound by issue: 505 warp
+// instructions for 32 sites, 86 of them FP64, at 68% of the issue slots and 48% of the
+// DRAM rate.  Two OMF4 steps (10 passes and a kick) on a B200: 768^2 185 -> 125 us, 1024^2
+// 231 -> 200, 2048^2 1043 -> 731, 4096^2 3924 -> 2732 (about 6.3 TB/s); K = 1 at 4096^2
+// 2948, K = 4 (spills, idle halo warps) 3195.  Passes alternate between upward and
+// downward (`back`), so that the next one starts with what the last left in L2: 1024^2
+// 211 -> 200, 2048^2 755 -> 731, 4096^2 2770 -> 2732.
+template <int K>
+__global__ void __launch_bounds__(TILE, K == 1 ? 6 : 4)
+    k_updt_kick(double2* __restrict__ Uout, const double2* __restrict__ Uin, double* __restrict__ mom_out,
+                const double* __restrict__ mom_in, Lat g, double beta, double eu, double ek, int back) {
+    constexpr int W = TILE / 32, H = W * K;   // warps, rows of a tile
+    __shared__ double2 s_low[W + 1][TX];      // U1 of every warp's lowest row, and of the row above the tile
+    __shared__ double2 s_b2[TX + 1];          // U2 of the row below, columns 0..32
+    __shared__ double2 s_r2[H], s_l1[H + 1], s_l2[H];   // U2 of column 32; U1, U2 of column -1
+    __shared__ double s_top[W + 1][TX];       // v of the row below the tile and of every warp's highest row
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nt1 = g.L1 / TX;
+    int t1 = blockIdx.x, t2 = blockIdx.y;
+    if (gridDim.y == 1 && g.L2 > H) {   // more rows of tiles than a grid's second dimension holds
+        t2 = t1 / nt1;
+        t1 -= t2 * nt1;
     }
-    const long long V = g.V;
-    const int i10 = t1 * TX, i20 = t2 * TY;
-    // the updated link of direction mu at tile position (row, col), periodic
-    auto upd = [&](int mu, int row, int col, bool own) {
-        int i1 = i10 + col, i2 = i20 + row;
-        i1 = i1 < 0 ? i1 + g.L1 : (i1 >= g.L1 ? i1 - g.L1 : i1);
-        i2 = i2 < 0 ? i2 + g.L2 : (i2 >= g.L2 ? i2 - g.L2 : i2);
-        const long long x = i1 + (long long)g.L1 * i2 + (mu ? V : 0);
+    if (back) t2 = g.L2 / H - 1 - t2;
+    const int L1 = g.L1, V = L1 * g.L2;   // 2V < 2^31 is checked at context creation
+    const int x0 = t1 * TX, y0 = t2 * H;
+    const int xl = x0 == 0 ? L1 - 1 : x0 - 1, xr = x0 + TX == L1 ? 0 : x0 + TX;
+    const int yb = y0 == 0 ? g.L2 - 1 : y0 - 1, ya = y0 + H == g.L2 ? 0 : y0 + H;
+    auto updated = [&](double2 u, double m) {
         double s, c;
-        sincos(eu * mom_in[x], &s, &c);
-        const double2 u = cmul(make_double2(c, s), Uin[x]);
-        if (own) Uout[x] = u;
-        return u;
+        sincos(eu * m, &s, &c);
+        return cmul(make_double2(c, s), u);
     };
-    for (int e = threadIdx.x; e < R1 * C1; e += TILE) {
-        const int row = e / C1 - 1, col = e % C1 - 1;
-        s1[e] = upd(0, row, col, row >= 0 && row < TY && col >= 0);
+    // own links
+    const int x = x0 + lane + L1 * (y0 + w * K);
+    double2 u1[K], u2[K];
+    double m1[K], m2[K];
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        const int i = x + j * L1;
+        u1[j] = Uin[i];
+        u2[j] = Uin[i + V];
+        m1[j] = mom_in[i];
+        m2[j] = mom_in[i + V];
     }
-    for (int e = threadIdx.x; e < R2 * C2; e += TILE) {
-        const int row = e / C2 - 1, col = e % C2 - 1;
-        s2[e] = upd(1, row, col, row >= 0 && col >= 0 && col < TX);
+    // halo: rows 0 U1 above, 1 U1 below, 2 U2 below; from 3 on the columns' links, a lane each
+    int hx = -1;
+    double2* to = nullptr;
+    if (w < 3) {
+        hx = x0 + lane + L1 * (w == 0 ? ya : yb) + (w == 2 ? V : 0);
+        to = w == 0 ? &s_low[W][lane] : w == 2 ? &s_b2[lane] : nullptr;
+    } else {
+        const int i = threadIdx.x - 96;
+        if (i < H) hx = xl + L1 * (y0 + i), to = s_l1 + i;
+        else if (i < 2 * H) hx = xl + L1 * (y0 + i - H) + V, to = s_l2 + i - H;
+        else if (i < 3 * H) hx = xr + L1 * (y0 + i - 2 * H) + V, to = s_r2 + i - 2 * H;
+        else if (i == 3 * H) hx = xl + L1 * ya, to = s_l1 + H;
+        else if (i == 3 * H + 1) hx = xr + L1 * yb + V, to = s_b2 + TX;
     }
+    double2 hu = make_double2(0, 0);
+    if (hx >= 0) {
+        hu = updated(Uin[hx], mom_in[hx]);
+        if (to) *to = hu;
+    }
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        const int i = x + j * L1;
+        u1[j] = updated(u1[j], m1[j]);
+        u2[j] = updated(u2[j], m2[j]);
+        Uout[i] = u1[j];
+        Uout[i + V] = u2[j];
+    }
+    s_low[w][lane] = u1[0];
     __syncthreads();
     // v(y) = beta Im P(y) from U1(y), U2(y + 1), U1(y + 2), U2(y)
-    for (int e = threadIdx.x; e < (TY + 1) * (TX + 1); e += TILE) {
-        const int row = e / (TX + 1) - 1, col = e % (TX + 1) - 1;
-        if (row >= 0 && col >= 0 || row < 0 && col >= 0 || row >= 0 && col < 0) {   // not the corner
-            const double2 u1y = s1[(row + 1) * C1 + col + 1], u1yp2 = s1[(row + 2) * C1 + col + 1];
-            const double2 u2y = s2[(row + 1) * C2 + col + 1], u2yp1 = s2[(row + 1) * C2 + col + 2];
-            sv[e] = beta * plaquette_of(u1y, u2yp1, u1yp2, u2y).y;
-        }
+    double v[K];
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        double2 r = make_double2(__shfl_down_sync(0xffffffffu, u2[j].x, 1), __shfl_down_sync(0xffffffffu, u2[j].y, 1));
+        if (lane == 31) r = s_r2[w * K + j];
+        v[j] = beta * plaquette_of(u1[j], r, j + 1 < K ? u1[j + 1 < K ? j + 1 : j] : s_low[w + 1][lane], u2[j]).y;
+    }
+    s_top[w + 1][lane] = v[K - 1];
+    if (w == 1) {   // the row below
+        s_top[0][lane] = beta * plaquette_of(hu, s_b2[lane + 1], s_low[0][lane], s_b2[lane]).y;
     }
     __syncthreads();
-    const int lx = threadIdx.x & (TX - 1), ly = threadIdx.x >> 5;
-    const long long x = (i10 + lx) + (long long)g.L1 * (i20 + ly);
-    const double v = sv[(ly + 1) * (TX + 1) + lx + 1];
-    const double F1 = -v + sv[ly * (TX + 1) + lx + 1];
-    const double F2 = v - sv[(ly + 1) * (TX + 1) + lx];
-    mom_out[x] = mom_in[x] + ek * F1;
-    mom_out[x + V] = mom_in[x + V] + ek * F2;
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        const int i = x + j * L1;
+        double l = __shfl_up_sync(0xffffffffu, v[j], 1);
+        if (lane == 0)
+            l = beta * plaquette_of(s_l1[w * K + j], u2[j], s_l1[w * K + j + 1], s_l2[w * K + j]).y;
+        mom_out[i] = m1[j] + ek * (-v[j] + (j > 0 ? v[j > 0 ? j - 1 : 0] : s_top[w][lane]));
+        mom_out[i + V] = m2[j] + ek * (v[j] - l);
+    }
 }
 
-// y = a x + b z (complex scalars; z may alias y)
 __global__ void k_zaxpby(double2* y, double2 a, const double2* x, double2 b, const double2* z,
                          long long n) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -558,9 +602,13 @@ int launch_random_normal(Ctx& c, double* out, int64_t n, uint64_t seed, uint32_t
 bool updt_kick_fits(const Ctx& c) { return c.g.L1 % TX == 0 && c.g.L2 % TY == 0; }
 
 int launch_updt_kick(Ctx& c, double2* Uout, const double2* Uin, double* mom_out, const double* mom_in, double eu,
-                     double ek) {
+                     double ek, bool back) {
     if (!updt_kick_fits(c)) return QED2D_ERR_UNSUPPORTED;
-    k_updt_kick<<<tiles_grid2(c.g), TILE, 0, c.stream>>>(Uout, Uin, mom_out, mom_in, c.g, c.beta, eu, ek);
+    const int K = c.g.L2 % (2 * TY) == 0 ? 2 : 1;
+    const unsigned nt1 = c.g.L1 / TX, nt2 = c.g.L2 / (TY * K);
+    const dim3 grid = nt2 <= 65535 ? dim3(nt1, nt2) : dim3(nt1 * nt2);
+    if (K == 2) k_updt_kick<2><<<grid, TILE, 0, c.stream>>>(Uout, Uin, mom_out, mom_in, c.g, c.beta, eu, ek, back);
+    else k_updt_kick<1><<<grid, TILE, 0, c.stream>>>(Uout, Uin, mom_out, mom_in, c.g, c.beta, eu, ek, back);
     return post_launch("k_updt_kick");
 }
 

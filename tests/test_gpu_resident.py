@@ -265,3 +265,10 @@ def test_gauge_md_vs_separate_kernels(L1, L2):
     m2 = torch.from_numpy(np.random.default_rng(5).standard_normal((2, L2, L1))).cuda()
     qed2d.OMF4_(m2, U2, eps, ns, prm, None)
     assert torch.equal(U1, U2) and torch.equal(m1, m2)
+
+
+@pytest.mark.parametrize("L1,L2", [(32, 8888), (64, 4448), (576, 576), (1024, 1000)])
+def test_large_gauge_md_vs_separate_kernels(L1, L2):
+    """The same beyond what fits on chip: one pass per link update and kick, tiles of 8 and of
+    16 rows, one tile across (it is its own neighbour), passes in both directions."""
+    test_gauge_md_vs_separate_kernels(L1, L2)
