@@ -458,6 +458,13 @@ int qed2d_ctx_set_stream(qed2d_ctx* ctx, void* stream) {
     return QED2D_OK;
 }
 
+int qed2d_ctx_bind(qed2d_ctx* ctx, double beta, void* stream) {
+    QCTX(ctx);
+    c.beta = beta;
+    c.stream = (cudaStream_t)stream;
+    return QED2D_OK;
+}
+
 int qed2d_ctx_set_precision(qed2d_ctx* ctx, int precision) {
     QCTX(ctx);
     if (precision < QED2D_PREC_F64 || precision > QED2D_PREC_PLAIN) return bad_arg("unknown precision");

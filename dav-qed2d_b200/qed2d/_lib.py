@@ -45,6 +45,7 @@ SIGNATURES = {
     "qed2d_ctx_destroy": (I, [P]),
     "qed2d_ctx_set_beta": (I, [P, D]),
     "qed2d_ctx_set_stream": (I, [P, P]),
+    "qed2d_ctx_bind": (I, [P, D, P]),
     "qed2d_ctx_set_precision": (I, [P, I]),
     "qed2d_ctx_get_dims": (I, [P, PI, PI]),
     "qed2d_ctx_set_schedule": (I, [P, I, I]),

@@ -98,6 +98,7 @@ int qed2d_ctx_create(int L1, int L2, double beta, qed2d_ctx** out);
 int qed2d_ctx_destroy(qed2d_ctx* ctx);
 int qed2d_ctx_set_beta(qed2d_ctx* ctx, double beta);
 int qed2d_ctx_set_stream(qed2d_ctx* ctx, void* cuda_stream);
+int qed2d_ctx_bind(qed2d_ctx* ctx, double beta, void* cuda_stream);   /* both of these */
 int qed2d_ctx_set_precision(qed2d_ctx* ctx, int precision);
 int qed2d_ctx_get_dims(const qed2d_ctx* ctx, int* L1, int* L2);
 /* Reduction schedule of a persistent solver, selected by `precision`:
