@@ -64,15 +64,14 @@ B_OMF4_STEP = 6 * 64.0 + 5 * 80.0   # one pure-gauge OMF4 step as the reference'
 # figure is reported beside.)
 B_ITER_F32 = 256.0
 B_ITER_F64 = 512.0
-# Measured traffic per site-iteration of k_u_cg_mixed at 4 x 512^2, from one ncu
-# capture of a 100-iteration launch of the tuned kernel (independent replicas,
-# lean reduction, phase-A stencil on r, links staged in shared memory, 32 x 16
-# tiles): DRAM read + write (5.391 GB over 1,048,576 sites x 100) and L1 <-> L2
-# (13.29 GB read + 6.56 GB written); both grow in proportion to the iterations
-# at fixed size
-U_DRAM_PER_SITE_ITER = 51.4
-U_L2_PER_SITE_ITER = 189.3
-U_L2_THROUGHPUT = 0.360   # lts__throughput.avg.pct_of_peak_sustained_elapsed of the same capture
+# Measured traffic per site-iteration of k_res_cg (the on-chip mixed CG) at 4 x 512^2,
+# from one ncu capture of a launch of 4 solves of 362 iterations: DRAM read + write
+# (133 MB over 1,048,576 sites x 362: sources, links and solutions once per solve) and
+# L2 (12.70 GB, halos between blocks and their polls); both grow with the iterations
+U_DRAM_PER_SITE_ITER = 0.35
+U_L2_PER_SITE_ITER = 33.5
+U_L2_THROUGHPUT = 0.090   # lts__throughput.avg.pct_of_peak_sustained_elapsed of the same capture
+U_ISSUE = 0.456           # smsp__issue_active.avg.pct_of_peak_sustained_active
 ENS_NS, ENS_EPS = 10, 0.1   # replica ensemble: leapfrog ns=10, eps=0.1
 CPU_TRAJ = 2                # trajectories of the GPU arm's CPU-baseline sample
 
@@ -276,8 +275,9 @@ def run_configs(qed2d, torch, dev):
     for _ in range(10):
         qed2d.HMC_(U2, 0.1, 10, [], p2, None)   # pure-gauge thermalisation
     c2, sched = {}, {}
-    names = {0: "grid, last block publishes", 1: "grid, every block sums", 2: "one thread-block cluster"}
-    names.update({k + 4: v + "; stencil on r, links in shared memory" for k, v in list(names.items())})
+    # untuned solves that fit keep their state on chip: one cluster (2, 6) or a grid (1, 5)
+    names = {1: "on chip, grid", 2: "on chip, one thread-block cluster"}
+    names.update({k + 4: v for k, v in list(names.items())})
     for prec in ("mixed", "f64", "plain"):
         qed2d.set_precision(prec)
         Uc = U2.clone()
@@ -304,7 +304,7 @@ def run_configs(qed2d, torch, dev):
                                    "solver_layout": {0: "32x8 tiles, one thread per site", 1: "32x8 tiles, two threads per site",
                                                      2: "32x4 tiles, four threads per site",
                                                      3: "32x4 tiles, two threads per site"}.get(
-                                       qed2d.get_multishift_layout(p3), "untuned"),
+                                       qed2d.get_multishift_layout(p3), "on chip, shifts in shared memory"),
                                    "trajectories": 10}
     del U, U2, U3
     # C5
@@ -445,10 +445,7 @@ def run_ours(args):
                     "cg_iterations_per_traj_mean": sum(p[0] for p in per_rep) / (n_traj * len(sizes)),
                     "accepted": sum(p[1] for p in per_rep), "of": n_traj * len(sizes),
                     "timed": f"{n_traj} batched trajectories after 1 warm-up",
-                    "solver": {2: "one launch over all replicas, grid barriers",
-                               3: "one thread-block cluster per replica",
-                               6: "one thread-block cluster per replica, phase-A stencil on r"}.get(eb.schedule,
-                                                                                                    "untuned")}
+                    "solver": "on chip: a team of blocks per replica, one launch per lattice size"}
         del eb, Ue
         torch.cuda.empty_cache()
 
@@ -480,7 +477,8 @@ def run_ours(args):
     traffic = V * sum(its) * U_DRAM_PER_SITE_ITER
     l2_bytes = V * sum(its) * U_L2_PER_SITE_ITER
     l2_peak = l2_copy_peak(torch, dev)
-    roofline = {"kernel": "k_u_cg_mixed", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    roofline = {"kernel": "k_res_cg", "bound": "issue and exchange latency (state on chip)",
+                "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                 "dram_achieved": traffic / t_k / 1e9, "dram_frac": traffic / t_k / 1e9 / peak,
                 "fused_model_achieved": fused_k / t_k / 1e9,
@@ -490,22 +488,16 @@ def run_ours(args):
                        "probe_kind": "best of a copy, an add and a sum on L2-resident buffers in this run "
                                      "(torch kernels; below what the L2 sustains for this kernel's mix)"},
                 "launch_us": t_k * 1e6,
-                "schedule": {0: "last block publishes the sums", 1: "every block sums",
-                             4: "independent replicas (a barrier per replica)",
-                             5: "independent replicas, lean reduction",
-                             7: "independent replicas, lean reduction, TMA-staged stencil operands",
-                             8: "independent replicas, lean reduction, phase-A stencil on r",
-                             9: "independent replicas, lean reduction, phase-A stencil on r, links in shared "
-                                "memory"}.get(
-                                 batch.schedule, "untuned"),
-                "tile_rows": batch.tile_rows,
+                "issue_active": U_ISSUE,
+                "schedule": "on chip: a team of blocks per replica, links and FP32 vectors in registers and "
+                            "shared memory for the whole solve",
                 "note": f"one launch = one solve of all {B} replicas: per replica iterations {min(its)}-{max(its)} "
                         f"x {B_ITER_F32:.0f} B/site + reliable updates {min(upd)}-{max(upd)} x {B_ITER_F64:.0f} "
-                        f"B/site (algorithmic); the {B} x {L}^2 FP32 working set is mostly L2-resident, so the "
+                        f"B/site (algorithmic); the state stays in registers and shared memory, so the "
                         f"algorithmic rate exceeds the DRAM copy bandwidth; traffic = ncu DRAM bytes per "
                         f"site-iteration x the solve's site-iterations (dram_achieved = traffic / time); l2 = "
-                        f"ncu L1<->L2 bytes per site-iteration x site-iterations against an L2-resident copy "
-                        f"measured in this run; neither is saturated: the kernel is latency- and barrier-bound"}
+                        f"ncu L2 bytes per site-iteration x site-iterations (halos, sums and their polls); the "
+                        f"kernel waits for exchanges between blocks and issues in {U_ISSUE:.0%} of its cycles"}
 
     # --- single-chain baselines on the same field and draws as replica 0's first
     # timed step: mixed (no batching), fused FP64, and the plain FP64 GPU path
