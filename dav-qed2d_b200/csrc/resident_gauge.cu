@@ -2,19 +2,20 @@
 // chip for the whole integration (one launch).
 //
 // Tiles, faces and slots as in resident.cuh: a thread holds a column of K sites (links
-// and momenta in registers), so a kick needs two exchanges with the neighbouring tiles
-// and nothing else:
-//   U2 of the first column goes left, U1 of the lowest row down: every site's plaquette;
-//   v of the last column goes right, of the highest row up:       every site's force.
-// Nothing is summed, so a tile waits for its four neighbours only.  A slot is reused
-// two kicks later; its sender has by then the receiver's answer to it (the plaquettes
-// travel against the links), so it has been read.
+// and momenta in registers).  A plaquette needs U1 of the row above the tile and U2 of the
+// column to its right as well; these are carried along (their momenta get the force that
+// their owners compute), so a kick needs one exchange with the neighbouring tiles: the
+// plaquettes' v of the first and last column and of the lowest and highest row.  Nothing
+// is summed, so a tile waits for its four neighbours only.  A slot is sent to again two
+// kicks later; its sender has by then the receiver's v of the kick between, sent after the
+// slot was read.
 //
-// What bounds it: the two exchanges of a kick (about 1000 cycles each through L2), and
-// from about 256^2 on FP64 arithmetic, half of it the two sincos of a link update.
-// OMF4 step (5 link updates, 6 kicks) on a B200 against one kernel per update and kick
-// (launch and L2 round trips, 5.8 us a pass): 32^2 37.6 -> 7.5 us, 128^2 35.0 -> 10.8,
-// 256^2 35.1 -> 15.2, 512^2 49.5 -> 25.3.
+// What bounds it: the exchange of a kick (about 1000 cycles through L2) and the chain of a
+// link update (sincos, plaquette); from about 400^2 on FP64 arithmetic, half of it the
+// sincos of link updates.  OMF4 step (5 link updates, 6 kicks) on a B200 against one
+// kernel per update and kick (launch and L2 round trips, 5.8 us a pass): 32^2 37.6 -> 6.6
+// us, 128^2 35.0 -> 9.3, 256^2 35.1 -> 11.6, 512^2 49.5 -> 22.5.  With two exchanges a kick
+// (the links to the right and above sent first, then v) 128^2 took 10.8, 256^2 15.2, 512^2 25.3.
 #include <algorithm>
 
 #include "resident.cuh"
@@ -49,7 +50,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_gauge(const __g
     constexpr int BOX = 2 * K + 64, E = 32;   // bytes of a face entry
     constexpr int TOP = K > 1 ? K - 2 : 0;    // the highest row is K - 1 or this
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double2* box = reinterpret_cast<double2*>(dyn);
+    double* const boxes = reinterpret_cast<double*>(dyn);   // two copies of the inboxes, in turn
     if (threadIdx.x == 0) {
         B.rep = P.rep;
         B.C.nb = P.nb;
@@ -87,103 +88,113 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_gauge(const __g
             m2[j] = P.mom[g + V];
         }
     }
+    // the links beyond the tile that its plaquettes need, carried along with their momenta:
+    // U1 of the row above (a lane a column) and U2 of the column to the right (lane j row j)
+    double2 ua = make_double2(0, 0), ur = ua;
+    double ma = 0.0, mr = 0.0, Fa = 0.0, Fr = 0.0;
+    if (on && v_ok) {
+        const long long g = t4.x + lane + (long long)L1 * (t4.y + h == P.rep.L2 ? 0 : t4.y + h);
+        ua = P.U[g];
+        ma = P.mom[g];
+    }
+    if (on && lane < h) {
+        const long long g = V + (t4.x + w == L1 ? 0 : t4.x + w) + (long long)L1 * (t4.y + lane);
+        ur = P.U[g];
+        mr = P.mom[g];
+    }
     unsigned seq = 0;
     bool ok = true;
-    // waits for the slots of one exchange: the first K lanes a row of the column from
-    // side sx (into this warp's inbox), every lane its row entry from side sy
-    auto receive = [&](int sx, int sy, bool link, double2& row) {
-        const u64 slots = B.C.slots + (u64)(seq & 1u) * P.nslots * 16;
-        double2* mine = box + warp * BOX;
-        const bool rx = on && W.warp[sx] < 0 && lane < h, ry = on && W.warp[sy] < 0;
-        const u64 px = slots + W.from[sx] + E * lane, py = slots + W.from[sy] + E * lane;
-        if (W.warp[sx] < 0 || W.warp[sy] < 0) {
+    // F of the present links; false when a wait gave up (in all threads of the block)
+    auto force = [&]() -> bool {
+        double v[K];
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+            double2 r = make_double2(__shfl_sync(0xffffffffu, u2[j].x, srcR), __shfl_sync(0xffffffffu, u2[j].y, srcR));
+            const double2 e = make_double2(__shfl_sync(0xffffffffu, ur.x, j), __shfl_sync(0xffffffffu, ur.y, j));
+            if (er) r = e;
+            double2 a = j + 1 < K ? u1[j + 1 < K ? j + 1 : j] : ua;
+            if (j == TOP && K > 1) a = make_double2(full ? a.x : ua.x, full ? a.y : ua.y);
+            v[j] = P.beta * plaquette_of(u1[j], r, a, u2[j]).y;
+        }
+        const double top = full ? v[K - 1] : v[TOP];
+        ++seq;
+        double* const box = boxes + (seq & 1u) * nw * BOX;
+        double* const mine = box + warp * BOX;
+        const u64 from = B.C.slots + (u64)(seq & 1u) * P.nslots * 16;
+        const u64 to = CL ? (u64)(seq & 1u) * P.nslots * 16 : from;   // W.to holds addresses in a cluster
+        if (on) {
+            if (W.warp[2] >= 0) box[W.warp[2] * BOX + 2 * K + 32 + lane] = v[0];
+            else send1<CL>(to + W.to[2] + E * lane, v[0], seq);
+            if (W.warp[3] >= 0) box[W.warp[3] * BOX + 2 * K + lane] = top;
+            else send1<CL>(to + W.to[3] + E * lane, top, seq);
+            if (el) {
+#pragma unroll
+                for (int j = 0; j < K; j++) {
+                    if (W.warp[0] >= 0) box[W.warp[0] * BOX + K + j] = v[j];
+                    else send1<CL>(to + W.to[0] + E * j, v[j], seq);
+                }
+            }
+            if (er) {
+#pragma unroll
+                for (int j = 0; j < K; j++) {
+                    if (W.warp[1] >= 0) box[W.warp[1] * BOX + j] = v[j];
+                    else send1<CL>(to + W.to[1] + E * j, v[j], seq);
+                }
+            }
+        }
+        if (__syncthreads_or(!ok)) return false;
+        double down = 0.0, up = 0.0;
+        if (on) {
+            const int side = lane >= K ? 1 : 0;   // the first 2K lanes read a row each of the left and right columns
+            const bool rx = lane < 2 * K && W.warp[side] < 0 && lane - side * K < h;
+            const bool rd = W.warp[2] < 0, ru = W.warp[3] < 0;
+            const u64 px = from + W.from[side] + E * (lane - side * K);
+            ulonglong2 qx, qd, qu;
             Patience pt;
             for (;;) {
-                ulonglong2 x0, x1, y0, y1;
-                bool ready = true;
-                if (rx) {
-                    x0 = ld_slot<CL>(px);
-                    if (link) x1 = ld_slot<CL>(px + 16);
-                }
-                if (ry) {
-                    y0 = ld_slot<CL>(py);
-                    if (link) y1 = ld_slot<CL>(py + 16);
-                }
-                if (rx) ready = tagged(x0, seq) && (!link || tagged(x1, seq));
-                if (ry) ready = ready && tagged(y0, seq) && (!link || tagged(y1, seq));
-                if (__all_sync(0xffffffffu, ready)) {
-                    if (rx) mine[(sx == 1 ? K : 0) + lane] = make_double2(slot_double(x0), link ? slot_double(x1) : 0.0);
-                    if (ry) row = make_double2(slot_double(y0), link ? slot_double(y1) : 0.0);
-                    break;
-                }
+                if (rd) qd = ld_slot<CL>(from + W.from[2] + E * lane);
+                if (ru) qu = ld_slot<CL>(from + W.from[3] + E * lane);
+                if (rx) qx = ld_slot<CL>(px);
+                const bool ready = (!rd || tagged(qd, seq)) && (!ru || tagged(qu, seq)) && (!rx || tagged(qx, seq));
+                if (__all_sync(0xffffffffu, ready)) break;
                 if (!pt.more(B.C.err)) {
                     ok = false;
                     break;
                 }
             }
+            if (rx) mine[lane] = slot_double(qx);
             __syncwarp();
+            down = rd ? slot_double(qd) : mine[2 * K + lane];
+            up = ru ? slot_double(qu) : mine[2 * K + 32 + lane];
         }
-        if (on && W.warp[sy] >= 0) row = mine[2 * K + (sy == 3 ? 32 : 0) + lane];
-    };
-    // F of the present links; false when a wait gave up (in all threads of the block)
-    auto force = [&]() -> bool {
-        ++seq;
-        const u64 slots = (CL ? 0 : B.C.slots) + (u64)(seq & 1u) * P.nslots * 16;   // W.to holds addresses in a cluster
-        if (on) {
-            if (W.warp[2] >= 0) box[W.warp[2] * BOX + 2 * K + 32 + lane] = u1[0];
-            else send2<CL>(slots + W.to[2] + E * lane, u1[0], seq);
-            if (el) {
-#pragma unroll
-                for (int j = 0; j < K; j++) {
-                    if (W.warp[0] >= 0) box[W.warp[0] * BOX + K + j] = u2[j];
-                    else send2<CL>(slots + W.to[0] + E * j, u2[j], seq);
-                }
-            }
-        }
-        if (__syncthreads_or(!ok)) return false;
-        double2 up = make_double2(0, 0);
-        receive(1, 3, true, up);
-        double v[K];
-        const double2* mine = box + warp * BOX;
-#pragma unroll
-        for (int j = 0; j < K; j++) {
-            double2 r = make_double2(__shfl_sync(0xffffffffu, u2[j].x, srcR), __shfl_sync(0xffffffffu, u2[j].y, srcR));
-            if (er && (j < K - 1 || full)) r = mine[K + j];
-            double2 a = j + 1 < K ? u1[j + 1 < K ? j + 1 : j] : up;
-            if (j == TOP && K > 1) a = make_double2(full ? a.x : up.x, full ? a.y : up.y);
-            v[j] = P.beta * plaquette_of(u1[j], r, a, u2[j]).y;
-        }
-        if (on) {
-            const double top = full ? v[K - 1] : v[TOP];
-            if (W.warp[3] >= 0) box[W.warp[3] * BOX + 2 * K + lane].x = top;
-            else send1<CL>(slots + W.to[3] + E * lane, top, seq);
-            if (er) {
-#pragma unroll
-                for (int j = 0; j < K; j++) {
-                    if (W.warp[1] >= 0) box[W.warp[1] * BOX + j].x = v[j];
-                    else send1<CL>(slots + W.to[1] + E * j, v[j], seq);
-                }
-            }
-        }
-        if (__syncthreads_or(!ok)) return false;
-        double2 down = make_double2(0, 0);
-        receive(0, 2, false, down);
+        double vr = 0.0;   // lane j: v of the tile's last column, row j
 #pragma unroll
         for (int j = 0; j < K; j++) {
             double l = __shfl_sync(0xffffffffu, v[j], srcL);
-            if (el && (j < K - 1 || full)) l = mine[j].x;
-            const double d = j > 0 ? v[j > 0 ? j - 1 : 0] : down.x;
-            F1[j] = -v[j] + d;
+            if (el && (j < K - 1 || full)) l = mine[j];
+            F1[j] = -v[j] + (j > 0 ? v[j > 0 ? j - 1 : 0] : down);
             F2[j] = v[j] - l;
+            const double e = __shfl_sync(0xffffffffu, v[j], max(w - 1, 0));
+            if (lane == j) vr = e;
         }
+        Fa = -up + top;
+        if (on && lane < h) Fr = mine[K + lane] - vr;
         return true;
     };
+    // explicit fma: the carried links' momenta get the bits that their owners' get
     auto kick = [&](double e) {
 #pragma unroll
         for (int j = 0; j < K; j++) {
-            m1[j] = m1[j] + e * F1[j];
-            m2[j] = m2[j] + e * F2[j];
+            m1[j] = fma(e, F1[j], m1[j]);
+            m2[j] = fma(e, F2[j], m2[j]);
         }
+        ma = fma(e, Fa, ma);
+        mr = fma(e, Fr, mr);
+    };
+    auto move = [&](double2 u, double em) {
+        double s, c;
+        sincos(em, &s, &c);
+        return cmul(make_double2(c, s), u);
     };
     bool alive = force();
     if (alive) kick(P.first);
@@ -192,12 +203,11 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_gauge(const __g
             const double e = P.u[k];
 #pragma unroll
             for (int j = 0; j < K; j++) {
-                double s1, c1, s2, c2;
-                sincos(e * m1[j], &s1, &c1);
-                sincos(e * m2[j], &s2, &c2);
-                u1[j] = cmul(make_double2(c1, s1), u1[j]);
-                u2[j] = cmul(make_double2(c2, s2), u2[j]);
+                u1[j] = move(u1[j], e * m1[j]);
+                u2[j] = move(u2[j], e * m2[j]);
             }
+            ua = move(ua, e * ma);
+            ur = move(ur, e * mr);
             alive = force();
             if (alive) kick(i == P.ns - 1 && k == P.m - 1 ? P.last : P.c[k]);
         }
@@ -266,8 +276,9 @@ static int gauge_dispatch(const ResGaugeP& P, const ResPlan& p, cudaStream_t s, 
     }
 }
 
-// The split with the least modelled cycles per kick: FP64 arithmetic of the busiest
-// SM (about 125 a row of 32 sites) and two exchanges.  K = 0: the fields do not fit.
+// The split with the least modelled cycles per link update and kick: the exchange, the
+// chain of a thread's column, and what the block's warps issue.  Fitted to 16 splits of
+// lattices from 64^2 to 256^2 (2945 to 6050 cycles, within 7%).  K = 0: the fields do not fit.
 static int gauge_plan(int L1, int L2, int num_sms, ResPlan* best) {
     for (int mc : {kResCluster, 8, 0}) {
         best->K = 0;
@@ -278,7 +289,7 @@ static int gauge_plan(int L1, int L2, int num_sms, ResPlan* best) {
                 for (int by = 1; by <= std::min(nty, num_sms / bx); by++) {
                     ResPlan p{K, bx * by <= mc ? 1 : 0, 1, bx, by, (ntx + bx - 1) / bx, (nty + by - 1) / by, ntx, nty, 0.0};
                     if (p.wx * p.wy > kResWarps) continue;
-                    p.cost = 125.0 * p.wx * p.wy * K + 500 + (bx * by == 1 ? 0 : p.cl ? 900 : 2000);
+                    p.cost = 300.0 * K + 60 * K * K + 30 * p.wx * p.wy * (K + 1) + (bx * by == 1 ? 1700 : p.cl ? 2100 : 3160);
                     if (!best->K || p.cost < best->cost) *best = p;
                 }
         }
