@@ -1278,6 +1278,20 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_cg(const __grid
 
 // ---------------------------------------------------------------------------
 // host side
+// A kernel's limit of dynamic shared memory belongs to the function on the device, whoever
+// launches it: every launch and query asks for all that the device has beside the kernel's
+// static shared memory, so that host threads with contexts of other sizes, which share the
+// function, never lower the limit under one another's launches.
+inline int res_allow_smem(const void* kern) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa{};
+    QCHECK(cudaGetDevice(&dev));
+    QCHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    QCHECK(cudaFuncGetAttributes(&fa, kern));
+    QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    return QED2D_OK;
+}
+
 inline int res_slots(const ResPlan& p, int per) { return per * (2 * p.wy * p.K + 2 * p.wx * 32); }   // of one buffer of a block
 
 template <class R, int K>
@@ -1290,7 +1304,7 @@ template <class R, int K>
 static int res_clusters_k(const ResPlan& plan) {
     const void* kern = (const void*)k_res_cg<R, K, true>;
     const size_t sm = res_smem<R, K>(plan);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess ||
+    if (res_allow_smem(kern) != QED2D_OK ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -1318,7 +1332,7 @@ template <class R, int K, bool CL>
 static int res_launch_k(const ResP& P, const ResPlan& plan, cudaStream_t stream) {
     const void* kern = (const void*)k_res_cg<R, K, CL>;
     const size_t sm = res_smem<R, K>(plan);
-    QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    QTRY(res_allow_smem(kern));
     if (CL) QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P.nb * P.nteams);

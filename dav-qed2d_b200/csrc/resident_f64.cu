@@ -159,7 +159,7 @@ int res_ms_launch(const ResP& P0, const ResPlan& plan, const ResMs& m, cudaStrea
     M.nw = nw;
     const size_t sm = res_ms_smem(plan, M.n);
     const void* kern = plan.K == 1 ? (const void*)k_res_ms<1> : (const void*)k_res_ms<2>;
-    QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    QTRY(res_allow_smem(kern));
     const int items = nw * plan.K * (M.n - 1), shift_warps = items < kResWarps - nw ? items : kResWarps - nw;
     void* args[] = {(void*)&P, (void*)&M};
     QCHECK(cudaLaunchCooperativeKernel(kern, dim3(P.nb), dim3(32 * (1 + nw + shift_warps)), args, sm, stream));

@@ -236,7 +236,7 @@ template <int K, bool CL>
 static int gauge_launch(const ResGaugeP& P, const ResPlan& p, cudaStream_t stream, bool query, int* clusters) {
     const void* kern = (const void*)k_res_gauge<K, CL>;
     const size_t sm = gauge_smem(p);
-    QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    QTRY(res_allow_smem(kern));
     if (CL) QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.blocks());
