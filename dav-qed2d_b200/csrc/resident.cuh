@@ -36,9 +36,16 @@
 //   w = g5Dw t + mu^2 r halo of t; the sum of both meanwhile, and p, x of the last iteration
 //   beta = |r|^2 / |r_old|^2,  alpha = |r|^2 / (<r, A r> - beta |r|^2 / alpha_old)
 //   q = w + beta q (= A p),  r -= alpha q;  later p = r_old + beta p, x += alpha p
-// Iteration counts and residuals are those of the other forms (64^2, 128^2, masses down
-// to 0.02 and -0.05, residuals to 1e-14), and 128^2 takes 3.0 us an iteration instead of
-// 4.4.  The mixed solver does not use them, although 256^2 would take 2.9 us instead of
+// 128^2 takes 3.1 us an iteration instead of 4.4.  The difference in alpha's denominator
+// (= <p, A p>) multiplies the relative error of the last one by
+// beta alpha / alpha_old = (what is subtracted) / (what is left).  Where that exceeds one,
+// errors would grow from iteration to iteration, and the iteration is made directly:
+//   p = r + beta p,  t = g5Dw p,  sum <p, A p> = |t|^2 + mu^2 |p|^2,  q = g5Dw t + mu^2 p.
+// Counts and residuals then are those of the two-sum form in ill-conditioned systems too
+// (free links 64^2, m0 = 0.001: 267 iterations to 1e-12 and a true residual of 4e-11 in
+// both, 355 and 6.5e-11 without; Gaussian links of width 0.45 on 40^2, m0 = -0.157: 800 in
+// both, 1020 without), where a sixth to a third of the iterations are direct; at masses
+// from -0.1 up on such links (128^2) none is.  The mixed solver does not use them, although 256^2 would take 2.9 us instead of
 // 3.5: FP32 rounding and the jumps of r at reliable updates break the identity behind
 // alpha near the critical mass, where solves that converge otherwise did not.  One extra
 // warp per block does the block's sum, the team's sum and the scalar recurrences.
@@ -48,7 +55,7 @@
 // seen, plus 0.25 us of skew between the blocks, 0.2 us for the block's own sum and 0.25
 // us for the recurrences, whatever the split; in a cluster about half of that, which the
 // stencil's own chain (0.8 us) hides.  us an iteration, mixed: 64^2 1.95, 128^2 2.7, 256^2
-// 3.5, 512^2 4.3; FP64: 64^2 2.2, 128^2 3.0, 256^2 4.2, 350x370 6.6.
+// 3.5, 512^2 4.3; FP64: 64^2 2.2, 128^2 3.1, 256^2 4.05, 350x370 6.8.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -102,7 +109,7 @@ struct ResP {
     int single;               // write the context's solve record
 };
 
-enum { RF_GO, RF_UPD, RF_FIN, RF_STOP, RF_ZERO, RF_ABORT };   // the last three end the solve
+enum { RF_GO, RF_DIR, RF_UPD, RF_FIN, RF_STOP, RF_ZERO, RF_ABORT };   // the last three end the solve
 
 // what the scalar warp hands to the workers after an exchange
 struct ResSc {
@@ -298,11 +305,16 @@ __device__ __forceinline__ bool cluster_sum_slots(const TeamComm& C, unsigned se
     return ok;
 }
 
+// the exponent that scales this lane's words in team_sum_fixed, from an earlier sum
+__device__ __forceinline__ int fixed_exponent(Sums est) {
+    const double e = (threadIdx.x & 2) ? est.d : est.g;
+    return min(max((int)((u64)__double_as_longlong(e) >> 52 & 0x7ff) - 1023, -900), 900);
+}
 // The same through atomic words (teams over global memory): a partial in 80-bit fixed
-// point, 40 bits a word, scaled by a power of two that every block derives from an
-// earlier sum, with a count of the blocks in the top byte of each word.  Integer
+// point, 40 bits a word, scaled by a power of two (2^-ex) that every block derives from
+// an earlier sum, with a count of the blocks in the top byte of each word.  Integer
 // additions commute, so the sum does not depend on the order; it is exact to 2^-76 of
-// that earlier sum `est` (and repeated through the slots when that leaves less than 52
+// that earlier sum (and repeated through the slots when that leaves less than 52
 // bits of it).  The words only grow (modulo 2^64), two sets in turn, so nothing is
 // cleared; `base` is the set's value before the exchange.  A partial out of range (or
 // NaN) is counted in the next byte instead, and then every block falls back to
@@ -314,12 +326,11 @@ __device__ __forceinline__ bool cluster_sum_slots(const TeamComm& C, unsigned se
 // counter and partials behind it, and 2740 through 7 clusters of 16 blocks (distributed
 // shared memory, then L2 between the clusters' first blocks).
 template <int NV>
-__device__ __forceinline__ bool team_sum_fixed(const TeamComm& C, unsigned seq, Sums v, Sums est, u64& base, Sums& tot,
+__device__ __forceinline__ bool team_sum_fixed(const TeamComm& C, unsigned seq, Sums v, int ex, u64& base, Sums& tot,
                                                bool need_d, bool& exact) {
     const int lane = threadIdx.x & 31;
     u64* acc = C.acc + 16 * (seq & 1u) + (lane & 3);
-    const double e = (lane & 2) ? est.d : est.g, x = (lane & 2) ? v.d : v.g;
-    const int ex = min(max((int)((u64)__double_as_longlong(e) >> 52 & 0x7ff) - 1023, -900), 900);
+    const double x = (lane & 2) ? v.d : v.g;
     if (lane < 2 * NV) {
         const double y = x * __longlong_as_double((long long)(1023 + 36 - ex) << 52);   // exact
         const bool fits = y < 1099511627776.0;   // 2^40; false for NaN
@@ -631,14 +642,15 @@ struct ResBlock {
 template <bool MIXED, bool CL, bool MS = false>
 __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsigned seq, u64& base0, u64& base1,
                                                const ResMs* M = nullptr, ResMsBlock* S = nullptr) {
-    enum { X_BEGIN, X_RR, X_PAP, X_FENCE, X_TRUE };   // what the coming exchange sums (X_PAP: mixed only)
+    enum { X_BEGIN, X_RR, X_PAP, X_FENCE, X_TRUE };   // what the coming exchange sums (X_PAP in FP64: a direct iteration)
     constexpr int NV = MIXED ? 1 : 2;
     const int nw = MS ? M->nw : (int)(blockDim.x >> 5) - 1, nth = 32 * (nw + 1), lane = threadIdx.x & 31;
     // |r|^2, its inverse, the inverse of the last alpha
     double rr = 0.0, inv_rr = 0.0, inv_a = 0.0, beta = 0.0;
     double maxrr = 0.0, thr = 0.0;   // the largest |r|^2 since the last update; below thr: update
     double s = 1.0, rr64 = 0.0, bb = 0.0, tol = 0.0;
-    double rr_last = 1.0, pap_last = 4.0;   // the last sums: the fixed-point scales
+    double rr_last = 1.0, pap_last = 4.0, dir_est = 1.0;   // the last sums
+    int ex = 0;   // the coming ones' fixed-point scale (team_sum_fixed)
     int k = 0, nupd = 0, fences = 0, flag = RF_GO, next = X_BEGIN;
     bool conv = false, fresh = true;
     // MS: lane i's shift; the base system's last alpha and the alpha and beta before
@@ -675,9 +687,8 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
         } else {
             bool exact = false;
             if (next != X_BEGIN) {
-                const Sums e{next == X_RR ? rr_last : next == X_PAP ? pap_last : next == X_TRUE ? rr64 : 1.0, pap_last};
                 u64 bs = (seq & 1u) ? base1 : base0;
-                ok = team_sum_fixed<NV>(B.C, seq, v, e, bs, tot, next == X_RR, exact);
+                ok = team_sum_fixed<NV>(B.C, seq, v, ex, bs, tot, next == X_RR, exact);
                 if (seq & 1u) base1 = bs;
                 else base0 = bs;
             }
@@ -687,9 +698,10 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
         const double inv_old = inv_rr;
         const bool all = MS && (next == X_BEGIN || next == X_RR);   // the shift warps join this barrier
         const bool step = MS && next == X_RR && !fresh;             // and an iteration is behind them
-        if (MIXED && next == X_PAP) {   // <p, (A + mu2) p>
+        if (next == X_PAP) {   // <p, (A + mu2) p>
             alpha = rr / tot.g;
-            pap_last = tot.g;
+            if (MIXED) pap_last = tot.g;
+            flag = RF_GO;
             k++;
             next = X_RR;
         } else if (next == X_RR) {   // |r|^2; FP64: and |g5Dw r|^2
@@ -707,8 +719,17 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
                     next = X_PAP;
                 } else {
                     pap_last = tot.d;
-                    alpha = tot.g / (tot.d + P.mu2 * tot.g - beta * (tot.g * inv_a));   // beta = inv_a = 0 at first
+                    const double rar = tot.d + P.mu2 * tot.g, pap = rar - beta * (tot.g * inv_a);   // beta = inv_a = 0 at first
+                    const bool dir = !fresh && !(pap > 0.5 * rar);   // more subtracted than left
+                    alpha = tot.g / pap;
+                    dir_est = rar;
                     k++;
+                    if (__builtin_expect(dir, 0)) {
+                        alpha = 0.0;
+                        k--;
+                        flag = RF_DIR;
+                        next = X_PAP;
+                    }
                 }
                 if (fresh) maxrr = tot.g;
                 fresh = false;
@@ -780,9 +801,9 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
                 a_last = a_now;
                 b_now = b_new;
             }
+            if (alpha != 0.0) a_now = alpha;   // a direct iteration's comes one sum later
             if (all) {
-                a_now = alpha;
-                if (lane == 0) S->flag[round & 1] = flag;
+                if (lane == 0) S->flag[round & 1] = flag == RF_DIR ? RF_GO : flag;
                 round++;
                 bar_arrive_n(4, blockDim.x - 32 * nw);
             }
@@ -793,6 +814,7 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
         if (!MIXED && alpha != 0.0) inv_a = 1.0 / alpha;
         maxrr = fmax(maxrr, rr);
         thr = fmax(P.delta2 * maxrr, tol * s * s);
+        ex = fixed_exponent(Sums{next == X_RR ? rr_last : next == X_PAP ? (MIXED ? pap_last : dir_est) : next == X_TRUE ? rr64 : 1.0, pap_last});
     }
     if (flag != RF_ABORT && B.C.rank == 0 && lane == 0) {
         const int it = conv ? k : P.maxiter;
@@ -1169,6 +1191,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
             for (int j = 0; j < K; j++) qs[j * nwk] = t[j];
         } else {
             bool adv = false;   // an iteration's p and x are still to be formed
+            bool dir = false;   // a direct iteration: p in the place of r, which waits in qs
             for (;;) {
                 ++seq;   // t = g5Dw r
                 stencil_inner<R, K, CL>(T, r, u1, u2, m2, box0, to0, seq, t);
@@ -1180,7 +1203,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
                 });
 #pragma unroll
                 for (int j = 0; j < K; j++) d += norm4<R, PK>(t[j]);
-                put_part(B, (double)g, (double)d);
+                put_part(B, dir ? d + P.mu2 * g : (double)g, (double)d);
                 ++seq;   // w = g5Dw t
                 stencil_inner<R, K, CL>(T, t, u1, u2, m2, box1, to1, seq, w);
                 bar_sync_n(2, nwk);
@@ -1200,20 +1223,35 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
                     if constexpr (OLD) ro[j] = r[j];
                     t[j] = qs[j * nwk];
                 }
-                flag = wait_scalar<MIXED>(B, MS);
-                if (flag != RF_GO) break;
+                flag = wait_scalar<MIXED>(B, MS && !dir);
                 alpha = (R)B.sc.alpha;
                 beta = (R)B.sc.beta;
+                if (flag > RF_DIR) break;
+                if (__builtin_expect(flag == RF_DIR, 0)) {
+                    dir = true;
+                    adv = false;
+#pragma unroll
+                    for (int j = 0; j < K; j++) {
+                        qs[j * nwk] = r[j];
+                        r[j] = axpy4<R, PK>(beta, ps[j * nwk], r[j]);
+                    }
+                    continue;
+                }
                 adv = true;
                 m++;
 #pragma unroll
-                for (int j = 0; j < K; j++) {   // q = A r + beta q, r -= alpha q
-                    const V4<R> q = axpy4<R, PK>(beta, t[j], w[j]);
+                for (int j = 0; j < K; j++) {   // q = A r + beta q (direct: A p), r -= alpha q
+                    V4<R> q = axpy4<R, PK>(beta, t[j], w[j]);
+                    if (__builtin_expect(dir, 0)) {
+                        q = w[j];
+                        r[j] = ro[j] = t[j];
+                    }
                     qs[j * nwk] = q;
                     if constexpr (!OLD) ps[j * nwk] = axpy4<R, PK>(beta, ps[j * nwk], r[j]);
                     r[j] = axpy4<R, PK>(-alpha, q, r[j]);
                     if constexpr (MS) rbuf[((m & 1) * K + j) * nwk + threadIdx.x - 32] = r[j];
                 }
+                dir = false;
             }
             if (flag == RF_FIN) res_finish(P, B, xs);
             return seq;
