@@ -313,14 +313,14 @@ __device__ __forceinline__ int fixed_exponent(Sums est) {
 // The same through atomic words (teams over global memory): a partial in 80-bit fixed
 // point, 40 bits a word, scaled by a power of two (2^-ex) that every block derives from
 // an earlier sum, with a count of the blocks in the top byte of each word.  Integer
-// additions commute, so the sum does not depend on the order; it is exact to 2^-76 of
-// that earlier sum (and repeated through the slots when that leaves less than 52
-// bits of it).  The words only grow (modulo 2^64), two sets in turn, so nothing is
-// cleared; `base` is the set's value before the exchange.  A partial out of range (or
-// NaN) is counted in the next byte instead, and then every block falls back to
-// team_sum_slots.  A lane per word, side by side, so that a block's atomics are one
-// request and its poll another: with a line for each word 128^2 and 256^2 in FP64 took
-// 2% more, with two polls in flight 13%.  Measured with 144
+// additions commute, so the sum does not depend on the order; each block's
+// part is exact to 2^-76 of that earlier sum, the sum of 148 to 2^-68 (and repeated through
+// the slots when it is below 2^-16 of the earlier one, which would leave less than 52 bits).
+// The words only grow (modulo 2^64), two sets in turn, so nothing is cleared; `base` is the
+// set's value before the exchange.  A partial out of range (or NaN) is counted in the next
+// byte instead, and then every block falls back to team_sum_slots.  A lane per word, side by
+// side, so that a block's atomics are one request and its poll another: with a line for each
+// word 128^2 and 256^2 in FP64 took 2% more, with two polls in flight 13%.  Measured with 144
 // blocks: 1610 cycles an exchange, against 2970 with a row of slots per block (whose
 // polls grow with the square of the team), 4660 with one row, 2440 with an arrival
 // counter and partials behind it, and 2740 through 7 clusters of 16 blocks (distributed
@@ -355,8 +355,8 @@ __device__ __forceinline__ bool team_sum_fixed(const TeamComm& C, unsigned seq, 
     const double s = (w + __shfl_xor_sync(0xffffffffu, w, 1) * 0x1p-40) * __longlong_as_double((long long)(1023 - 36 + ex) << 52);
     tot.g = __shfl_sync(0xffffffffu, s, 0);
     if (NV > 1) tot.d = __shfl_sync(0xffffffffu, s, 2);
-    // no block out of range, and 52 bits left of the sum
-    const bool good = ((d >> 48) & 0xff) == 0 && s >= __longlong_as_double((long long)(1023 - 24 + ex) << 52);
+    // no block out of range, and the sum of up to 255 blocks' truncated parts holds 52 bits
+    const bool good = ((d >> 48) & 0xff) == 0 && s >= __longlong_as_double((long long)(1023 - 16 + ex) << 52);
     exact = __all_sync(0xffffffffu, good || !(lane == 0 || (NV > 1 && lane == 2 && need_d)));
     return ok;
 }
