@@ -664,6 +664,7 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
         Sums tot{0.0, 0.0}, v;
         bool ok = true;
         bar_sync_n(1, nth);   // the workers' partials are in
+        if (next == X_FENCE) __threadfence();   // releases what the block's workers stored before this barrier
         {
             double a[4] = {0.0, 0.0, 0.0, 0.0}, c[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
@@ -735,7 +736,7 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
                 fresh = false;
                 rr = tot.g;
             }
-        } else if (next == X_FENCE) {   // orders the blocks' FP64 stores
+        } else if (next == X_FENCE) {   // orders the blocks' FP64 stores: the others' are acquired
             __threadfence();
             if (flag == RF_FIN) flag = RF_STOP;
             if (--fences == 0) next = X_TRUE;
