@@ -955,6 +955,7 @@ struct qed2d_batch {
     };
     std::vector<ResClass> res;
     int res_fits = -1;              // -1: not planned yet, 0: some replica does not fit on chip
+    bool on_chip = false;           // the last solve ran on chip
     bool res_on = false;            // the schedule was chosen by the library and stands for the on-chip form
     ResOut* d_resout = nullptr;     // [nrep]
     cudaEvent_t res_fork = nullptr;
@@ -1325,6 +1326,7 @@ int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* 
             }
         }
     }
+    h->on_chip = h->res_on;
     if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
     RCGP P{};
     P.nrep = h->nrep;
@@ -1782,6 +1784,12 @@ int qed2d_batch_set_schedule(qed2d_batch* h, int schedule) {
 int qed2d_batch_get_schedule(const qed2d_batch* h, int* schedule) {
     if (!h || !schedule) return QED2D_ERR_BAD_ARG;
     *schedule = h->uniform ? h->usched : h->rsched;
+    return QED2D_OK;
+}
+
+int qed2d_batch_get_on_chip(const qed2d_batch* h, int* on) {
+    if (!h || !on) return QED2D_ERR_BAD_ARG;
+    *on = h->on_chip ? 1 : 0;
     return QED2D_OK;
 }
 

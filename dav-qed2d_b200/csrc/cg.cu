@@ -1302,6 +1302,7 @@ int cg_solve(Ctx& c, const SolveArgs& a, int precision) {
             c.sched[slot] = (p.cl ? 2 : 1) + (slot ? 4 : 0);
         }
     }
+    c.on_chip[slot] = c.res_on[slot];
     if (c.res_on[slot]) return cg_resident(c, a, slot);
     CGP P{};
     P.g = c.g;
@@ -1531,6 +1532,7 @@ static int multishift_resident(Ctx& c, const ResPlan& p, const double2* U, const
 int multishift_solve(Ctx& c, const double2* U, const double2* b, double2* const* x, const double* mu2, int n,
                      double am0, int maxiter, double eps) {
     if (n < 1 || n > kMaxShifts) return QED2D_ERR_BAD_ARG;
+    c.on_chip[2] = false;
     if ((c.sched[2] < 0 && c.ms_layout < 0 && c.g.V < kMs32Sites) || c.res_on[2]) {
         auto it = c.res_ms.find(n);
         if (it == c.res_ms.end()) {
@@ -1539,6 +1541,7 @@ int multishift_solve(Ctx& c, const double2* U, const double2* b, double2* const*
             it = c.res_ms.emplace(n, p).first;
         }
         if (it->second.K > 0) {
+            c.on_chip[2] = true;
             c.res_on[2] = true;
             c.sched[2] = 1;
             return multishift_resident(c, it->second, U, b, x, mu2, n, am0, maxiter, eps);

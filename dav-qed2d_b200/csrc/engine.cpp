@@ -310,7 +310,7 @@ static int md_omf4_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MD
     const double r5 = 0.5 - R1 - R3, r6 = 1.0 - 2.0 * (R2 + R4);
     const double cm[6] = {R1, R3, r5, r5, R3, R1};
     const double cu[5] = {R2, R4, r6, R4, R2};
-    if (ns > 0 && !s.U32 && res_gauge_fits(c)) {
+    if ((c.on_chip[3] = ns > 0 && !s.U32 && res_gauge_fits(c))) {
         ResMd md{cm[0] * eps, {}, {}, cm[5] * eps, 5, ns, 1};
         for (int k = 0; k < 5; k++) {
             md.u[k] = eps * cu[k];
@@ -327,7 +327,7 @@ static int md_omf4_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MD
 }
 
 static int md_leapfrog_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MDState& s) {
-    if (ns > 0 && !s.U32 && res_gauge_fits(c))
+    if ((c.on_chip[3] = ns > 0 && !s.U32 && res_gauge_fits(c)))
         return res_gauge_md(c, mom, U, ResMd{0.5 * eps, {eps}, {eps}, 0.5 * eps, 1, ns, 0});
     GaugePingPong pp(c, U, mom, s);
     QTRY(pp.kick(0.5 * eps));
@@ -510,6 +510,14 @@ int qed2d_ctx_get_schedule(const qed2d_ctx* ctx, int precision, int* schedule) {
     const int slot = sched_slot(precision);
     if (slot < 0) return bad_arg("schedule: QED2D_PREC_F64, QED2D_PREC_MIXED or QED2D_MULTISHIFT only");
     *schedule = ctx->c.sched[slot];
+    return QED2D_OK;
+}
+
+int qed2d_ctx_get_on_chip(const qed2d_ctx* ctx, int what, int* on) {
+    if (!ctx || !on) return bad_arg("context or on is NULL");
+    const int slot = what == QED2D_GAUGE_MD ? 3 : sched_slot(what);
+    if (slot < 0) return bad_arg("on_chip: QED2D_PREC_F64, QED2D_PREC_MIXED, QED2D_MULTISHIFT or QED2D_GAUGE_MD only");
+    *on = ctx->c.on_chip[slot] ? 1 : 0;
     return QED2D_OK;
 }
 

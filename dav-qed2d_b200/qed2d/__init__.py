@@ -39,7 +39,7 @@ __all__ = [
     "gamm5Dw_sqr_sqr", "gamm5", "Dw", "CG", "save_gauge", "load_gauge", "get_rhmc_params", "power_method",
     "reweighting_factor", "R", "MultiCG", "generate_pseudofermion_", "plwv", "LuscherZ", "LuscherZp",
     "k", "v", "a_r", "c_r", "mu", "nu", "rho_mu", "rho_nu", "P", "d", "A", "delta", "error",
-    "seed", "set_precision", "set_schedule", "get_schedule", "set_multishift_layout", "get_multishift_layout", "Qed2dError", "cfield", "rfield", "context",
+    "seed", "set_precision", "set_schedule", "get_schedule", "on_chip", "set_multishift_layout", "get_multishift_layout", "Qed2dError", "cfield", "rfield", "context",
 ]
 
 
@@ -334,6 +334,16 @@ def get_schedule(prm: LattParm, precision="mixed") -> int:
     v = C.c_int(0)
     check(lib().qed2d_ctx_get_schedule(_c(prm), _PRECS[precision], C.byref(v)), "get_schedule")
     return v.value
+
+
+def on_chip(prm: LattParm, what="mixed") -> bool:
+    """Whether the last solve on this lattice with `what` ("f64", "mixed",
+    "multishift"), or its last pure-gauge integration ("gauge"), kept its state in
+    registers and shared memory.  get_schedule then reports a number that, set,
+    selects another form: restore the library's choice with set_schedule(prm, -1)."""
+    v = C.c_int(0)
+    check(lib().qed2d_ctx_get_on_chip(_c(prm), _lib.GAUGE_MD if what == "gauge" else _PRECS[what], C.byref(v)), "on_chip")
+    return bool(v.value)
 
 
 def set_graphs(prm: LattParm, on: bool) -> None:
@@ -807,6 +817,14 @@ class Batch:
     @schedule.setter
     def schedule(self, s: int) -> None:
         check(lib().qed2d_batch_set_schedule(self.h, int(s)), "batch_set_schedule")
+
+    @property
+    def on_chip(self) -> bool:
+        """Whether the last solve kept every replica's state on chip (schedule then
+        reports 9 or 6; -1 restores the library's choice)."""
+        v = C.c_int(0)
+        check(lib().qed2d_batch_get_on_chip(self.h, C.byref(v)), "batch_get_on_chip")
+        return bool(v.value)
 
     @property
     def tile_rows(self) -> int:

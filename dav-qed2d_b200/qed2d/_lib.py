@@ -14,6 +14,7 @@ NOALLOC_MAX_SITES = 16384
 OK, NOT_CONVERGED, TIMEOUT, BAD_ARG, CUDA_ERR, NO_MEMORY, UNSUPPORTED = range(7)
 PREC_F64, PREC_MIXED, PREC_PLAIN = 0, 1, 2
 MULTISHIFT = 3   # schedule selector of the multishift solver (QED2D_MULTISHIFT)
+GAUGE_MD = 4     # pure-gauge integration in qed2d_ctx_get_on_chip (QED2D_GAUGE_MD)
 LEAPFROG, OMF4 = 0, 1
 STREAM_MOMENTA, STREAM_METROPOLIS, STREAM_POWER, STREAM_NOISE, STREAM_REWEIGHT = 1, 3, 4, 16, 64
 
@@ -49,6 +50,7 @@ SIGNATURES = {
     "qed2d_ctx_set_precision": (I, [P, I]),
     "qed2d_ctx_get_dims": (I, [P, PI, PI]),
     "qed2d_ctx_set_schedule": (I, [P, I, I]),
+    "qed2d_ctx_get_on_chip": (I, [P, I, PI]),
     "qed2d_ctx_get_schedule": (I, [P, I, PI]),
     "qed2d_ctx_set_multishift_layout": (I, [P, I]),
     "qed2d_ctx_get_multishift_layout": (I, [P, PI]),
@@ -106,6 +108,7 @@ SIGNATURES = {
     "qed2d_batch_create_ragged": (I, [I, PI, PI, PD, C.POINTER(C.c_void_p)]),
     "qed2d_batch_layout": (I, [P, C.POINTER(C.c_int64)]),
     "qed2d_batch_set_schedule": (I, [P, I]),
+    "qed2d_batch_get_on_chip": (I, [P, PI]),
     "qed2d_batch_get_schedule": (I, [P, PI]),
     "qed2d_batch_set_tile_rows": (I, [P, I]),
     "qed2d_batch_get_tile_rows": (I, [P, PI]),

@@ -131,6 +131,13 @@ int qed2d_ctx_get_dims(const qed2d_ctx* ctx, int* L1, int* L2);
 #define QED2D_MULTISHIFT 3   /* schedule selector of the multishift solver (FP64) */
 int qed2d_ctx_set_schedule(qed2d_ctx* ctx, int precision, int schedule);
 int qed2d_ctx_get_schedule(const qed2d_ctx* ctx, int precision, int* schedule);
+/* Whether the most recent solve of QED2D_PREC_F64, QED2D_PREC_MIXED or
+ * QED2D_MULTISHIFT, or the most recent pure-gauge integration (QED2D_GAUGE_MD),
+ * of this context kept its state on chip.  The schedule that get reports for such a
+ * solve is shared with another form, which setting it would select: to restore the
+ * library's choice, set -1. */
+#define QED2D_GAUGE_MD 4
+int qed2d_ctx_get_on_chip(const qed2d_ctx* ctx, int what, int* on);
 /* Layout of the FP64 multishift kernel (schedules 0-2; no reference
  * counterpart: it takes the role of KernelParm's launch geometry for the RHMC
  * solves).  0 = tiles of 32 x 8 sites, one thread per site; 1 = 32 x 8 tiles,
@@ -365,6 +372,7 @@ int qed2d_batch_set_stream(qed2d_batch* batch, void* cuda_stream);
  * only); -1 = tune again on the next solve (get: -1 while untuned). */
 int qed2d_batch_set_schedule(qed2d_batch* batch, int schedule);
 int qed2d_batch_get_schedule(const qed2d_batch* batch, int* schedule);
+int qed2d_batch_get_on_chip(const qed2d_batch* batch, int* on);   /* as qed2d_ctx_get_on_chip */
 /* Tile height of the equal-size batched solver: tiles of 32 x rows sites, rows =
  * 4, 8 or 16 (blocks of 128, 256 or 512 threads, so more or fewer blocks share a
  * replica's tiles and barriers).  It takes the role of the reference's

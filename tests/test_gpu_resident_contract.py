@@ -108,3 +108,55 @@ def test_ill_conditioned_fp64(system, solver):
     note(f"iterations, residuals ({system}, {solver}) on chip / two sums", [its, res])
     assert its[-1] <= its[1] * 1.02, its
     assert all(a <= 1.35 * c for a, c in zip(res[-1], res[1])), res
+
+
+def cg_once(q, prm, prec):
+    q.set_precision(prec)
+    q.CG(q.cfield(*prm.iL), to_dev(hot_links(*prm.iL, 3)), to_dev(cgauss(*prm.iL, 4, 2)), 1.0, 2000, 1e-12,
+         q.gamm5Dw_sqr_msq, prm, None)
+    q.set_precision("f64")
+
+
+# the sizes at which the on-chip solvers are tested for their results, and beyond the chip
+@pytest.mark.parametrize("L1,L2,on", [(2, 2, "mfsg"), (3, 5, "mfsg"), (31, 2, "mfsg"), (33, 7, "mfsg"), (32, 32, "mfsg"),
+                                      (64, 64, "mfsg"), (65, 31, "mfsg"), (100, 37, "mfsg"), (128, 128, "mfsg"),
+                                      (40, 250, "mfsg"), (257, 66, "mfsg"), (256, 256, "mfsg"), (330, 97, "mfsg"),
+                                      (350, 370, "mfg"), (400, 400, "mg"), (512, 512, "mg"), (544, 400, "mg"),
+                                      (576, 576, "")])
+def test_which_sizes_run_on_chip(L1, L2, on):
+    """Mixed CG, FP64 CG, multishift with 4 shifts (352 bytes of shared memory a site: about
+    90 thousand sites on 148 SMs), pure-gauge integration."""
+    import qed2d as q
+    prm = q.LattParm((L1, L2), 4.0)
+    got = ""
+    for prec in ("mixed", "f64"):
+        q.set_schedule(prm, 1, prec)
+        cg_once(q, prm, prec)
+        assert not q.on_chip(prm, prec)   # a schedule set by the caller is the form it names
+        q.set_schedule(prm, -1, prec)
+        cg_once(q, prm, prec)
+        got += prec[0] if q.on_chip(prm, prec) else ""
+    q.set_schedule(prm, -1, "multishift")
+    q.multishift_CG([q.cfield(L1, L2) for _ in range(4)], to_dev(hot_links(L1, L2, 3)), to_dev(cgauss(L1, L2, 4, 2)), 1.0,
+                    [0.3, 0.4, 0.5, 0.6], 2000, 1e-12, prm)
+    got += "s" if q.on_chip(prm, "multishift") else ""
+    q.OMF4_(q.rfield(L1, L2), to_dev(hot_links(L1, L2, 3)), 0.01, 1, prm, None)
+    got += "g" if q.on_chip(prm, "gauge") else ""
+    assert got == on
+
+
+@pytest.mark.parametrize("sizes", [[(33, 7)] * 2, [(64, 64)] * 37, [(256, 256)] * 3, [(32, 32), (100, 37), (128, 128), (2, 3)],
+                                   [(64, 48), (300, 200), (64, 48)]])
+def test_which_batches_run_on_chip(sizes):
+    import qed2d
+    b = qed2d.Batch.ragged(sizes, [4.0] * len(sizes))
+    U, src = b.field(), b.field()
+    for r, s in enumerate(sizes):
+        b.replica(U, r).copy_(to_dev(hot_links(*s, r)))
+        b.replica(src, r).copy_(to_dev(cgauss(*s, r, 2)))
+    assert not b.on_chip
+    b.cg(b.field(), U, src, 1.0, 2000, 1e-12)
+    assert b.on_chip
+    b.schedule = 5 if b.uniform else 2
+    b.cg(b.field(), U, src, 1.0, 2000, 1e-12)
+    assert not b.on_chip
