@@ -1532,8 +1532,10 @@ static int multishift_resident(Ctx& c, const ResPlan& p, const double2* U, const
 int multishift_solve(Ctx& c, const double2* U, const double2* b, double2* const* x, const double* mu2, int n,
                      double am0, int maxiter, double eps) {
     if (n < 1 || n > kMaxShifts) return QED2D_ERR_BAD_ARG;
+    // The choice is each call's own, by its number of shifts; sched[2] and ms_layout are
+    // the other forms', tuned by the first solve that needs one of them.
     c.on_chip[2] = false;
-    if ((c.sched[2] < 0 && c.ms_layout < 0 && c.g.V < kMs32Sites) || c.res_on[2]) {
+    if (!c.ms_sched_set && !c.ms_layout_set && c.g.V < kMs32Sites) {
         auto it = c.res_ms.find(n);
         if (it == c.res_ms.end()) {
             ResPlan p;
@@ -1542,13 +1544,7 @@ int multishift_solve(Ctx& c, const double2* U, const double2* b, double2* const*
         }
         if (it->second.K > 0) {
             c.on_chip[2] = true;
-            c.res_on[2] = true;
-            c.sched[2] = 1;
             return multishift_resident(c, it->second, U, b, x, mu2, n, am0, maxiter, eps);
-        }
-        if (c.res_on[2]) {   // more shifts than fit: the choice is the tuner's after all
-            c.res_on[2] = false;
-            c.sched[2] = -1;
         }
     }
     if (c.sched[2] == 3) return multishift32_solve(c, U, b, x, mu2, n, am0, maxiter, eps);

@@ -501,7 +501,9 @@ int qed2d_ctx_set_schedule(qed2d_ctx* ctx, int precision, int schedule) {
                        : slot == 1 ? "mixed CG schedule must be -1, 0, 1, 2, 4, 5 or 6"
                                    : "schedule must be -1, 0, 1 or 2");
     c.sched[slot] = schedule;
-    c.res_on[slot] = false;   // a schedule set by the caller is the form it names
+    c.on_chip[slot] = false;   // a schedule set by the caller is the form it names
+    if (slot < 2) c.res_on[slot] = false;
+    else c.ms_sched_set = schedule >= 0;
     return QED2D_OK;
 }
 
@@ -509,7 +511,7 @@ int qed2d_ctx_get_schedule(const qed2d_ctx* ctx, int precision, int* schedule) {
     if (!ctx || !schedule) return bad_arg("context or schedule is NULL");
     const int slot = sched_slot(precision);
     if (slot < 0) return bad_arg("schedule: QED2D_PREC_F64, QED2D_PREC_MIXED or QED2D_MULTISHIFT only");
-    *schedule = ctx->c.sched[slot];
+    *schedule = slot == 2 && ctx->c.on_chip[2] ? 1 : ctx->c.sched[slot];
     return QED2D_OK;
 }
 
@@ -525,14 +527,18 @@ int qed2d_ctx_set_multishift_layout(qed2d_ctx* ctx, int layout) {
     QCTX(ctx);
     if (layout < -1 || layout >= kMsLayoutCount) return bad_arg("multishift layout must be -1, 0, 1, 2 or 3");
     c.ms_layout = layout;
-    if (layout >= 0) c.res_on[2] = false;   // a layout is the grid and cluster kernels'
-    if (layout < 0 && c.sched[2] >= 0 && c.sched[2] != 3) c.sched[2] = -1;   // tune both on the next solve
+    c.ms_layout_set = layout >= 0;   // a layout is the grid and cluster kernels'
+    c.on_chip[2] = false;
+    if (layout < 0 && c.sched[2] >= 0 && c.sched[2] != 3) {   // tune both on the next solve
+        c.sched[2] = -1;
+        c.ms_sched_set = false;
+    }
     return QED2D_OK;
 }
 
 int qed2d_ctx_get_multishift_layout(const qed2d_ctx* ctx, int* layout) {
     if (!ctx || !layout) return bad_arg("context or layout is NULL");
-    *layout = ctx->c.ms_layout;
+    *layout = ctx->c.on_chip[2] ? -1 : ctx->c.ms_layout;
     return QED2D_OK;
 }
 
@@ -1175,7 +1181,7 @@ int qed2d_hmc_nf2(qed2d_ctx* ctx, double* U, double am0, double eps, int ns, int
     } else {
         GraphKey k;
         k.i(2).p(U).p(mom).p(X).p(F).p(g5DX).d(am0).d(eps).i(ns).i(integrator).i(maxiter).d(tol).d(c.beta);
-        k.i(c.precision).i(c.res_on[0]).i(c.res_on[1]).i(c.res_on[2]).i(c.sched[0]).i(c.sched[1]).i((long long)c.ws_gen);
+        k.i(c.precision).i(c.res_on[0]).i(c.res_on[1]).i(c.sched[0]).i(c.sched[1]).i((long long)c.ws_gen);
         QTRY(run_graphed(c.md_graph, c.stream, k.s, md));
     }
     QTRY(launch_reduce_gauge(c, C2(U), mom, 4));
@@ -1243,7 +1249,7 @@ int qed2d_hmc_rhmc(qed2d_ctx* ctx, double* U, int nf, const double* am0, double 
     } else {
         GraphKey k;
         k.i(3).p(U).p(mom).p(X).p(g5DX).i(nf).d(eps).i(ns).i(maxiter).d(tol).d(c.beta);
-        k.i(c.precision).i(c.res_on[0]).i(c.res_on[1]).i(c.res_on[2]).i(c.sched[0]).i(c.sched[1]).i(c.sched[2]).i(c.ms_layout).i((long long)c.ws_gen);
+        k.i(c.precision).i(c.res_on[0]).i(c.res_on[1]).i(c.ms_sched_set).i(c.ms_layout_set).i(c.sched[0]).i(c.sched[1]).i(c.sched[2]).i(c.ms_layout).i((long long)c.ws_gen);
         for (int j = 0; j < nf; j++) {
             k.p(F[j]).d(am0[j]).i(rprm[j].n);
             for (int i = 0; i < rprm[j].n; i++) k.d(rprm[j].mu[i]).d(rprm[j].rho[i]);

@@ -89,7 +89,8 @@ struct Ctx {
     int sched[3] = {-1, -1, -1};   // reduction schedule of the F64 / MIXED / multishift solvers (-1: not tuned yet)
     int ms_layout = -1;            // layout of the multishift kernel (kMsLayouts; -1: tuned with the schedule)
     ResPlan res_plan[2];           // split of the on-chip F64 / MIXED solver (K < 0: not planned, 0: does not fit)
-    bool res_on[3] = {false, false, false};   // sched[i] was chosen by the library and stands for the on-chip form
+    bool res_on[2] = {false, false};   // sched[i] was chosen by the library and stands for the on-chip form
+    bool ms_sched_set = false, ms_layout_set = false;   // sched[2], ms_layout are the caller's: no multishift solve on chip
     bool on_chip[4] = {};          // the last solve of each solver (as sched) and pure-gauge integration ran on chip
     ResPlan res_gauge;             // split of the on-chip pure-gauge integration (K < 0: not planned, 0: does not fit)
     std::map<int, ResPlan> res_ms;   // splits of the on-chip multishift solver by the number of shifts

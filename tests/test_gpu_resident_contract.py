@@ -160,3 +160,35 @@ def test_which_batches_run_on_chip(sizes):
     b.schedule = 5 if b.uniform else 2
     b.cg(b.field(), U, src, 1.0, 2000, 1e-12)
     assert not b.on_chip
+
+
+def test_multishift_route_does_not_depend_on_earlier_calls():
+    """Solves with a single shift, or with more shifts than the chip holds, run another form;
+    the next one that fits is on chip again, with the same bits.  A layout set after an
+    on-chip solve is tuned with its schedule, not run with the number that stood for the
+    on-chip form."""
+    import qed2d as q
+    L = 160
+    prm = q.LattParm((L, L), 4.0)
+    U, b = to_dev(hot_links(L, L, 3)), to_dev(cgauss(L, L, 4, 2))
+
+    def solve(n):
+        xs = [q.cfield(L, L) for _ in range(n)]
+        q.multishift_CG(xs, U, b, 0.5, [0.1 + 0.05 * i for i in range(n)], 2000, 1e-20, prm)
+        return [to_host(x) for x in xs], q.on_chip(prm, "multishift")
+
+    first, on = solve(4)
+    assert on and q.get_multishift_layout(prm) == -1
+    for n in (1, 32, 12):
+        _, on = solve(n)
+        assert on == (n == 12) and q.get_schedule(prm, "multishift") in (0, 1, 2)
+        again, on = solve(4)
+        assert on and all(np.array_equal(x, y) for x, y in zip(first, again))
+    q.set_multishift_layout(prm, -1)
+    solve(4)
+    q.set_multishift_layout(prm, 0)
+    assert q.get_schedule(prm, "multishift") == -1
+    _, on = solve(4)
+    assert not on and q.get_multishift_layout(prm) == 0 and q.get_schedule(prm, "multishift") in (0, 1, 2)
+    q.set_multishift_layout(prm, -1)
+    assert solve(4)[1]
