@@ -944,9 +944,10 @@ struct qed2d_batch {
         ws[name] = {p, bytes};
         return p;
     }
-    // The on-chip solver (resident.cu): one class of replicas per size, each a launch.
+    // The on-chip solver (resident.cu): classes of replicas, each a launch.
     struct ResClass {
-        ResPlan plan;
+        ResGeom geom;
+        double work;
         int n, nteams;
         const ResRep* d_reps;
         void* slots;
@@ -1210,11 +1211,15 @@ int tune_ragged(qed2d_batch* h, const RCGP& P, const CCGP& C, int maxiter, Launc
 template <class T>
 int upload(T** d, const std::vector<T>& v);
 
-// Plans the on-chip solver: replicas of one size are a class with a split of its
-// own.  Classes run side by side, the one with the most work on the batch's stream
-// and each other on its own: clusters stream through the SMs that the others leave.  Teams
-// larger than a cluster wait for one another over the whole GPU, so their classes
-// share the batch's stream, where two such launches never overlap.
+// Plans the on-chip solver: every size gets a split of its own, and sizes whose teams have as
+// many blocks (clusters), or of whose teams as many fit on the device (grids), make a class,
+// one launch: its teams and blocks are those of the largest member, and its replicas come
+// longest first.  (A launch for each size took 7.1 ms for 96 lattices of as many sizes
+// from 16 x 16 to 64 x 64, on nine streams, and 2.0 ms in the other forms.)  Classes run
+// side by side, the one with the most work on the batch's stream and each other on its own:
+// clusters stream through the SMs that the others leave.  Teams larger than a cluster wait
+// for one another over the whole GPU, so their classes share the batch's stream, where two
+// such launches never overlap.
 int res_plan_classes(qed2d_batch* h) {
     h->res_fits = 0;
     std::map<std::pair<int, int>, std::vector<int>> by;
@@ -1227,14 +1232,26 @@ int res_plan_classes(qed2d_batch* h) {
     }
     const std::vector<ResPlan> plans = res_plan_batch(sizes, n, h->num_sms);
     if (plans.empty()) return QED2D_OK;
-    std::vector<ResRep> reps;
+    std::map<std::vector<int>, std::vector<size_t>> classes;   // (rows of a column, cluster, blocks or teams) -> sizes
     for (size_t i = 0; i < sizes.size(); i++) {
+        const ResPlan& p = plans[i];
+        classes[{p.K, p.cl, p.cl ? p.blocks() : h->num_sms / p.blocks()}].push_back(i);
+    }
+    std::vector<ResRep> reps;
+    for (auto& kv : classes) {
+        std::vector<size_t>& m = kv.second;
+        std::stable_sort(m.begin(), m.end(), [&](size_t a, size_t b) { return plans[a].cost > plans[b].cost; });
         qed2d_batch::ResClass c{};
-        c.plan = plans[i];
-        c.n = n[i];
-        c.nteams = c.plan.cl ? c.n : std::min(c.n, h->num_sms / c.plan.blocks());
-        for (int r : by[sizes[i]])
-            reps.push_back(res_rep(c.plan, sizes[i].first, sizes[i].second, h->reps[r].off, 0.0, r));
+        c.geom = res_geom(plans[m[0]]);
+        for (size_t i : m) {
+            const ResPlan& p = plans[i];
+            c.geom = res_join(c.geom, res_geom(p));
+            c.n += n[i];
+            c.work += p.cost * p.blocks() * n[i];
+            for (int r : by[sizes[i]])
+                reps.push_back(res_rep(p, sizes[i].first, sizes[i].second, h->reps[r].off, 0.0, r));
+        }
+        c.nteams = c.geom.cl ? c.n : std::min(c.n, h->num_sms / c.geom.nb);
         h->res.push_back(c);
     }
     ResRep* d = (ResRep*)h->buf("res_reps", sizeof(ResRep) * reps.size());
@@ -1247,22 +1264,22 @@ int res_plan_classes(qed2d_batch* h) {
         auto& c = h->res[i];
         c.d_reps = d + at;
         at += c.n;
-        c.slots = h->buf("res_slots_" + std::to_string(i), res_slot_bytes(c.plan, c.nteams));
+        c.slots = h->buf("res_slots_" + std::to_string(i), res_slot_bytes(c.geom, c.nteams));
         if (!c.slots) return QED2D_ERR_NO_MEMORY;
     }
-    // grid teams first, then the longest
+    // grid teams first, then the most work
     std::stable_sort(h->res.begin(), h->res.end(), [](const qed2d_batch::ResClass& a, const qed2d_batch::ResClass& b) {
-        if (a.plan.cl != b.plan.cl) return a.plan.cl < b.plan.cl;
-        return a.plan.cost * a.plan.blocks() * a.n > b.plan.cost * b.plan.blocks() * b.n;
+        if (a.geom.cl != b.geom.cl) return a.geom.cl < b.geom.cl;
+        return a.work > b.work;
     });
-    const bool grid = !h->res[0].plan.cl;
+    const bool grid = !h->res[0].geom.cl;
     if (h->res.size() > 1) QCHECK(cudaEventCreateWithFlags(&h->res_fork, cudaEventDisableTiming));
     constexpr size_t kSides = 8;   // streams beside the batch's; further classes follow on them
     std::vector<cudaStream_t> sides;
     size_t k = 0;
     for (size_t i = 0; i < h->res.size(); i++) {
         auto& c = h->res[i];
-        if (!c.plan.cl || (i == 0 && !grid)) continue;
+        if (!c.geom.cl || (i == 0 && !grid)) continue;
         if (sides.size() < kSides) {
             cudaStream_t s = nullptr;
             QCHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -1300,7 +1317,7 @@ int res_solve_batch(qed2d_batch* h, const double2* U, const double2* b, double2*
         a.ctl = h->ctl;
         a.reset = false;
         if (c.side) QCHECK(cudaStreamWaitEvent(c.side, h->res_fork, 0));
-        const int l = res_launch(a, c.plan, c.nteams, c.side ? c.side : h->stream);
+        const int l = res_launch(a, c.geom, c.nteams, c.side ? c.side : h->stream);
         if (c.side) QCHECK(cudaEventRecord(c.done, c.side));
         if (st == QED2D_OK) st = l;
     }

@@ -1284,11 +1284,11 @@ static int cg_resident(Ctx& c, const SolveArgs& a, int slot) {
     r.maxiter = a.maxiter;
     r.guess = a.guess ? 1 : 0;
     r.out = (ResOut*)c.buf("res_out", sizeof(ResOut));
-    r.slots = c.buf(slot ? "res_slots" : "res_slots64", res_slot_bytes(p, 1));
+    r.slots = c.buf(slot ? "res_slots" : "res_slots64", res_slot_bytes(res_geom(p), 1));
     r.ctl = c.ctl;
     r.single = 1;
     if (!r.t64 || !r.r64 || !r.out || !r.slots) return QED2D_ERR_NO_MEMORY;
-    return res_launch(r, p, 1, c.stream);
+    return res_launch(r, res_geom(p), 1, c.stream);
 }
 
 int cg_solve(Ctx& c, const SolveArgs& a, int precision) {
@@ -1522,7 +1522,7 @@ static int multishift_resident(Ctx& c, const ResPlan& p, const double2* U, const
     r.eps = eps;
     r.maxiter = maxiter;
     r.out = (ResOut*)c.buf("res_out", sizeof(ResOut));
-    r.slots = c.buf("res_slots_ms", res_slot_bytes(p, 1));
+    r.slots = c.buf("res_slots_ms", res_slot_bytes(res_geom(p), 1));
     r.ctl = c.ctl;
     r.single = 1;
     if (!r.t64 || !r.out || !r.slots) return QED2D_ERR_NO_MEMORY;

@@ -7,8 +7,8 @@
 namespace qed2d {
 
 // resident_f64.cu
-int res_f64_clusters(const ResPlan& p);
-int res_f64_launch(const ResP& P, const ResPlan& plan, cudaStream_t stream);
+int res_f64_clusters(const ResGeom& g);
+int res_f64_launch(const ResP& P, const ResGeom& g, cudaStream_t stream);
 int res_ms_limit(int device, size_t* limit);
 bool res_ms_fits(const ResPlan& p, int n, size_t limit);
 int res_ms_launch(const ResP& P, const ResPlan& plan, const ResMs& m, cudaStream_t stream);
@@ -53,10 +53,14 @@ ResRep res_rep(const ResPlan& p, int L1, int L2, long long off, double m2, int i
     return ResRep{L1, L2, off, m2, p.ntx, p.nty, p.bx, p.by, p.wx, p.wy, id, 0};
 }
 
-// clusters of this plan that the device runs at a time
-int res_clusters(const ResPlan& p) {
-    if (p.f64) return res_f64_clusters(p);
-    return p.K == 1 ? res_clusters_k<float, 1>(p) : p.K == 2 ? res_clusters_k<float, 2>(p) : res_clusters_k<float, 4>(p);
+ResGeom res_geom(const ResPlan& p) {
+    return ResGeom{p.K, p.cl, p.f64, p.blocks(), p.wx * p.wy, res_slots(p, p.f64 ? 2 : 1)};
+}
+
+// clusters of this shape that the device runs at a time
+int res_clusters(const ResGeom& g) {
+    if (g.f64) return res_f64_clusters(g);
+    return g.K == 1 ? res_clusters_k<float, 1>(g) : g.K == 2 ? res_clusters_k<float, 2>(g) : res_clusters_k<float, 4>(g);
 }
 
 // A single lattice: the split with the least time.  Clusters of up to 16 blocks
@@ -69,7 +73,7 @@ ResPlan res_plan_single(int L1, int L2, int nb, bool f64) {
         best.K = 0;
         for (const ResPlan& p : res_plans(L1, L2, nb, mc, f64))
             if (!best.K || p.cost < best.cost) best = p;
-        if (best.K == 0 || !best.cl || res_clusters(best) > 0) return best;
+        if (best.K == 0 || !best.cl || res_clusters(res_geom(best)) > 0) return best;
     }
     return ResPlan{};
 }
@@ -98,7 +102,7 @@ int res_plan_ms(int L1, int L2, int nb, int n, int device, ResPlan* best) {
 // Modelled time per iteration of n equal lattices under plan p: rounds of as many
 // teams as run at a time.
 static double res_time(const ResPlan& p, int n, int num_sms) {
-    const int at = p.cl ? res_clusters(p) : num_sms / p.blocks();
+    const int at = p.cl ? res_clusters(res_geom(p)) : num_sms / p.blocks();
     if (at < 1) return 1e30;
     const int m = std::min(n, at), share = ceil_div(m * p.blocks(), num_sms);
     return ceil_div(n, at) * res_cost(p.K, p.wx * p.wy, p.bx, p.by, p.cl, share, p.f64);
@@ -115,7 +119,7 @@ std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& size
     for (const auto& sz : sizes) {
         cand.push_back({});
         for (const ResPlan& p : res_plans(sz.first, sz.second, num_sms, kResCluster, false))
-            if (!p.cl || res_clusters(p) > 0) cand.back().push_back(p);
+            if (!p.cl || res_clusters(res_geom(p)) > 0) cand.back().push_back(p);
         if (cand.back().empty()) return {};
     }
     if (sizes.size() == 1) {
@@ -145,19 +149,18 @@ std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& size
     return out;
 }
 
-size_t res_slot_bytes(const ResPlan& p, int nteams) {
-    const size_t nslots = res_slots(p, p.f64 ? 2 : 1), nb = p.blocks();
-    if (p.cl) return 16;
-    return sizeof(ulonglong2) * nteams * (nb * (2 * nslots + 4) + kResAcc / 2) + 16;
+size_t res_slot_bytes(const ResGeom& g, int nteams) {
+    if (g.cl) return 16;
+    return sizeof(ulonglong2) * nteams * ((size_t)g.nb * (2 * g.nslots + 4) + kResAcc / 2) + 16;
 }
 
 // the kernel's parameters; clears the slots
-static int res_fill(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream, ResP& P) {
+static int res_fill(const ResArgs& a, const ResGeom& g, int nteams, cudaStream_t stream, ResP& P) {
     P.reps = a.reps;
     P.rep0 = a.rep0;
     P.nrep = a.nrep;
     P.nteams = nteams;
-    P.nb = plan.blocks();
+    P.nb = g.nb;
     P.U = a.U;
     P.b = a.b;
     P.x = a.x;
@@ -169,7 +172,7 @@ static int res_fill(const ResArgs& a, const ResPlan& plan, int nteams, cudaStrea
     P.maxiter = a.maxiter;
     P.guess = a.guess;
     P.want_g5 = a.want_g5;
-    P.nslots = res_slots(plan, plan.f64 ? 2 : 1);
+    P.nslots = g.nslots;
     P.psum = (ulonglong2*)a.slots;
     P.slots = P.psum + (size_t)nteams * 4 * P.nb;
     P.acc = (u64*)(P.slots + (size_t)nteams * P.nb * 2 * P.nslots);
@@ -179,27 +182,27 @@ static int res_fill(const ResArgs& a, const ResPlan& plan, int nteams, cudaStrea
     P.ctl = a.ctl;
     P.single = a.single;
     if (a.reset) QCHECK(cudaMemsetAsync(&a.ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), stream));
-    if (!plan.cl) QCHECK(cudaMemsetAsync(a.slots, 0, res_slot_bytes(plan, nteams), stream));
+    if (!g.cl) QCHECK(cudaMemsetAsync(a.slots, 0, res_slot_bytes(g, nteams), stream));
     return QED2D_OK;
 }
 
-int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream) {
+int res_launch(const ResArgs& a, const ResGeom& g, int nteams, cudaStream_t stream) {
     ResP P{};
-    QTRY(res_fill(a, plan, nteams, stream, P));
-    if (plan.f64) return res_f64_launch(P, plan, stream);
-    switch (plan.K * 2 + plan.cl) {
-        case 2: return res_launch_k<float, 1, false>(P, plan, stream);
-        case 3: return res_launch_k<float, 1, true>(P, plan, stream);
-        case 4: return res_launch_k<float, 2, false>(P, plan, stream);
-        case 5: return res_launch_k<float, 2, true>(P, plan, stream);
-        case 8: return res_launch_k<float, 4, false>(P, plan, stream);
-        default: return res_launch_k<float, 4, true>(P, plan, stream);
+    QTRY(res_fill(a, g, nteams, stream, P));
+    if (g.f64) return res_f64_launch(P, g, stream);
+    switch (g.K * 2 + g.cl) {
+        case 2: return res_launch_k<float, 1, false>(P, g, stream);
+        case 3: return res_launch_k<float, 1, true>(P, g, stream);
+        case 4: return res_launch_k<float, 2, false>(P, g, stream);
+        case 5: return res_launch_k<float, 2, true>(P, g, stream);
+        case 8: return res_launch_k<float, 4, false>(P, g, stream);
+        default: return res_launch_k<float, 4, true>(P, g, stream);
     }
 }
 
 int res_launch_ms(const ResArgs& a, const ResPlan& plan, const ResShifts& s, cudaStream_t stream) {
     ResP P{};
-    QTRY(res_fill(a, plan, 1, stream, P));
+    QTRY(res_fill(a, res_geom(plan), 1, stream, P));
     ResMs M{};
     M.n = s.n;
     M.base = s.base;

@@ -1334,27 +1334,26 @@ inline int res_allow_smem(const void* kern) {
 inline int res_slots(const ResPlan& p, int per) { return per * (2 * p.wy * p.K + 2 * p.wx * 32); }   // of one buffer of a block
 
 template <class R, int K>
-static size_t res_smem(const ResPlan& p) {
-    return ResSm<R, K>::bytes(p.wx * p.wy) +
-           (p.cl ? sizeof(ulonglong2) * (4 * kResCluster + 2 * res_slots(p, Num<R>::SLOTS)) : 0);
+static size_t res_smem(const ResGeom& g) {
+    return ResSm<R, K>::bytes(g.nw) + (g.cl ? sizeof(ulonglong2) * (4 * kResCluster + 2 * g.nslots) : 0);
 }
 
 template <class R, int K>
-static int res_clusters_k(const ResPlan& plan) {
+static int res_clusters_k(const ResGeom& g) {
     const void* kern = (const void*)k_res_cg<R, K, true>;
-    const size_t sm = res_smem<R, K>(plan);
+    const size_t sm = res_smem<R, K>(g);
     if (res_allow_smem(kern) != QED2D_OK ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan.blocks());
-    cfg.blockDim = dim3(32 * (plan.wx * plan.wy + 1));
+    cfg.gridDim = dim3(g.nb);
+    cfg.blockDim = dim3(32 * (g.nw + 1));
     cfg.dynamicSmemBytes = sm;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = plan.blocks();
+    at[0].val.clusterDim.x = g.nb;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
@@ -1368,14 +1367,14 @@ static int res_clusters_k(const ResPlan& plan) {
 }
 
 template <class R, int K, bool CL>
-static int res_launch_k(const ResP& P, const ResPlan& plan, cudaStream_t stream) {
+static int res_launch_k(const ResP& P, const ResGeom& g, cudaStream_t stream) {
     const void* kern = (const void*)k_res_cg<R, K, CL>;
-    const size_t sm = res_smem<R, K>(plan);
+    const size_t sm = res_smem<R, K>(g);
     QTRY(res_allow_smem(kern));
     if (CL) QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P.nb * P.nteams);
-    cfg.blockDim = dim3(32 * (plan.wx * plan.wy + 1));
+    cfg.blockDim = dim3(32 * (g.nw + 1));
     cfg.dynamicSmemBytes = sm;
     cfg.stream = stream;
     cudaLaunchAttribute at[1];

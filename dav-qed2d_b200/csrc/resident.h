@@ -28,10 +28,24 @@ struct ResOut {
     double rr, bb;
 };
 
+// Shape of a launch: blocks of a team, worker warps of a block, halo slots of a block's buffer.
+struct ResGeom {
+    int K, cl, f64, nb, nw, nslots;
+};
+ResGeom res_geom(const ResPlan& p);
+// one that runs both (of the same K, cl and f64): teams and blocks of the larger, parts of
+// which idle in the smaller's systems
+inline ResGeom res_join(ResGeom a, const ResGeom& b) {
+    a.nb = a.nb > b.nb ? a.nb : b.nb;
+    a.nw = a.nw > b.nw ? a.nw : b.nw;
+    a.nslots = a.nslots > b.nslots ? a.nslots : b.nslots;
+    return a;
+}
+
 // K = 0 where the state does not fit on chip
 ResPlan res_plan_single(int L1, int L2, int nb, bool f64);
 std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& sizes, const std::vector<int>& n, int num_sms);
-int res_clusters(const ResPlan& p);
+int res_clusters(const ResGeom& g);
 ResRep res_rep(const ResPlan& p, int L1, int L2, long long off, double m2, int id);
 
 struct ResArgs {
@@ -48,7 +62,7 @@ struct ResArgs {
     int maxiter = 0, guess = 0;
     int want_g5 = 0;                // FP64: t64 = g5Dw x is wanted (the mixed solver always leaves it)
     ResOut* out = nullptr;          // [nrep]
-    void* slots = nullptr;          // res_slot_bytes(plan, nteams)
+    void* slots = nullptr;          // res_slot_bytes(geom, nteams)
     DevCtl* ctl = nullptr;
     bool reset = true;              // clear the control block's error flag first
     int single = 0;                 // write the context's record of the solve
@@ -70,8 +84,8 @@ struct ResMd {
 };
 bool res_gauge_fits(Ctx& c);
 int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s);
-size_t res_slot_bytes(const ResPlan& p, int nteams);
-// one launch: nteams teams of plan.blocks() blocks solve the nrep systems
-int res_launch(const ResArgs& a, const ResPlan& plan, int nteams, cudaStream_t stream);
+size_t res_slot_bytes(const ResGeom& g, int nteams);
+// one launch: nteams teams of geom.nb blocks solve the nrep systems
+int res_launch(const ResArgs& a, const ResGeom& geom, int nteams, cudaStream_t stream);
 
 }  // namespace qed2d

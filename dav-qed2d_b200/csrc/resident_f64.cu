@@ -4,16 +4,16 @@
 
 namespace qed2d {
 
-int res_f64_clusters(const ResPlan& p) {
-    return p.K == 1 ? res_clusters_k<double, 1>(p) : res_clusters_k<double, 2>(p);
+int res_f64_clusters(const ResGeom& g) {
+    return g.K == 1 ? res_clusters_k<double, 1>(g) : res_clusters_k<double, 2>(g);
 }
 
-int res_f64_launch(const ResP& P, const ResPlan& plan, cudaStream_t stream) {
-    switch (plan.K * 2 + plan.cl) {
-        case 2: return res_launch_k<double, 1, false>(P, plan, stream);
-        case 3: return res_launch_k<double, 1, true>(P, plan, stream);
-        case 4: return res_launch_k<double, 2, false>(P, plan, stream);
-        default: return res_launch_k<double, 2, true>(P, plan, stream);
+int res_f64_launch(const ResP& P, const ResGeom& g, cudaStream_t stream) {
+    switch (g.K * 2 + g.cl) {
+        case 2: return res_launch_k<double, 1, false>(P, g, stream);
+        case 3: return res_launch_k<double, 1, true>(P, g, stream);
+        case 4: return res_launch_k<double, 2, false>(P, g, stream);
+        default: return res_launch_k<double, 2, true>(P, g, stream);
     }
 }
 

@@ -5,7 +5,7 @@ import threading
 import numpy as np
 import pytest
 
-from helpers import cgauss, hot_links, note, to_dev, to_host
+from helpers import bound, cgauss, hot_links, note, rel, to_dev, to_host
 
 pytestmark = pytest.mark.gpu
 
@@ -192,3 +192,27 @@ def test_multishift_route_does_not_depend_on_earlier_calls():
     assert not on and q.get_multishift_layout(prm) == 0 and q.get_schedule(prm, "multishift") in (0, 1, 2)
     q.set_multishift_layout(prm, -1)
     assert solve(4)[1]
+
+
+def test_many_sizes_share_launches():
+    """A batch of 44 sizes, four of them beyond a cluster: sizes with like teams share a launch
+    (whose teams and blocks are those of its largest member, in part idle for the others), so
+    a solve makes far fewer launches than it has sizes.  Against the grid solver: as the
+    uneven batches of test_gpu_resident.py (1e-11)."""
+    import qed2d
+    sizes = [(16 + 2 * i, 17 + 3 * i) for i in range(40)] + [(180, 190), (200, 200), (201, 230), (250, 170)]
+    am0 = [0.2 + 0.05 * (r % 5) for r in range(len(sizes))]
+    b = qed2d.Batch.ragged(sizes, [4.0] * len(sizes))
+    U, src, x, x2 = (b.field() for _ in range(4))
+    for r, s in enumerate(sizes):
+        b.replica(U, r).copy_(to_dev(hot_links(*s, 900 + r)))
+        b.replica(src, r).copy_(to_dev(cgauss(*s, 950 + r, 2)))
+    b.cg(x, U, src, am0, 20000, 1e-24)
+    assert b.on_chip
+    n0 = qed2d.lib().qed2d_launch_count()
+    it, _ = b.cg(x, U, src, am0, 20000, 1e-24)
+    assert qed2d.lib().qed2d_launch_count() - n0 < len(sizes) // 2
+    b.schedule = 2
+    it2, _ = b.cg(x2, U, src, am0, 20000, 1e-24)
+    bound("on-chip batch of many sizes vs grid solver", rel(to_host(x), to_host(x2)), 1e-11)
+    assert all(abs(p - q) <= 2 + q // 100 for p, q in zip(it, it2)), (it, it2)
