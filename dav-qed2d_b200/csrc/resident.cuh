@@ -1321,13 +1321,13 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_cg(const __grid
 // launches it: every launch and query asks for all that the device has beside the kernel's
 // static shared memory, so that host threads with contexts of other sizes, which share the
 // function, never lower the limit under one another's launches.
-inline int res_allow_smem(const void* kern) {
+// (The static part is taken from the types: asking the driver costs 3 us a launch.)
+inline int res_allow_smem(const void* kern, size_t static_bytes = sizeof(ResBlock)) {
     int dev = 0, optin = 0;
-    cudaFuncAttributes fa{};
     QCHECK(cudaGetDevice(&dev));
     QCHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    QCHECK(cudaFuncGetAttributes(&fa, kern));
-    QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                optin - (int)((static_bytes + 15) / 16 * 16)));
     return QED2D_OK;
 }
 

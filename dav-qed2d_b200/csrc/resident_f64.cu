@@ -138,12 +138,12 @@ static size_t res_ms_smem(const ResPlan& p, int n) {
     return p.K == 1 ? ResMsSm<1>::bytes(nw, n) : ResMsSm<2>::bytes(nw, n);
 }
 
+constexpr size_t kMsStatic = (sizeof(ResBlock) + 15) / 16 * 16 + sizeof(ResMsBlock);   // static shared memory of k_res_ms
+
 int res_ms_limit(int device, size_t* limit) {
     int optin = 0;
-    cudaFuncAttributes fa{};
     QCHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    QCHECK(cudaFuncGetAttributes(&fa, (const void*)k_res_ms<1>));
-    *limit = (size_t)optin - fa.sharedSizeBytes;
+    *limit = (size_t)optin - (kMsStatic + 15) / 16 * 16;
     return QED2D_OK;
 }
 
@@ -159,7 +159,7 @@ int res_ms_launch(const ResP& P0, const ResPlan& plan, const ResMs& m, cudaStrea
     M.nw = nw;
     const size_t sm = res_ms_smem(plan, M.n);
     const void* kern = plan.K == 1 ? (const void*)k_res_ms<1> : (const void*)k_res_ms<2>;
-    QTRY(res_allow_smem(kern));
+    QTRY(res_allow_smem(kern, kMsStatic));
     const int items = nw * plan.K * (M.n - 1), shift_warps = items < kResWarps - nw ? items : kResWarps - nw;
     void* args[] = {(void*)&P, (void*)&M};
     QCHECK(cudaLaunchCooperativeKernel(kern, dim3(P.nb), dim3(32 * (1 + nw + shift_warps)), args, sm, stream));
