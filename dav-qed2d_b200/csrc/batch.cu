@@ -1294,7 +1294,7 @@ int res_plan_classes(qed2d_batch* h) {
     return QED2D_OK;
 }
 
-int res_solve_batch(qed2d_batch* h, const double2* U, const double2* b, double2* x, double2* g5x, int maxiter, double eps) {
+int res_enqueue(qed2d_batch* h, const double2* U, const double2* b, double2* x, double2* g5x, int maxiter, double eps) {
     double2* r64 = h->field("b_r64");
     if (!r64) return QED2D_ERR_NO_MEMORY;
     QCHECK(cudaMemsetAsync(&h->ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), h->stream));
@@ -1323,25 +1323,75 @@ int res_solve_batch(qed2d_batch* h, const double2* U, const double2* b, double2*
     }
     for (auto& c : h->res)
         if (c.side) QCHECK(cudaStreamWaitEvent(h->stream, c.done, 0));
-    if (st != QED2D_OK) return st;
+    return st;
+}
+
+int res_solve_batch(qed2d_batch* h, const double2* U, const double2* b, double2* x, double2* g5x, int maxiter, double eps) {
+    QTRY(res_enqueue(h, U, b, x, g5x, maxiter, eps));
     k_r_finish_res<<<1, 256, 0, h->stream>>>(h->d_resout, h->nrep, h->d_out, h->d_out + h->nrep, h->d_iters, h->ctl);
     return r_post("k_r_finish_res");
 }
 
+// From now on solves run on chip (until a schedule or a tile height is set).
+void res_choose(qed2d_batch* h) {
+    h->res_on = h->on_chip = true;
+    if (h->uniform) {
+        h->usched = 9;
+        h->utile = 0;
+    } else {
+        h->rsched = 6;
+    }
+}
+
+// First solve of a batch whose state fits on chip, once the other forms are tuned: times
+// `other` (the fastest of them) against the on-chip form on the caller's operator and
+// sources, capped at kRaceIters iterations, into the tuner's scratch outputs, and keeps
+// the faster; the control block is saved and restored.  On chip wins where few rounds of
+// teams hold the batch (per iteration: 37 x 64^2 7.9 -> 3.9 us, 5 x 256^2 12.2 -> 8.6, 4 x
+// 512^2 23.9 -> 18.5), and not where splits waste blocks while the other forms' working set
+// stays in L2 (64 x 128^2 21.8 -> 26.6, 16 x 256^2 23.4 -> 25.3, 8 x 384^2 25.8 -> 30.6).
+// QED2D_TUNE=0: on chip wherever it fits.
+constexpr int kRaceIters = 100;
+
+template <class Other>
+int race_on_chip(qed2d_batch* h, const double2* U, const double2* b, int maxiter, double eps, Other other) {
+    DevCtl saved;
+    QCHECK(cudaMemcpyAsync(&saved, h->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
+    QCHECK(cudaStreamSynchronize(h->stream));
+    double2 *x = h->field("tune_x"), *g5x = h->field("tune_g5x");
+    if (!x || !g5x) return QED2D_ERR_NO_MEMORY;
+    const int iters = std::min(maxiter, kRaceIters);
+    cudaEvent_t e0, e1;
+    QCHECK(cudaEventCreate(&e0));
+    QCHECK(cudaEventCreate(&e1));
+    float best[2] = {1e30f, 1e30f};
+    int st = QED2D_OK;
+    for (int rep = 0; rep < 3; rep++)
+        for (int c = 0; c < 2 && st == QED2D_OK; c++) {
+            cudaEventRecord(e0, h->stream);
+            st = c ? other(x, g5x, iters) : res_enqueue(h, U, b, x, g5x, iters, eps);
+            cudaEventRecord(e1, h->stream);
+            if (cudaEventSynchronize(e1) != cudaSuccess) st = cuda_status(cudaGetLastError(), "schedule tuning");
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, e0, e1);
+            if (rep > 0) best[c] = std::min(best[c], ms);   // the first round warms up
+        }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    QCHECK(cudaMemcpyAsync(h->ctl, &saved, sizeof(DevCtl), cudaMemcpyHostToDevice, h->stream));
+    QCHECK(cudaStreamSynchronize(h->stream));
+    if (st == QED2D_OK && best[0] <= best[1]) res_choose(h);
+    return st;
+}
+
 int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* b, double2* x, double2* g5x,
             int maxiter, double eps) {
-    // No schedule and no tile height set: on chip wherever every replica fits there.
+    // No schedule and no tile height set: on chip where every replica fits there and that is faster.
+    bool race = false;
     if (h->uniform ? (!h->usched_fixed && !h->utile_fixed && (h->usched < 0 || h->utile < 0)) : h->rsched < 0) {
         if (h->res_fits < 0) QTRY(res_plan_classes(h));
-        if (h->res_fits) {
-            h->res_on = true;
-            if (h->uniform) {
-                h->usched = 9;
-                h->utile = 0;
-            } else {
-                h->rsched = 6;
-            }
-        }
+        race = h->res_fits && tuning_enabled();
+        if (h->res_fits && !race) res_choose(h);
     }
     h->on_chip = h->res_on;
     if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
@@ -1445,6 +1495,16 @@ int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* 
             return QED2D_OK;
         };
         if (h->usched < 0 || h->utile < 0) QTRY(tune_uniform(h, Q, maxiter, launch));
+        if (race) {
+            QTRY(race_on_chip(h, U, b, maxiter, eps, [&](double2* tx, double2* tg, int iters) -> int {
+                UCGP T = Q;
+                T.x = tx;
+                T.t64 = tg;
+                T.maxiter = iters;
+                return launch(h->usched, h->utile, T);
+            }));
+            if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
+        }
         QTRY(launch(h->usched, h->utile, Q));
         k_r_finish<<<1, 256, 0, h->stream>>>(h->d_st, h->nrep, maxiter, h->d_out, h->d_out + h->nrep, h->d_iters,
                                               h->ctl);
@@ -1485,6 +1545,17 @@ int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* 
             return QED2D_OK;
         };
         if (h->rsched < 0) QTRY(tune_ragged(h, P, C, maxiter, launch));
+        if (race) {
+            QTRY(race_on_chip(h, U, b, maxiter, eps, [&](double2* tx, double2* tg, int iters) -> int {
+                RCGP TP = P;
+                CCGP TC = C;
+                TP.x = TC.x = tx;
+                TP.t64 = TC.t64 = tg;
+                TP.maxiter = TC.maxiter = iters;
+                return launch(h->rsched, TP, TC, h->rcs);
+            }));
+            if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
+        }
         QTRY(launch(h->rsched, P, C, h->rcs));
     }
     k_r_finish<<<1, 256, 0, h->stream>>>(h->d_st, h->nrep, maxiter, h->d_out, h->d_out + h->nrep, h->d_iters, h->ctl);

@@ -364,10 +364,10 @@ int qed2d_batch_set_stream(qed2d_batch* batch, void* cuda_stream);
  * barriers, 3 = one thread-block cluster per replica (no grid barrier; replicas
  * stream through the GPU, largest first), 6 = 3 with the first phase's stencil
  * on r (as 8); these group their sums differently.
- * Where no schedule (nor tile height) is set and the FP32 state of every replica
- * fits on chip (see qed2d_ctx_set_schedule), solves keep it there, in a few launches
- * that sizes with like teams of blocks share, and get reports 9 (equal sizes) or 6; otherwise
- * the first solve times the candidates and keeps the fastest; a schedule set
+ * Where no schedule (nor tile height) is set, the first solve times the candidates and
+ * keeps the fastest.  One of them, where the FP32 state of every replica fits on chip
+ * (see qed2d_ctx_set_schedule), keeps it there, in a few launches that sizes with like
+ * teams of blocks share; get then reports 9 (equal sizes) or 6.  A schedule set
  * here is kept (for equal sizes the first solve then tunes the tile height
  * only); -1 = tune again on the next solve (get: -1 while untuned). */
 int qed2d_batch_set_schedule(qed2d_batch* batch, int schedule);

@@ -216,3 +216,42 @@ def test_many_sizes_share_launches():
     it2, _ = b.cg(x2, U, src, am0, 20000, 1e-24)
     bound("on-chip batch of many sizes vs grid solver", rel(to_host(x), to_host(x2)), 1e-11)
     assert all(abs(p - q) <= 2 + q // 100 for p, q in zip(it, it2)), (it, it2)
+
+
+@pytest.mark.parametrize("sizes", [[(64, 64)] * 2, [(128, 128)] * 64, [(384, 384)] * 8, [(256, 256)] * 5,
+                                   [(16 + i, 64 - i) for i in range(48)], [(180 + 10 * i, 186 + 10 * i) for i in range(8)]])
+def test_untuned_batches_take_the_fastest_form(sizes):
+    """The form that a batch's first solve chooses is as fast as each of those that can be set
+    (the best of five solves each; 15% for the noise of short solves, and because the choice
+    itself is made on fewer iterations).  64 x 128^2 and 8 x 384^2 are slower on chip by 15
+    to 20%, the eight sizes around 200^2 were by half when each was a launch of its own."""
+    import time
+    import torch
+    import qed2d
+    g = torch.Generator(device="cuda").manual_seed(5)
+    b = (qed2d.Batch(len(sizes), *sizes[0], 4.0) if len(set(sizes)) == 1 else qed2d.Batch.ragged(sizes, [4.0] * len(sizes)))
+    U, src, x = b.field(), b.field(), b.field()
+    U.copy_(torch.polar(torch.ones(U.shape, dtype=torch.float64, device="cuda"),
+                        0.45 * torch.randn(U.shape, dtype=torch.float64, device="cuda", generator=g)))
+    src.copy_(torch.randn(src.shape, dtype=torch.complex128, device="cuda", generator=g))
+
+    def best():
+        out = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            b.cg(x, U, src, 0.15, 20000, 1e-24)
+            out.append(time.perf_counter() - t)
+        return min(out[1:])
+
+    mine = best()
+    chosen = (b.on_chip, b.schedule)
+    others = {}
+    for s in ((5, 8, 9) if b.uniform else (2, 3, 6)):
+        try:
+            b.schedule = s
+            others[s] = best()
+        except qed2d.Qed2dError:   # staged links that do not fit
+            continue
+    note(f"{len(sizes)} x {sizes[0]}: {chosen}", [mine, others])
+    assert mine <= 1.15 * min(others.values()), (chosen, mine, others)
