@@ -664,7 +664,6 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
         Sums tot{0.0, 0.0}, v;
         bool ok = true;
         bar_sync_n(1, nth);   // the workers' partials are in
-        if (next == X_FENCE) __threadfence();   // releases what the block's workers stored before this barrier
         {
             double a[4] = {0.0, 0.0, 0.0, 0.0}, c[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
@@ -693,7 +692,7 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
                 if (seq & 1u) base1 = bs;
                 else base0 = bs;
             }
-            if (!exact && next != X_FENCE && ok) ok = team_sum_slots<NV>(B.C, seq, v, tot);
+            if (!exact && ok) ok = team_sum_slots<NV>(B.C, seq, v, tot);
         }
         double alpha = 0.0;
         const double inv_old = inv_rr;
@@ -736,10 +735,6 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
                 fresh = false;
                 rr = tot.g;
             }
-        } else if (next == X_FENCE) {   // orders the blocks' FP64 stores: the others' are acquired
-            __threadfence();
-            if (flag == RF_FIN) flag = RF_STOP;
-            if (--fences == 0) next = X_TRUE;
         } else if (next == X_BEGIN) {   // |b|^2
             bb = rr64 = tot.g;
             tol = P.eps * bb;
@@ -815,6 +810,40 @@ __device__ __forceinline__ unsigned res_scalar(const ResP& P, ResBlock& B, unsig
         if (!MIXED && alpha != 0.0) inv_a = 1.0 / alpha;
         maxrr = fmax(maxrr, rr);
         thr = fmax(P.delta2 * maxrr, tol * s * s);
+        if (next == X_FENCE) {
+            // Exchanges that order the blocks' FP64 stores, apart from the loop's path (in it
+            // they cost a 64^2 mixed CG 4%).  The fences are this warp's own: the first releases
+            // what the workers stored before the barrier, the second acquires the others'.
+            do {
+                ++seq;
+                const bool lost = ld_volatile_int(&B.abort) != 0;
+                bool got = true;
+                Sums zero{0.0, 0.0}, sum;
+                bar_sync_n(1, nth);
+                __threadfence();
+                if (B.C.nb > 1) {
+                    if constexpr (CL) {
+                        got = cluster_sum_slots<1>(B.C, seq, zero, sum);
+                    } else {
+                        bool exact;
+                        u64 bs = (seq & 1u) ? base1 : base0;
+                        got = team_sum_fixed<NV>(B.C, seq, zero, 0, bs, sum, false, exact);
+                        if (seq & 1u) base1 = bs;
+                        else base0 = bs;
+                    }
+                }
+                __threadfence();
+                if (!got || lost) flag = RF_ABORT;
+                else if (flag == RF_FIN) flag = RF_STOP;
+                if (lane == 0) {
+                    if (MIXED) B.sc.cf = make_float2(0.f, __int_as_float(flag));
+                    else B.sc.flag = flag;
+                }
+                bar_sync_n(3, nth);
+            } while (--fences > 0 && flag < RF_STOP);
+            if (flag >= RF_STOP) break;
+            next = X_TRUE;
+        }
         ex = fixed_exponent(Sums{next == X_RR ? rr_last : next == X_PAP ? (MIXED ? pap_last : dir_est) : next == X_TRUE ? rr64 : 1.0, pap_last});
     }
     if (flag != RF_ABORT && B.C.rank == 0 && lane == 0) {
