@@ -1269,8 +1269,7 @@ static int tune_cg(Ctx& c, const CGP& P, int slot) {
 // B200: mixed 64^2 4.85 -> 1.95 us, 128^2 5.95 -> 2.7, 256^2 7.1 -> 3.5, 512^2 12.3 ->
 // 4.3; FP64 64^2 5.13 -> 2.2, 128^2 6.4 -> 3.1, 256^2
 // 8.05 -> 4.05, 350x370 11.1 -> 6.8.
-static int cg_resident(Ctx& c, const SolveArgs& a, int slot) {
-    const ResPlan& p = c.res_plan[slot];
+static int cg_resident(Ctx& c, const SolveArgs& a, int slot, const ResPlan& p, int missing = 0, unsigned polls = 0) {
     ResArgs r;
     r.rep0 = res_rep(p, c.g.L1, c.g.L2, 0, 2.0 + a.am0, 0);
     r.U = a.U;
@@ -1288,7 +1287,22 @@ static int cg_resident(Ctx& c, const SolveArgs& a, int slot) {
     r.ctl = c.ctl;
     r.single = 1;
     if (!r.t64 || !r.r64 || !r.out || !r.slots) return QED2D_ERR_NO_MEMORY;
-    return res_launch(r, res_geom(p), 1, c.stream);
+    ResGeom g = res_geom(p);
+    g.missing = missing;
+    g.polls = polls;
+    return res_launch(r, g, 1, c.stream);
+}
+
+int on_chip_timeout_probe(Ctx& c, int slot, unsigned polls, double2* U, double* mom) {
+    const ResPlan p = res_plan_pair(c.g.L1, c.g.L2, slot == 0);
+    if (p.K == 0) return QED2D_ERR_UNSUPPORTED;
+    if (slot == 3) return res_gauge_md(c, mom, U, ResMd{0.1, {0.1}, {0.1}, 0.1, 1, 4, 0}, p, 1, polls);
+    SolveArgs a;
+    a.U = a.b = U;   // any source
+    a.x = c.spinor("selftest_x");
+    a.maxiter = 100;
+    if (!a.x) return QED2D_ERR_NO_MEMORY;
+    return cg_resident(c, a, slot, p, 1, polls);
 }
 
 int cg_solve(Ctx& c, const SolveArgs& a, int precision) {
@@ -1303,7 +1317,7 @@ int cg_solve(Ctx& c, const SolveArgs& a, int precision) {
         }
     }
     c.on_chip[slot] = c.res_on[slot];
-    if (c.res_on[slot]) return cg_resident(c, a, slot);
+    if (c.res_on[slot]) return cg_resident(c, a, slot, c.res_plan[slot]);
     CGP P{};
     P.g = c.g;
     P.U = a.U;

@@ -316,7 +316,7 @@ static int md_omf4_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MD
             md.u[k] = eps * cu[k];
             md.c[k] = cm[k + 1] * eps;
         }
-        return res_gauge_md(c, mom, U, md);
+        return res_gauge_md(c, mom, U, md, c.res_gauge);
     }
     GaugePingPong pp(c, U, mom, s);
     for (int i = 0; i < ns; i++) {
@@ -328,7 +328,7 @@ static int md_omf4_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MD
 
 static int md_leapfrog_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MDState& s) {
     if ((c.on_chip[3] = ns > 0 && !s.U32 && res_gauge_fits(c)))
-        return res_gauge_md(c, mom, U, ResMd{0.5 * eps, {eps}, {eps}, 0.5 * eps, 1, ns, 0});
+        return res_gauge_md(c, mom, U, ResMd{0.5 * eps, {eps}, {eps}, 0.5 * eps, 1, ns, 0}, c.res_gauge);
     GaugePingPong pp(c, U, mom, s);
     QTRY(pp.kick(0.5 * eps));
     for (int i = 0; i < ns - 1; i++) QTRY(pp.links_then_kick(eps, eps, s));
@@ -564,6 +564,18 @@ int qed2d_selftest_barrier_timeout(qed2d_ctx* ctx, int64_t polls) {
     if (polls < 1 || polls > (1LL << 26)) return bad_arg("polls must be in [1, 2^26]");
     QTRY(reset_seq(c));
     QTRY(barrier_timeout_probe(c, (long long)polls));
+    return finish_seq(c, nullptr);
+}
+
+int qed2d_selftest_on_chip_timeout(qed2d_ctx* ctx, int what, int64_t polls, double* U, double* mom) {
+    QCTX(ctx);
+    QPTR(U);
+    QPTR(mom);
+    const int slot = what == QED2D_GAUGE_MD ? 3 : sched_slot(what);
+    if (slot < 0 || slot == 2) return bad_arg("on-chip self-test: QED2D_PREC_F64, QED2D_PREC_MIXED or QED2D_GAUGE_MD only");
+    if (polls < 1 || polls > (1LL << 22)) return bad_arg("polls must be in [1, 2^22]");
+    QTRY(reset_seq(c));
+    QTRY(on_chip_timeout_probe(c, slot, (unsigned)polls, C2(U), mom));
     return finish_seq(c, nullptr);
 }
 

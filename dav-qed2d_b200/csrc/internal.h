@@ -130,6 +130,8 @@ constexpr double kReliableDelta = 0.01;
 
 // launches the bounded-wait self-test kernel (cg.cu); the status lands in ctl->status
 int barrier_timeout_probe(Ctx& c, long long polls);
+// the same for the on-chip kernels: a solve (slot 0, 1) or integration (3) on a team of two blocks without its second
+int on_chip_timeout_probe(Ctx& c, int slot, unsigned polls, double2* U, double* mom);
 
 bool tuning_enabled();   // QED2D_TUNE=0 in the environment turns schedule tuning off
 int64_t launches();

@@ -78,6 +78,14 @@ ResPlan res_plan_single(int L1, int L2, int nb, bool f64) {
     return ResPlan{};
 }
 
+ResPlan res_plan_pair(int L1, int L2, bool f64) {
+    for (const ResPlan& p : res_plans(L1, L2, 2, 0, f64))
+        if (p.blocks() == 2) return p;
+    ResPlan none;
+    none.K = 0;
+    return none;
+}
+
 // A multishift solve with n shifts: the split over a grid of blocks with the least
 // time, where the shifts' vectors fit and their updates (about 36 cycles a row and
 // shift, all in shared memory) hide behind the iteration or bound it.
@@ -181,6 +189,7 @@ static int res_fill(const ResArgs& a, const ResGeom& g, int nteams, cudaStream_t
     P.out = a.out;
     P.ctl = a.ctl;
     P.single = a.single;
+    P.polls = g.polls ? g.polls : g.cl ? kWaitPolls<true> : kWaitPolls<false>;
     if (a.reset) QCHECK(cudaMemsetAsync(&a.ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), stream));
     if (!g.cl) QCHECK(cudaMemsetAsync(a.slots, 0, res_slot_bytes(g, nteams), stream));
     return QED2D_OK;

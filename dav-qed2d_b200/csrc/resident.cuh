@@ -107,6 +107,7 @@ struct ResP {
     ResOut* out;
     DevCtl* ctl;
     int single;               // write the context's solve record
+    unsigned polls;           // after which a wait gives up
 };
 
 enum { RF_GO, RF_DIR, RF_UPD, RF_FIN, RF_STOP, RF_ZERO, RF_ABORT };   // the last three end the solve
@@ -222,18 +223,23 @@ struct TeamComm {
     u64 psum;            // the team's partials, [2][value][block], or this block's rows of them (CL)
     u64* acc;            // the team's fixed-point sums: two sets of words (not CL)
     int nb, rank, nslots;
+    unsigned polls;      // after which a wait gives up
     int* err;
 };
 
-// Bounded wait of a warp: false when *err is set or the polls run out.
+// Bounded wait of a warp: false when *err is set or the polls run out.  An exchange takes a
+// few polls, another block's FP64 update some hundreds; a wait that lasts longer (another
+// stream's work holds SMs that the rest of the grid needs, say) gives up after some 40 s,
+// as the grid barriers do: 2^26 polls of L2 or 2^30 of shared memory.
+template <bool CL> constexpr unsigned kWaitPolls = CL ? 1u << 30 : 1u << 26;
 struct Patience {
     unsigned n = 0;
-    __device__ __forceinline__ bool more(int* err) {
+    __device__ __forceinline__ bool more(const TeamComm& C) {
         if ((++n & 255u) != 0) return true;
-        const int e = ld_volatile_int(err);
+        const int e = ld_volatile_int(C.err);
         if (__any_sync(0xffffffffu, e != 0)) return false;
-        if (n <= (1u << 22)) return true;
-        if ((threadIdx.x & 31) == 0) atomicExch(err, 2 /* QED2D_ERR_TIMEOUT */);
+        if (n <= C.polls) return true;
+        if ((threadIdx.x & 31) == 0) atomicExch(C.err, 2 /* QED2D_ERR_TIMEOUT */);
         return false;
     }
 };
@@ -265,7 +271,7 @@ __device__ __forceinline__ bool team_sum_slots(const TeamComm& C, unsigned seq, 
             for (;;) {
                 q = ld_slot<false>(rows + ((u64)k * nb + min(i + lane, nb - 1)) * 16);
                 if (__all_sync(0xffffffffu, tagged(q, seq))) break;
-                if (!(ok = pt.more(C.err))) break;
+                if (!(ok = pt.more(C))) break;
             }
             if (i + lane < nb) s[k] += slot_double(q);
         }
@@ -293,7 +299,7 @@ __device__ __forceinline__ bool cluster_sum_slots(const TeamComm& C, unsigned se
     for (;;) {
         q = ld_slot<true>(row + 16 * min(from, nb - 1));
         if (__all_sync(0xffffffffu, tagged(q, seq))) break;
-        if (!(ok = pt.more(C.err))) break;
+        if (!(ok = pt.more(C))) break;
     }
     // every group of n2 lanes adds the same values in the same tree
     double s = from < nb ? slot_double(q) : 0.0;
@@ -349,7 +355,7 @@ __device__ __forceinline__ bool team_sum_fixed(const TeamComm& C, unsigned seq, 
             base = q;
             break;
         }
-        if (!(ok = pt.more(C.err))) break;
+        if (!(ok = pt.more(C))) break;
     }
     const double w = (double)(long long)(d & ((lane & 1) ? (1ull << 56) - 1 : (1ull << 48) - 1));
     const double s = (w + __shfl_xor_sync(0xffffffffu, w, 1) * 0x1p-40) * __longlong_as_double((long long)(1023 - 36 + ex) << 52);
@@ -530,7 +536,7 @@ __device__ __forceinline__ void stencil_inner(const Tile& T, const V4<R> (&S)[K]
 // arrived by then is polled.  False when a wait gave up.
 template <class R, int K, bool CL, class F>
 __device__ __forceinline__ bool stencil_faces(const Tile& T, const V2<R> (&u1)[K], const V2<R> (&u2)[K], V2<R>* box,
-                                              u64 from, int* err, unsigned seq, V4<R> (&w)[K], F meanwhile) {
+                                              u64 from, const TeamComm& C, unsigned seq, V4<R> (&w)[K], F meanwhile) {
     constexpr int BOX = ResSm<R, K>::BOX;
     constexpr bool PK = kPacked<K, CL>;
     const int lane = threadIdx.x & 31;
@@ -551,7 +557,7 @@ __device__ __forceinline__ bool stencil_faces(const Tile& T, const V2<R> (&u1)[K
     for (;;) {
         const bool ready = (!T.rd || qd.here(seq)) && (!T.ru || qu.here(seq)) && (!T.rx || qx.here(seq));
         if (__all_sync(0xffffffffu, ready)) break;
-        if (!(ok = pt.more(err))) break;
+        if (!(ok = pt.more(C))) break;
         ask();
     }
     if (T.rx) mine[lane] = qx.val();
@@ -1118,7 +1124,6 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
     }
     // the slots of the two exchanges of an iteration (in a cluster WarpFace::to holds addresses)
     const u64 from1 = B.C.slots, from0 = from1 + (u64)B.C.nslots * 16, to1 = CL ? 0 : from1, to0 = to1 + (u64)B.C.nslots * 16;
-    int* const err = B.C.err;
     const V4<R> zero = mk4<R>(0, 0, 0, 0);
 #pragma unroll
     for (int j = 0; j < K; j++) xs[j * nwk] = ps[j * nwk] = qs[j * nwk] = zero;
@@ -1174,7 +1179,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
                 ++seq;   // w = g5Dw r
                 stencil_inner<R, K, CL>(T, r, u1, u2, m2, box0, to0, seq, w);
                 bar_sync_n(2, nwk);
-                note(B, stencil_faces<R, K, CL>(T, u1, u2, box0, from0, err, seq, w, [&]() {   // x += alpha p of the last iteration
+                note(B, stencil_faces<R, K, CL>(T, u1, u2, box0, from0, B.C, seq, w, [&]() {   // x += alpha p of the last iteration
 #pragma unroll
                     for (int j = 0; j < K; j++) xs[j * nwk] = axpy4<R, PK>(alpha, ps[j * nwk], xs[j * nwk]);
                 }));
@@ -1204,7 +1209,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
                 ++seq;   // w = g5Dw t
                 stencil_inner<R, K, CL>(T, t, u1, u2, m2, box1, to1, seq, w);
                 bar_sync_n(2, nwk);
-                note(B, stencil_faces<R, K, CL>(T, u1, u2, box1, from1, err, seq, w, [&]() {
+                note(B, stencil_faces<R, K, CL>(T, u1, u2, box1, from1, B.C, seq, w, [&]() {
                     if (mu2 == R(0))
 #pragma unroll
                         for (int j = 0; j < K; j++) ps[j * nwk] = axpy4<R, PK>(beta, ps[j * nwk], r[j]);
@@ -1227,7 +1232,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
                 stencil_inner<R, K, CL>(T, r, u1, u2, m2, box0, to0, seq, t);
                 bar_sync_n(2, nwk);
                 R g = 0, d = 0;
-                bool ok = stencil_faces<R, K, CL>(T, u1, u2, box0, from0, err, seq, t, [&]() {
+                bool ok = stencil_faces<R, K, CL>(T, u1, u2, box0, from0, B.C, seq, t, [&]() {
 #pragma unroll
                     for (int j = 0; j < K; j++) g += norm4<R, PK>(r[j]);
                 });
@@ -1237,7 +1242,7 @@ __device__ __forceinline__ unsigned res_worker(const ResP& P, ResBlock& B, char*
                 ++seq;   // w = g5Dw t
                 stencil_inner<R, K, CL>(T, t, u1, u2, m2, box1, to1, seq, w);
                 bar_sync_n(2, nwk);
-                ok &= stencil_faces<R, K, CL>(T, u1, u2, box1, from1, err, seq, w, []() {});
+                ok &= stencil_faces<R, K, CL>(T, u1, u2, box1, from1, B.C, seq, w, []() {});
                 note(B, ok);
                 if (adv) {   // p = r_old + beta p, x += alpha p
 #pragma unroll
@@ -1300,6 +1305,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_cg(const __grid
         B.C.nb = P.nb;
         B.C.rank = blockIdx.x - team * P.nb;
         B.C.nslots = P.nslots;
+        B.C.polls = P.polls;
         B.C.err = &P.ctl->err;
         if constexpr (CL) {
             B.C.psum = smem_u32(dyn + ResSm<R, K>::bytes((blockDim.x >> 5) - 1));
@@ -1339,7 +1345,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_cg(const __grid
         __syncthreads();
         next = P.nteams + (int)B.next;
     }
-    if (B.C.rank == 0 && threadIdx.x == 0 && ld_volatile_int(B.C.err) != 0)
+    if (B.C.rank == 0 && threadIdx.x == 0 && ld_volatile_int(&P.ctl->err) != 0)
         atomicCAS(&P.ctl->status, 0, QED2D_ERR_TIMEOUT);
     if constexpr (CL) cooperative_groups::this_cluster().sync();   // others may still write here
 }
@@ -1402,7 +1408,7 @@ static int res_launch_k(const ResP& P, const ResGeom& g, cudaStream_t stream) {
     QTRY(res_allow_smem(kern));
     if (CL) QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(P.nb * P.nteams);
+    cfg.gridDim = dim3(P.nb * P.nteams - g.missing);
     cfg.blockDim = dim3(32 * (g.nw + 1));
     cfg.dynamicSmemBytes = sm;
     cfg.stream = stream;

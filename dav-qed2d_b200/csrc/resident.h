@@ -31,6 +31,8 @@ struct ResOut {
 // Shape of a launch: blocks of a team, worker warps of a block, halo slots of a block's buffer.
 struct ResGeom {
     int K, cl, f64, nb, nw, nslots;
+    int missing = 0;      // self-test: blocks left out of the launch,
+    unsigned polls = 0;   // polls after which a wait gives up (0: the default)
 };
 ResGeom res_geom(const ResPlan& p);
 // one that runs both (of the same K, cl and f64): teams and blocks of the larger, parts of
@@ -44,6 +46,7 @@ inline ResGeom res_join(ResGeom a, const ResGeom& b) {
 
 // K = 0 where the state does not fit on chip
 ResPlan res_plan_single(int L1, int L2, int nb, bool f64);
+ResPlan res_plan_pair(int L1, int L2, bool f64);   // a grid of two blocks
 std::vector<ResPlan> res_plan_batch(const std::vector<std::pair<int, int>>& sizes, const std::vector<int>& n, int num_sms);
 int res_clusters(const ResGeom& g);
 ResRep res_rep(const ResPlan& p, int L1, int L2, long long off, double m2, int id);
@@ -83,7 +86,7 @@ struct ResMd {
     int m, ns, each;
 };
 bool res_gauge_fits(Ctx& c);
-int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s);
+int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s, const ResPlan& p, int missing = 0, unsigned polls = 0);
 size_t res_slot_bytes(const ResGeom& g, int nteams);
 // one launch: nteams teams of geom.nb blocks solve the nrep systems
 int res_launch(const ResArgs& a, const ResGeom& geom, int nteams, cudaStream_t stream);

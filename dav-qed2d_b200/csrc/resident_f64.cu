@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1)
         B.C.nb = P.nb;
         B.C.rank = blockIdx.x;
         B.C.nslots = P.nslots;
+        B.C.polls = P.polls;
         B.C.err = &P.ctl->err;
         B.C.slots = (u64)P.slots;
         B.C.psum = (u64)P.psum;
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1)
     if (threadIdx.x < 32) res_scalar<false, false, true>(P, B, 0, base0, base1, &M, &S);
     else if ((int)threadIdx.x < 32 * (M.nw + 1)) res_worker<double, K, false, true>(P, B, dyn, 0, rbuf);
     else res_shifts<K>(P, M, B, S, rbuf, sx);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && ld_volatile_int(B.C.err) != 0)
+    if (blockIdx.x == 0 && threadIdx.x == 0 && ld_volatile_int(&P.ctl->err) != 0)
         atomicCAS(&P.ctl->status, 0, QED2D_ERR_TIMEOUT);
 }
 

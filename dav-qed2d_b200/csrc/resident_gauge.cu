@@ -33,6 +33,7 @@ struct ResGaugeP {
     double first, u[5], c[5], last;
     int m, ns, each;
     ulonglong2* slots;
+    unsigned polls;
     DevCtl* ctl;
 };
 
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_gauge(const __g
         B.C.nb = P.nb;
         B.C.rank = blockIdx.x;
         B.C.nslots = P.nslots;
+        B.C.polls = P.polls;
         B.C.err = &P.ctl->err;
         B.C.slots = CL ? smem_u32(dyn + (size_t)nw * BOX * sizeof(double2)) : (u64)P.slots;
     }
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_gauge(const __g
                 if (rx) qx = ld_slot<CL>(px);
                 const bool ready = (!rd || tagged(qd, seq)) && (!ru || tagged(qu, seq)) && (!rx || tagged(qx, seq));
                 if (__all_sync(0xffffffffu, ready)) break;
-                if (!pt.more(B.C.err)) {
+                if (!pt.more(B.C)) {
                     ok = false;
                     break;
                 }
@@ -213,9 +215,10 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_gauge(const __g
         }
         if (P.each && i < P.ns - 1) kick(P.first);   // the next step's first kick: the same links
     }
+    alive = !__syncthreads_or(!ok || !alive);   // a block that gave up leaves its fields as they were
 #pragma unroll
     for (int j = 0; j < K; j++)
-        if (v_ok && j < h) {
+        if (alive && v_ok && j < h) {
             const long long g = g0 + (long long)j * L1;
             P.U[g] = u1[j];
             P.U[g + V] = u2[j];
@@ -233,13 +236,13 @@ static size_t gauge_smem(const ResPlan& p) {
 }
 
 template <int K, bool CL>
-static int gauge_launch(const ResGaugeP& P, const ResPlan& p, cudaStream_t stream, bool query, int* clusters) {
+static int gauge_launch(const ResGaugeP& P, const ResPlan& p, cudaStream_t stream, bool query, int* clusters, int missing) {
     const void* kern = (const void*)k_res_gauge<K, CL>;
     const size_t sm = gauge_smem(p);
     QTRY(res_allow_smem(kern));
     if (CL) QCHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.blocks());
+    cfg.gridDim = dim3(p.blocks() - missing);
     cfg.blockDim = dim3(32 * p.wx * p.wy);
     cfg.dynamicSmemBytes = sm;
     cfg.stream = stream;
@@ -265,14 +268,14 @@ static int gauge_launch(const ResGaugeP& P, const ResPlan& p, cudaStream_t strea
     return QED2D_OK;
 }
 
-static int gauge_dispatch(const ResGaugeP& P, const ResPlan& p, cudaStream_t s, bool query, int* n) {
+static int gauge_dispatch(const ResGaugeP& P, const ResPlan& p, cudaStream_t s, bool query, int* n, int missing = 0) {
     switch (p.K * 2 + p.cl) {
-        case 2: return gauge_launch<1, false>(P, p, s, query, n);
-        case 3: return gauge_launch<1, true>(P, p, s, query, n);
-        case 4: return gauge_launch<2, false>(P, p, s, query, n);
-        case 5: return gauge_launch<2, true>(P, p, s, query, n);
-        case 8: return gauge_launch<4, false>(P, p, s, query, n);
-        default: return gauge_launch<4, true>(P, p, s, query, n);
+        case 2: return gauge_launch<1, false>(P, p, s, query, n, missing);
+        case 3: return gauge_launch<1, true>(P, p, s, query, n, missing);
+        case 4: return gauge_launch<2, false>(P, p, s, query, n, missing);
+        case 5: return gauge_launch<2, true>(P, p, s, query, n, missing);
+        case 8: return gauge_launch<4, false>(P, p, s, query, n, missing);
+        default: return gauge_launch<4, true>(P, p, s, query, n, missing);
     }
 }
 
@@ -306,8 +309,7 @@ bool res_gauge_fits(Ctx& c) {
     return c.res_gauge.K > 0;
 }
 
-int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s) {
-    const ResPlan& p = c.res_gauge;
+int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s, const ResPlan& p, int missing, unsigned polls) {
     ResGaugeP P{};
     P.rep = res_rep(p, c.g.L1, c.g.L2, 0, 0.0, 0);
     P.nb = p.blocks();
@@ -324,6 +326,7 @@ int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s) {
         P.u[k] = s.u[k];
         P.c[k] = s.c[k];
     }
+    P.polls = polls ? polls : p.cl ? kWaitPolls<true> : kWaitPolls<false>;
     P.ctl = c.ctl;
     QCHECK(cudaMemsetAsync(&c.ctl->bar, 0, 2 * sizeof(unsigned long long) + sizeof(int), c.stream));
     if (!p.cl) {
@@ -332,7 +335,7 @@ int res_gauge_md(Ctx& c, double* mom, double2* U, const ResMd& s) {
         if (!P.slots) return QED2D_ERR_NO_MEMORY;
         QCHECK(cudaMemsetAsync(P.slots, 0, bytes, c.stream));
     }
-    return gauge_dispatch(P, p, c.stream, false, nullptr);
+    return gauge_dispatch(P, p, c.stream, false, nullptr, missing);
 }
 
 }  // namespace qed2d

@@ -177,6 +177,14 @@ int qed2d_ctx_graph_stats(const qed2d_ctx* ctx, int* on, int64_t* captures, int6
  * solver's barrier does when a block never arrives, and the call returns
  * QED2D_ERR_TIMEOUT; the context stays usable for the next call. */
 int qed2d_selftest_barrier_timeout(qed2d_ctx* ctx, int64_t polls);
+/* The same for the on-chip kernels' waits, which give up after some 40 s as the
+ * grid barriers do: what = QED2D_PREC_F64 or QED2D_PREC_MIXED, a solve with links
+ * and source U, or QED2D_GAUGE_MD, an integration of (U, mom), on a team of two
+ * blocks whose second is never launched, with waits of `polls` polls (1..2^22,
+ * rounded up to a multiple of 256).  Returns QED2D_ERR_TIMEOUT
+ * (QED2D_ERR_UNSUPPORTED where the lattice does not fit two blocks); blocks that
+ * give up leave U and mom as they were. */
+int qed2d_selftest_on_chip_timeout(qed2d_ctx* ctx, int what, int64_t polls, double* U, double* mom);
 /* iterations, final |r|^2/|b|^2 and (QED2D_PREC_MIXED) FP64 reliable updates of
  * the most recent solve on this context; any pointer may be NULL */
 int qed2d_last_solve(const qed2d_ctx* ctx, int64_t* iterations, double* rel_residual_sq,

@@ -255,3 +255,30 @@ def test_untuned_batches_take_the_fastest_form(sizes):
             continue
     note(f"{len(sizes)} x {sizes[0]}: {chosen}", [mine, others])
     assert mine <= 1.15 * min(others.values()), (chosen, mine, others)
+
+
+@pytest.mark.parametrize("what", ["f64", "mixed", "gauge"])
+def test_on_chip_wait_gives_up(what):
+    """A team of two blocks whose second is never launched: the waits for sums (solves) and
+    faces (integration) end after a few polls with a status that the host reads, links and
+    momenta stay as they were, and the same context then works as usual."""
+    import torch
+    import qed2d as q
+    from qed2d import _lib
+    L1, L2 = 64, 12
+    prm = q.LattParm((L1, L2), 4.0)
+    U, mom = to_dev(hot_links(L1, L2, 31)), torch.randn(2, L2, L1, dtype=torch.float64, device="cuda")
+    U0, mom0 = U.clone(), mom.clone()
+    code = _lib.GAUGE_MD if what == "gauge" else q._PRECS[what]
+    call = q.lib().qed2d_selftest_on_chip_timeout
+    for polls in (256, 4096):   # twice: the error does not stick to the context
+        assert call(q._c(prm), code, polls, q._cp(U, prm), q._rp(mom, prm)) == _lib.TIMEOUT
+        assert torch.equal(U, U0) and torch.equal(mom, mom0)
+    assert call(q._c(prm), code, 0, q._cp(U, prm), q._rp(mom, prm)) == _lib.BAD_ARG
+    if what == "gauge":
+        q.OMF4_(mom, U, 0.1, 1, prm, None)
+        assert q.on_chip(prm, "gauge") and not torch.equal(U, U0)
+    else:
+        q.set_schedule(prm, -1, what)
+        cg_once(q, prm, what)
+        assert q.on_chip(prm, what)
