@@ -128,7 +128,10 @@ def set_precision(p) -> None:
 def context(L1: int, L2: int, beta: float = 0.0):
     """The library context of an L1 x L2 lattice on the current device (cached)."""
     dev = torch.cuda.current_device()
-    h = _ctx.get((L1, L2, dev))
+    try:
+        h = _ctx.get((L1, L2, dev))
+    except TypeError:   # extents that int() takes but a dict does not (0-dimensional arrays)
+        h = None
     if h is None:
         key = (int(L1), int(L2), dev)
         h = _ctx.get(key)
@@ -143,8 +146,10 @@ def context(L1: int, L2: int, beta: float = 0.0):
 
 
 def _raw_stream(dev):
-    """The handle of torch's current stream (without building a Stream object, 0.9 us)."""
-    return torch._C._cuda_getCurrentRawStream(dev)
+    """The handle of torch's current stream; a torch without its internal getter builds a
+    Stream object for it (0.9 us)."""
+    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return get(dev) if get else torch.cuda.current_stream(dev).cuda_stream
 
 
 def _c(prm: LattParm):
