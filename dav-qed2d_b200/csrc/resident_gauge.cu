@@ -183,7 +183,9 @@ __global__ void __launch_bounds__(32 * (kResWarps + 1), 1) k_res_gauge(const __g
         if (on && lane < h) Fr = mine[K + lane] - vr;
         return true;
     };
-    // explicit fma: the carried links' momenta get the bits that their owners' get
+    // explicit fma: the carried links' momenta get the bits that their owners' get (and the
+    // compiler contracts the rest alike in every row: a test moves the field by some sites
+    // and wants the same bits moved)
     auto kick = [&](double e) {
 #pragma unroll
         for (int j = 0; j < K; j++) {

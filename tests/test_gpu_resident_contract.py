@@ -282,3 +282,23 @@ def test_on_chip_wait_gives_up(what):
         q.set_schedule(prm, -1, what)
         cg_once(q, prm, what)
         assert q.on_chip(prm, what)
+
+
+@pytest.mark.parametrize("L1,L2", [(64, 64), (100, 37), (128, 128), (350, 370)])
+def test_gauge_integration_is_translation_invariant(L1, L2):
+    """The on-chip integration carries copies of the links beyond a tile's upper and right
+    edges, which must get the bits of their owners, in whatever tile and row those lie.
+    Moving the field moves every site to another place in its tile: after 20 OMF4 steps
+    (100 link updates) the moved field gives the moved result, bit for bit."""
+    import torch
+    import qed2d
+    prm = qed2d.LattParm((L1, L2), 5.0)
+    U = to_dev(hot_links(L1, L2, 3))
+    mom = torch.from_numpy(np.random.default_rng(3).standard_normal((2, L2, L1))).cuda()
+    U1, m1 = U.clone(), mom.clone()
+    qed2d.OMF4_(m1, U1, 0.1, 20, prm, None)
+    assert qed2d.on_chip(prm, "gauge")
+    for shift in ((1, 0), (0, 1), (5, 3)):
+        U2, m2 = (torch.roll(t, shift, (1, 2)).contiguous() for t in (U, mom))
+        qed2d.OMF4_(m2, U2, 0.1, 20, prm, None)
+        assert torch.equal(torch.roll(U1, shift, (1, 2)), U2) and torch.equal(torch.roll(m1, shift, (1, 2)), m2)
