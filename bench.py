@@ -55,8 +55,8 @@ B_KRNL_FORCE = 64.0      # krnl_force!: links in 32 + frc1, frc2 out 16 + 16
 B_UPDT_FLD = 80.0        # updt_fld!: momenta in 16 + links in and out 32 + 32
 B_TR_DQWDU = 112.0       # tr_dQwdU: links 32 + X 32 + g5Dw X 32 in, force out 16
 B_PLAQ_FIELD = 40.0      # plaquette!: links in 32 + per-site plaquette out 8
-B_OMF4_STEP = 6 * 64.0 + 5 * 80.0   # one pure-gauge OMF4 step as the reference's kernels move it: 6 kicks
-                                    # (links 32 + momenta r/w 32), 5 link updates (the fused passes move 544)
+B_OMF4_STEP = 64.0 + 5 * 96.0   # one pure-gauge OMF4 step beyond the chip: a kick (links 32 + momenta r/w 32) and 5
+                                # passes of a link update and a kick (links and momenta in and out 64 + 32)
 # Roofline units of the headline kernel.  Algorithmic bytes per site of one CG
 # iteration on (g5Dw)^2: 256 B in FP32 (two applies at 48 B + ten vector passes
 # at 16 B), 512 B in FP64 -- an FP64 reliable update is counted as one FP64
@@ -72,6 +72,7 @@ U_DRAM_PER_SITE_ITER = 0.35
 U_L2_PER_SITE_ITER = 33.5
 U_L2_THROUGHPUT = 0.090   # lts__throughput.avg.pct_of_peak_sustained_elapsed of the same capture
 U_ISSUE = 0.456           # smsp__issue_active.avg.pct_of_peak_sustained_active
+U_INST_PER_SITE_ITER = 262 / 32   # warp instructions (smsp__inst_executed.sum of the same capture)
 ENS_NS, ENS_EPS = 10, 0.1   # replica ensemble: leapfrog ns=10, eps=0.1
 CPU_TRAJ = 2                # trajectories of the GPU arm's CPU-baseline sample
 
@@ -275,9 +276,13 @@ def run_configs(qed2d, torch, dev):
     for _ in range(10):
         qed2d.HMC_(U2, 0.1, 10, [], p2, None)   # pure-gauge thermalisation
     c2, sched = {}, {}
-    # untuned solves that fit keep their state on chip: one cluster (2, 6) or a grid (1, 5)
-    names = {1: "on chip, grid", 2: "on chip, one thread-block cluster"}
-    names.update({k + 4: v for k, v in list(names.items())})
+
+    def form(prm, what):   # the form of the last solve
+        s = qed2d.get_schedule(prm, what)
+        if qed2d.on_chip(prm, what):   # a grid (1, 5) or one cluster (2, 6)
+            return "on chip, one thread-block cluster" if s in (2, 6) else "on chip, grid"
+        return {0: "grid, last block publishes", 1: "grid, every block sums", 2: "one thread-block cluster"}.get(
+            s & 3 if what == "mixed" else s, "untuned")
     for prec in ("mixed", "f64", "plain"):
         qed2d.set_precision(prec)
         Uc = U2.clone()
@@ -285,7 +290,7 @@ def run_configs(qed2d, torch, dev):
         st()
         c2[prec] = timed(st, 10)
         if prec != "plain":
-            sched[prec] = names.get(qed2d.get_schedule(p2, prec), "untuned")
+            sched[prec] = form(p2, prec)
     qed2d.set_precision("f64")
     out["C2_nf2_64_leapfrog"] = {"unit": "traj/s", "mixed": c2["mixed"], "f64_fused": c2["f64"], "plain_f64": c2["plain"],
                                  "mixed_vs_plain": c2["mixed"] / c2["plain"], "trajectories": 10,
@@ -300,11 +305,12 @@ def run_configs(qed2d, torch, dev):
     st3 = lambda: qed2d.HMC_(U3, [0.1], 0.05, 20, [], MAXITER, TOL, p3, None, rp)
     st3()
     out["C3_rhmc_128_12_poles"] = {"value": timed(st3, 10), "unit": "traj/s", "solver": "FP64 multi-shift, one launch for all poles",
-                                   "solver_schedule": names.get(qed2d.get_schedule(p3, "multishift"), "untuned"),
+                                   "solver_schedule": form(p3, "multishift"),
                                    "solver_layout": {0: "32x8 tiles, one thread per site", 1: "32x8 tiles, two threads per site",
                                                      2: "32x4 tiles, four threads per site",
                                                      3: "32x4 tiles, two threads per site"}.get(
-                                       qed2d.get_multishift_layout(p3), "on chip, shifts in shared memory"),
+                                       qed2d.get_multishift_layout(p3),
+                                       "shifts in shared memory" if qed2d.on_chip(p3, "multishift") else "untuned"),
                                    "trajectories": 10}
     del U, U2, U3
     # C5
@@ -445,7 +451,9 @@ def run_ours(args):
                     "cg_iterations_per_traj_mean": sum(p[0] for p in per_rep) / (n_traj * len(sizes)),
                     "accepted": sum(p[1] for p in per_rep), "of": n_traj * len(sizes),
                     "timed": f"{n_traj} batched trajectories after 1 warm-up",
-                    "solver": "on chip: a team of blocks per replica, one launch per lattice size"}
+                    "solver": ("on chip: a team of blocks per replica, sizes with like teams in one launch" if eb.on_chip
+                               else {2: "one launch over all replicas, grid barriers", 3: "one thread-block cluster per replica",
+                                     6: "one thread-block cluster per replica, phase-A stencil on r"}.get(eb.schedule, "untuned"))}
         del eb, Ue
         torch.cuda.empty_cache()
 
@@ -477,11 +485,17 @@ def run_ours(args):
     traffic = V * sum(its) * U_DRAM_PER_SITE_ITER
     l2_bytes = V * sum(its) * U_L2_PER_SITE_ITER
     l2_peak = l2_copy_peak(torch, dev)
-    roofline = {"kernel": "k_res_cg", "bound": "issue and exchange latency (state on chip)",
-                "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                "dram_achieved": traffic / t_k / 1e9, "dram_frac": traffic / t_k / 1e9 / peak,
-                "fused_model_achieved": fused_k / t_k / 1e9,
+    # the state stays on chip, so the roof is what the SMs can issue: 4 warp instructions a cycle and SM
+    props = torch.cuda.get_device_properties(dev)
+    sm_max = (clk or {}).get("sm_max_mhz") or 1965
+    issued, issue_peak = V * sum(its) * U_INST_PER_SITE_ITER / t_k / 1e9, 4 * props.multi_processor_count * sm_max / 1e3
+    roofline = {"kernel": "k_res_cg" if batch.on_chip else f"batch schedule {batch.schedule}",
+                "bound": "issue and exchange latency (state on chip)", "achieved": issued, "peak": issue_peak,
+                "unit": "G warp instructions/s", "frac": issued / issue_peak,
+                "peak_kind": "4 a cycle and SM at the maximum SM clock",
+                "algorithmic": {"achieved": achieved, "unit": "GB/s", "copy_peak": peak, "copy_peak_kind": peak_kind,
+                                "fused_model_achieved": fused_k / t_k / 1e9},
+                "traffic": traffic, "dram_achieved": traffic / t_k / 1e9, "dram_frac": traffic / t_k / 1e9 / peak,
                 "l2": {"achieved": l2_bytes / t_k / 1e9, "unit": "GB/s", "frac": U_L2_THROUGHPUT,
                        "frac_kind": "ncu lts__throughput of this kernel, fraction of the L2 peak",
                        "probe_GBs": l2_peak,
@@ -489,8 +503,8 @@ def run_ours(args):
                                      "(torch kernels; below what the L2 sustains for this kernel's mix)"},
                 "launch_us": t_k * 1e6,
                 "issue_active": U_ISSUE,
-                "schedule": "on chip: a team of blocks per replica, links and FP32 vectors in registers and "
-                            "shared memory for the whole solve",
+                "schedule": ("on chip: a team of blocks per replica, links and FP32 vectors in registers and "
+                             "shared memory for the whole solve" if batch.on_chip else "not on chip"),
                 "note": f"one launch = one solve of all {B} replicas: per replica iterations {min(its)}-{max(its)} "
                         f"x {B_ITER_F32:.0f} B/site + reliable updates {min(upd)}-{max(upd)} x {B_ITER_F64:.0f} "
                         f"B/site (algorithmic); the state stays in registers and shared memory, so the "

@@ -294,8 +294,8 @@ __global__ void __launch_bounds__(TILE, FERM ? 4 : 6) k_mom_kick(double* __restr
 // has.  With tiles of 8 rows staged in shared memory by a loop over their links (index
 // divisions, wrapping and 64-bit addresses for each) it was bound by issue: 505 warp
 // instructions for 32 sites, 86 of them FP64, at 68% of the issue slots and 48% of the
-// DRAM rate.  Two OMF4 steps (10 passes and a kick) on a B200: 768^2 185 -> 125 us, 1024^2
-// 231 -> 200, 2048^2 1043 -> 731, 4096^2 3924 -> 2732 (about 6.3 TB/s); K = 1 at 4096^2
+// DRAM rate.  Two OMF4 steps (10 passes and two kicks) on a B200: 768^2 185 -> 125 us, 1024^2
+// 231 -> 200, 2048^2 1043 -> 731, 4096^2 3924 -> 2732 (18.3 GB at 6.7 TB/s); K = 1 at 4096^2
 // 2948, K = 4 (spills, idle halo warps) 3195.  Passes alternate between upward and
 // downward (`back`), so that the next one starts with what the last left in L2: 1024^2
 // 211 -> 200, 2048^2 755 -> 731, 4096^2 2770 -> 2732.
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(TILE, K == 1 ? 6 : 4)
         t1 -= t2 * nt1;
     }
     if (back) t2 = g.L2 / H - 1 - t2;
-    const int L1 = g.L1, V = L1 * g.L2;   // 2V < 2^31 is checked at context creation
+    const int L1 = g.L1, V = L1 * g.L2;   // V <= 2^30 is checked at context creation: 2V - 1 fits
     const int x0 = t1 * TX, y0 = t2 * H;
     const int xl = x0 == 0 ? L1 - 1 : x0 - 1, xr = x0 + TX == L1 ? 0 : x0 + TX;
     const int yb = y0 == 0 ? g.L2 - 1 : y0 - 1, ya = y0 + H == g.L2 ? 0 : y0 + H;
@@ -390,6 +390,7 @@ __global__ void __launch_bounds__(TILE, K == 1 ? 6 : 4)
     }
 }
 
+// y = a x + b z (complex scalars; z may alias y)
 __global__ void k_zaxpby(double2* y, double2 a, const double2* x, double2 b, const double2* z,
                          long long n) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
