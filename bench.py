@@ -64,15 +64,17 @@ B_OMF4_STEP = 64.0 + 5 * 96.0   # one pure-gauge OMF4 step beyond the chip: a ki
 # figure is reported beside.)
 B_ITER_F32 = 256.0
 B_ITER_F64 = 512.0
-# Measured traffic per site-iteration of k_res_cg (the on-chip mixed CG) at 4 x 512^2,
-# from one ncu capture of a launch of 4 solves of 362 iterations: DRAM read + write
-# (133 MB over 1,048,576 sites x 362: sources, links and solutions once per solve) and
-# L2 (12.70 GB, halos between blocks and their polls); both grow with the iterations
-U_DRAM_PER_SITE_ITER = 0.35
-U_L2_PER_SITE_ITER = 33.5
+# Measured traffic of k_res_cg (the on-chip mixed CG) at 4 x 512^2, from ncu captures of one
+# launch (4 solves of 240 to 243 iterations and 6 updates): DRAM read + write 131.8 MB over
+# 1,048,576 sites (sources, links and solutions, once per solve) and L2 9.66 GB; an earlier
+# capture of 362 iterations had 12.7 GB, so an iteration moves 24 B a site (halos between
+# blocks, sums and their polls) and an FP64 update 565 B
+U_DRAM_PER_SITE = 126.0
+U_L2_PER_SITE_ITER = 24.1
+U_L2_PER_SITE_UPDATE = 565.0
 U_L2_THROUGHPUT = 0.090   # lts__throughput.avg.pct_of_peak_sustained_elapsed of the same capture
-U_ISSUE = 0.456           # smsp__issue_active.avg.pct_of_peak_sustained_active
-U_INST_PER_SITE_ITER = 262 / 32   # warp instructions (smsp__inst_executed.sum of the same capture)
+U_ISSUE = 0.436           # smsp__issue_active.avg.pct_of_peak_sustained_active
+U_INST_PER_SITE_ITER = 265 / 32   # warp instructions, updates included (smsp__inst_executed.sum of the same capture)
 ENS_NS, ENS_EPS = 10, 0.1   # replica ensemble: leapfrog ns=10, eps=0.1
 CPU_TRAJ = 2                # trajectories of the GPU arm's CPU-baseline sample
 
@@ -482,8 +484,8 @@ def run_ours(args):
     bytes_k = V * sum(i * B_ITER_F32 + u * B_ITER_F64 for i, u in zip(its, upd))
     fused_k = V * sum(B_MIXED_SETUP + i * B_MIXED_ITER + u * B_MIXED_UPDATE for i, u in zip(its, upd))
     achieved = bytes_k / t_k / 1e9
-    traffic = V * sum(its) * U_DRAM_PER_SITE_ITER
-    l2_bytes = V * sum(its) * U_L2_PER_SITE_ITER
+    traffic = V * len(its) * U_DRAM_PER_SITE
+    l2_bytes = V * (sum(its) * U_L2_PER_SITE_ITER + sum(upd) * U_L2_PER_SITE_UPDATE)
     l2_peak = l2_copy_peak(torch, dev)
     # the state stays on chip, so the roof is what the SMs can issue: 4 warp instructions a cycle and SM
     props = torch.cuda.get_device_properties(dev)
@@ -509,8 +511,8 @@ def run_ours(args):
                         f"x {B_ITER_F32:.0f} B/site + reliable updates {min(upd)}-{max(upd)} x {B_ITER_F64:.0f} "
                         f"B/site (algorithmic); the state stays in registers and shared memory, so the "
                         f"algorithmic rate exceeds the DRAM copy bandwidth; traffic = ncu DRAM bytes per "
-                        f"site-iteration x the solve's site-iterations (dram_achieved = traffic / time); l2 = "
-                        f"ncu L2 bytes per site-iteration x site-iterations (halos, sums and their polls); the "
+                        f"site of a solve x sites (dram_achieved = traffic / time); l2 = ncu L2 bytes per "
+                        f"site-iteration (halos, sums and their polls) and per update; the "
                         f"kernel waits for exchanges between blocks and issues in {U_ISSUE:.0%} of its cycles"}
 
     # --- single-chain baselines on the same field and draws as replica 0's first
