@@ -1266,9 +1266,8 @@ static int tune_cg(Ctx& c, const CGP& P, int slot) {
 // The solve with its whole state on chip (resident.cuh): the library's choice
 // wherever the state fits (mixed: up to about 530^2 on 148 SMs, FP64: 370^2), a rule
 // on the size without timing.  Per iteration against the fastest of the other forms,
-// B200: mixed 64^2 4.85 -> 1.95 us, 128^2 5.95 -> 2.7, 256^2 7.1 -> 3.5, 512^2 12.3 ->
-// 4.3; FP64 64^2 5.13 -> 2.2, 128^2 6.4 -> 3.1, 256^2
-// 8.05 -> 4.05, 350x370 11.1 -> 6.8.
+// B200: mixed 64^2 4.85 -> 1.95 us, 128^2 5.95 -> 2.8, 256^2 7.1 -> 3.5, 512^2 12.3 ->
+// 4.3; FP64 64^2 5.13 -> 2.2, 128^2 6.4 -> 3.0, 256^2 8.05 -> 4.0, 350x370 11.1 -> 6.8.
 static int cg_resident(Ctx& c, const SolveArgs& a, int slot, const ResPlan& p, int missing = 0, unsigned polls = 0) {
     ResArgs r;
     r.rep0 = res_rep(p, c.g.L1, c.g.L2, 0, 2.0 + a.am0, 0);

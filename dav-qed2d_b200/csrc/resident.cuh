@@ -36,7 +36,7 @@
 //   w = g5Dw t + mu^2 r halo of t; the sum of both meanwhile, and p, x of the last iteration
 //   beta = |r|^2 / |r_old|^2,  alpha = |r|^2 / (<r, A r> - beta |r|^2 / alpha_old)
 //   q = w + beta q (= A p),  r -= alpha q;  later p = r_old + beta p, x += alpha p
-// 128^2 takes 3.1 us an iteration instead of 4.4.  The difference in alpha's denominator
+// 128^2 takes 3.0 us an iteration instead of 4.4.  The difference in alpha's denominator
 // (= <p, A p>) multiplies the relative error of the last one by
 // beta alpha / alpha_old = (what is subtracted) / (what is left).  Where that exceeds one,
 // errors would grow from iteration to iteration, and the iteration is made directly:
@@ -54,8 +54,8 @@
 // issue.  A sum over a grid takes 1.15 us from the last block's contribution until it is
 // seen, plus 0.25 us of skew between the blocks, 0.2 us for the block's own sum and 0.25
 // us for the recurrences, whatever the split; in a cluster about half of that, which the
-// stencil's own chain (0.8 us) hides.  us an iteration, mixed: 64^2 1.95, 128^2 2.7, 256^2
-// 3.5, 512^2 4.3; FP64: 64^2 2.2, 128^2 3.1, 256^2 4.05, 350x370 6.8.
+// stencil's own chain (0.8 us) hides.  us an iteration, mixed: 64^2 1.95, 128^2 2.8, 256^2
+// 3.5, 512^2 4.3; FP64: 64^2 2.2, 128^2 3.0, 256^2 4.0, 350x370 6.8.
 #pragma once
 
 #include <cooperative_groups.h>
