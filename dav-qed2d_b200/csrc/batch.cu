@@ -1345,8 +1345,9 @@ void res_choose(qed2d_batch* h) {
 
 // First solve of a batch whose state fits on chip, once the other forms are tuned: times
 // `other` (the fastest of them) against the on-chip form on the caller's operator and
-// sources, capped at kRaceIters iterations, into the tuner's scratch outputs, and keeps
-// the faster; the control block is saved and restored.  On chip wins where few rounds of
+// sources, capped at kRaceIters iterations (whatever the caller's cap: a capped first solve
+// would time little but its setup), into the tuner's scratch outputs, and keeps the
+// faster; the control block is saved and restored.  On chip wins where few rounds of
 // teams hold the batch (per iteration: 37 x 64^2 7.9 -> 3.9 us, 5 x 256^2 12.2 -> 8.6, 4 x
 // 512^2 23.9 -> 18.5), and not where splits waste blocks while the other forms' working set
 // stays in L2 (64 x 128^2 21.8 -> 26.6, 16 x 256^2 23.4 -> 25.3, 8 x 384^2 25.8 -> 30.6).
@@ -1354,13 +1355,12 @@ void res_choose(qed2d_batch* h) {
 constexpr int kRaceIters = 100;
 
 template <class Other>
-int race_on_chip(qed2d_batch* h, const double2* U, const double2* b, int maxiter, double eps, Other other) {
+int race_on_chip(qed2d_batch* h, const double2* U, const double2* b, double eps, Other other) {
     DevCtl saved;
     QCHECK(cudaMemcpyAsync(&saved, h->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
     QCHECK(cudaStreamSynchronize(h->stream));
     double2 *x = h->field("tune_x"), *g5x = h->field("tune_g5x");
     if (!x || !g5x) return QED2D_ERR_NO_MEMORY;
-    const int iters = std::min(maxiter, kRaceIters);
     cudaEvent_t e0, e1;
     QCHECK(cudaEventCreate(&e0));
     QCHECK(cudaEventCreate(&e1));
@@ -1369,7 +1369,7 @@ int race_on_chip(qed2d_batch* h, const double2* U, const double2* b, int maxiter
     for (int rep = 0; rep < 3; rep++)
         for (int c = 0; c < 2 && st == QED2D_OK; c++) {
             cudaEventRecord(e0, h->stream);
-            st = c ? other(x, g5x, iters) : res_enqueue(h, U, b, x, g5x, iters, eps);
+            st = c ? other(x, g5x) : res_enqueue(h, U, b, x, g5x, kRaceIters, eps);
             cudaEventRecord(e1, h->stream);
             if (cudaEventSynchronize(e1) != cudaSuccess) st = cuda_status(cudaGetLastError(), "schedule tuning");
             float ms = 0.f;
@@ -1496,11 +1496,11 @@ int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* 
         };
         if (h->usched < 0 || h->utile < 0) QTRY(tune_uniform(h, Q, maxiter, launch));
         if (race) {
-            QTRY(race_on_chip(h, U, b, maxiter, eps, [&](double2* tx, double2* tg, int iters) -> int {
+            QTRY(race_on_chip(h, U, b, eps, [&](double2* tx, double2* tg) -> int {
                 UCGP T = Q;
                 T.x = tx;
                 T.t64 = tg;
-                T.maxiter = iters;
+                T.maxiter = kRaceIters;
                 return launch(h->usched, h->utile, T);
             }));
             if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
@@ -1546,12 +1546,12 @@ int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* 
         };
         if (h->rsched < 0) QTRY(tune_ragged(h, P, C, maxiter, launch));
         if (race) {
-            QTRY(race_on_chip(h, U, b, maxiter, eps, [&](double2* tx, double2* tg, int iters) -> int {
+            QTRY(race_on_chip(h, U, b, eps, [&](double2* tx, double2* tg) -> int {
                 RCGP TP = P;
                 CCGP TC = C;
                 TP.x = TC.x = tx;
                 TP.t64 = TC.t64 = tg;
-                TP.maxiter = TC.maxiter = iters;
+                TP.maxiter = TC.maxiter = kRaceIters;
                 return launch(h->rsched, TP, TC, h->rcs);
             }));
             if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
