@@ -86,9 +86,16 @@ ResPlan res_plan_pair(int L1, int L2, bool f64) {
     return none;
 }
 
-// A multishift solve with n shifts: the split over a grid of blocks with the least
-// time, where the shifts' vectors fit and their updates (about 36 cycles a row and
-// shift, all in shared memory) hide behind the iteration or bound it.
+// A multishift solve with n shifts: the split with the least time, where the shifts'
+// vectors fit and their updates hide behind the iteration or bound it.  Cycles an iteration
+// measured on a B200 over 90 splits of lattices from 8^2 to 64^2, 2 to 12 shifts, and 128^2
+// with 24: the base system as in res_cost, but 1400 more in a single block, whose sums no
+// longer are cheap when the shift warps join them; shifts, K = 1: 3650 and 355 for each item
+// (row and shift) of a shift warp, and no less than 106 for each of the block's (12^2 in one
+// block, 3 shift warps: 4 shifts 7850, 6 shifts 10700; 128^2 over 128: 24 shifts 9800); K = 2:
+// 1650 for each item of a warp (7 items: 11200 to 14500).  With 36 cycles an item and no
+// penalty 16^2 with 4 shifts ran in one block in 5.8 us an iteration; spread over four
+// 2.95, the grid kernel 5.0.
 int res_plan_ms(int L1, int L2, int nb, int n, int device, ResPlan* best) {
     size_t limit = 0;
     QTRY(res_ms_limit(device, &limit));
@@ -99,8 +106,9 @@ int res_plan_ms(int L1, int L2, int nb, int n, int device, ResPlan* best) {
             for (int by = 1; by <= std::min(nty, nb / bx); by++) {
                 ResPlan p{K, 0, 1, bx, by, ceil_div(ntx, bx), ceil_div(nty, by), ntx, nty, 0.0};
                 if (p.wx * p.wy > kResWarps || !res_ms_fits(p, n, limit)) continue;
-                const double shifts = 36.0 * p.wx * p.wy * K * (n - 1) / 1920;
-                p.cost = std::max(res_cost(K, p.wx * p.wy, bx, by, false, 1, true), shifts);
+                const int nw = p.wx * p.wy, items = nw * K * (n - 1), per = ceil_div(items, std::min(items, kResWarps - nw));
+                const double shifts = K == 1 ? std::max(3650 + 355 * per, 106 * items) : 1650 * per;
+                p.cost = std::max(res_cost(K, nw, bx, by, false, 1, true) + (bx * by == 1 ? 1400 : 0) / 1920.0, shifts / 1920);
                 if (!best->K || p.cost < best->cost) *best = p;
             }
     }

@@ -316,3 +316,37 @@ def test_capped_first_solve_chooses_like_any_other():
             b.cg(b.field(), U, src, 0.2, cap, 1e-24)
         b.cg(b.field(), U, src, 0.2, 20000, 1e-24)
         assert b.on_chip   # 2.5 us an iteration against 6.2
+
+
+@pytest.mark.parametrize("L1,L2,n", [(16, 16, 4), (20, 12, 6), (64, 64, 4), (128, 128, 12)])
+def test_untuned_multishift_is_no_slower_than_the_set_schedules(L1, L2, n):
+    """The multishift solve that the library chooses takes no longer than each schedule that can
+    be set (the best of 20 solves each; 5% for noise).  16^2 with 4 shifts in a single block took
+    15% longer than the cluster schedule, 20 x 12 with 6 shifts 7%."""
+    import time
+    import torch
+    import qed2d as q
+    prm = q.LattParm((L1, L2), 4.0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    U = torch.polar(torch.ones(2, L2, L1, dtype=torch.float64, device="cuda"),
+                    0.45 * torch.randn(2, L2, L1, dtype=torch.float64, device="cuda", generator=g))
+    src = torch.randn(2, L2, L1, dtype=torch.complex128, device="cuda", generator=g)
+    xs, mus = [q.cfield(L1, L2) for _ in range(n)], [0.05 * 1.4 ** i for i in range(n)]
+    took = {}
+    try:
+        for s in (-1, 0, 1, 2):
+            try:
+                q.set_schedule(prm, s, "multishift")
+                ts = []
+                for _ in range(21):
+                    torch.cuda.synchronize()
+                    t = time.perf_counter()
+                    q.multishift_CG(xs, U, src, 0.1, mus, 20000, 1e-24, prm)
+                    ts.append(time.perf_counter() - t)
+                took[s] = min(ts[1:])
+            except q.Qed2dError:   # a cluster schedule that does not fit
+                continue
+    finally:
+        q.set_schedule(prm, -1, "multishift")
+    note(f"multishift {L1}x{L2}, {n} shifts", took)
+    assert all(took[-1] <= 1.05 * t for t in took.values()), took
