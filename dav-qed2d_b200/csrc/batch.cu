@@ -1345,16 +1345,19 @@ void res_choose(qed2d_batch* h) {
 
 // First solve of a batch whose state fits on chip, once the other forms are tuned: times
 // `other` (the fastest of them) against the on-chip form on the caller's operator and
-// sources, capped at kRaceIters iterations (whatever the caller's cap: a capped first solve
-// would time little but its setup), into the tuner's scratch outputs, and keeps the
-// faster; the control block is saved and restored.  On chip wins where few rounds of
-// teams hold the batch (per iteration: 37 x 64^2 7.9 -> 3.9 us, 5 x 256^2 12.2 -> 8.6, 4 x
-// 512^2 23.9 -> 18.5), and not where splits waste blocks while the other forms' working set
-// stays in L2 (64 x 128^2 21.8 -> 26.6, 16 x 256^2 23.4 -> 25.3, 8 x 384^2 25.8 -> 30.6).
+// sources into the tuner's scratch outputs, and keeps the faster; the control block is
+// saved and restored.  On chip wins where few rounds of teams hold the batch (per iteration:
+// 37 x 64^2 7.9 -> 3.9 us, 5 x 256^2 12.2 -> 8.6, 4 x 512^2 23.9 -> 18.5), and not where splits
+// waste blocks while the other forms' working set stays in L2 (64 x 128^2 21.8 -> 26.6, 16 x
+// 256^2 23.4 -> 25.3, 8 x 384^2 25.8 -> 30.6).  The solves are the caller's, to convergence but
+// for no more than kRaceIters iterations (whatever the caller's cap: a capped first solve
+// would time little but its setup): replicas of an uneven batch need different numbers of
+// iterations, so which form wins shows over whole solves (20 lattices of 24..256 sites a
+// side: 100 iterations for all took the on-chip form, 2.86 ms a solve against 2.76).
 // QED2D_TUNE=0: on chip wherever it fits.
-constexpr int kRaceIters = 100;
+constexpr int kRaceIters = 400, kRaceWarmUp = 10;
 
-template <class Other>
+template <class Other>   // other(x, g5x, maxiter)
 int race_on_chip(qed2d_batch* h, const double2* U, const double2* b, double eps, Other other) {
     DevCtl saved;
     QCHECK(cudaMemcpyAsync(&saved, h->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
@@ -1364,23 +1367,27 @@ int race_on_chip(qed2d_batch* h, const double2* U, const double2* b, double eps,
     cudaEvent_t e0, e1;
     QCHECK(cudaEventCreate(&e0));
     QCHECK(cudaEventCreate(&e1));
-    float best[2] = {1e30f, 1e30f};
     int st = QED2D_OK;
-    for (int rep = 0; rep < 3; rep++)
-        for (int c = 0; c < 2 && st == QED2D_OK; c++) {
-            cudaEventRecord(e0, h->stream);
-            st = c ? other(x, g5x) : res_enqueue(h, U, b, x, g5x, kRaceIters, eps);
-            cudaEventRecord(e1, h->stream);
-            if (cudaEventSynchronize(e1) != cudaSuccess) st = cuda_status(cudaGetLastError(), "schedule tuning");
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (rep > 0) best[c] = std::min(best[c], ms);   // the first round warms up
-        }
+    auto timed = [&](int c, int maxiter) -> float {   // ms of form c (0: on chip)
+        float ms = 1e30f;
+        if (st != QED2D_OK) return ms;
+        cudaEventRecord(e0, h->stream);
+        st = c ? other(x, g5x, maxiter) : res_enqueue(h, U, b, x, g5x, maxiter, eps);
+        cudaEventRecord(e1, h->stream);
+        if (cudaEventSynchronize(e1) != cudaSuccess) st = cuda_status(cudaGetLastError(), "schedule tuning");
+        cudaEventElapsedTime(&ms, e0, e1);
+        return ms;
+    };
+    float t[2];
+    for (int c = 0; c < 2; c++) timed(c, kRaceWarmUp);
+    for (int c = 0; c < 2; c++) t[c] = timed(c, kRaceIters);
+    const int slower = t[0] > t[1] ? 0 : 1;   // once more, should something else have delayed it
+    t[slower] = std::min(t[slower], timed(slower, kRaceIters));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     QCHECK(cudaMemcpyAsync(h->ctl, &saved, sizeof(DevCtl), cudaMemcpyHostToDevice, h->stream));
     QCHECK(cudaStreamSynchronize(h->stream));
-    if (st == QED2D_OK && best[0] <= best[1]) res_choose(h);
+    if (st == QED2D_OK && t[0] <= t[1]) res_choose(h);
     return st;
 }
 
@@ -1496,11 +1503,11 @@ int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* 
         };
         if (h->usched < 0 || h->utile < 0) QTRY(tune_uniform(h, Q, maxiter, launch));
         if (race) {
-            QTRY(race_on_chip(h, U, b, eps, [&](double2* tx, double2* tg) -> int {
+            QTRY(race_on_chip(h, U, b, eps, [&](double2* tx, double2* tg, int cap) -> int {
                 UCGP T = Q;
                 T.x = tx;
                 T.t64 = tg;
-                T.maxiter = kRaceIters;
+                T.maxiter = cap;
                 return launch(h->usched, h->utile, T);
             }));
             if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
@@ -1546,12 +1553,12 @@ int r_solve(qed2d_batch* h, const double2* U, const float4* U32, const double2* 
         };
         if (h->rsched < 0) QTRY(tune_ragged(h, P, C, maxiter, launch));
         if (race) {
-            QTRY(race_on_chip(h, U, b, eps, [&](double2* tx, double2* tg) -> int {
+            QTRY(race_on_chip(h, U, b, eps, [&](double2* tx, double2* tg, int cap) -> int {
                 RCGP TP = P;
                 CCGP TC = C;
                 TP.x = TC.x = tx;
                 TP.t64 = TC.t64 = tg;
-                TP.maxiter = TC.maxiter = kRaceIters;
+                TP.maxiter = TC.maxiter = cap;
                 return launch(h->rsched, TP, TC, h->rcs);
             }));
             if (h->res_on) return res_solve_batch(h, U, b, x, g5x, maxiter, eps);
