@@ -270,38 +270,34 @@ static int md_kick_rhmc(Ctx& c, double* mom, const double2* U, double2* X, const
 // after OMF4 trajectories), not bit for bit.  Lattices of whole 32 x 8 tiles
 // (kernel requirement) without an FP32 link copy to refresh, beyond what the on-chip
 // integration holds.  Two OMF4 steps against the separate kernels: 768^2 185 -> 125 us,
-// 1024^2 231 -> 200, 1440^2 538 -> 379.
+// 1024^2 231 -> 200, 1440^2 538 -> 379.  Passes change buffers, so of an odd number the
+// first is made by the separate kernels in place (144 B/site) instead of copying the
+// result back (96 + 96): one step at 1024 x 1032 took 153 us with copies, 139 separately.
 struct GaugePingPong {
     Ctx& c;
     double2* U[2];
     double* mom[2];
     int cur = 0;
-    bool on = false;
-    GaugePingPong(Ctx& c_, double2* U0, double* m0, const MDState& s) : c(c_) {
+    bool on = false, in_place;   // fused passes; the next one by the separate kernels
+    GaugePingPong(Ctx& c_, double2* U0, double* m0, const MDState& s, long long passes) : c(c_), in_place(passes % 2) {
         U[0] = U0;
         mom[0] = m0;
         U[1] = nullptr;
         mom[1] = nullptr;
-        if (s.U32 || !updt_kick_fits(c)) return;
+        if (s.U32 || passes < 2 || !updt_kick_fits(c)) return;
         U[1] = c.spinor("md_u_alt");
         mom[1] = c.real2("md_mom_alt");
         on = U[1] && mom[1];
     }
     int kick(double eps) { return md_kick_gauge(c, mom[cur], U[cur], eps); }
     int links_then_kick(double eu, double ek, MDState& s) {
-        if (!on) {
+        if (!on || in_place) {
+            in_place = false;
             QTRY(md_links(c, U[cur], mom[cur], eu, s));
             return md_kick_gauge(c, mom[cur], U[cur], ek);
         }
         QTRY(launch_updt_kick(c, U[cur ^ 1], U[cur], mom[cur ^ 1], mom[cur], eu, ek, cur != 0));
         cur ^= 1;
-        return QED2D_OK;
-    }
-    int finish() {   // the result into the caller's arrays
-        if (cur == 0) return QED2D_OK;
-        QTRY(launch_copy(c, U[0], U[1], field_bytes(c)));
-        QTRY(launch_copy(c, mom[0], mom[1], sizeof(double) * 2 * (size_t)c.g.V));
-        cur = 0;
         return QED2D_OK;
     }
 };
@@ -318,22 +314,21 @@ static int md_omf4_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MD
         }
         return res_gauge_md(c, mom, U, md, c.res_gauge);
     }
-    GaugePingPong pp(c, U, mom, s);
+    GaugePingPong pp(c, U, mom, s, 5LL * ns);
     for (int i = 0; i < ns; i++) {
         QTRY(pp.kick(cm[0] * eps));
         for (int k = 0; k < 5; k++) QTRY(pp.links_then_kick(eps * cu[k], cm[k + 1] * eps, s));
     }
-    return pp.finish();
+    return QED2D_OK;
 }
 
 static int md_leapfrog_gauge(Ctx& c, double* mom, double2* U, double eps, int ns, MDState& s) {
     if ((c.on_chip[3] = ns > 0 && !s.U32 && res_gauge_fits(c)))
         return res_gauge_md(c, mom, U, ResMd{0.5 * eps, {eps}, {eps}, 0.5 * eps, 1, ns, 0}, c.res_gauge);
-    GaugePingPong pp(c, U, mom, s);
+    GaugePingPong pp(c, U, mom, s, ns < 1 ? 1 : ns);
     QTRY(pp.kick(0.5 * eps));
     for (int i = 0; i < ns - 1; i++) QTRY(pp.links_then_kick(eps, eps, s));
-    QTRY(pp.links_then_kick(eps, 0.5 * eps, s));
-    return pp.finish();
+    return pp.links_then_kick(eps, 0.5 * eps, s);
 }
 
 static int md_leapfrog_nf2(Ctx& c, double* mom, double2* U, double2* X, const double2* F, double2* g5DX,

@@ -383,3 +383,67 @@ def test_uneven_batch_choice_is_made_on_whole_solves():
         others[s] = best()
     note(f"20 uneven lattices: {chosen}", [mine, others])
     assert not chosen[0] or mine <= 1.02 * min(others.values()), (chosen, mine, others)
+
+
+@pytest.mark.parametrize("L1,L2", [(64, 4448), (1024, 1000)])
+@pytest.mark.parametrize("integrator,ns", [("omf4", 1), ("omf4", 3), ("leapfrog", 1), ("leapfrog", 2), ("leapfrog", 5)])
+def test_large_gauge_md_with_any_number_of_passes(L1, L2, integrator, ns):
+    """Pure-gauge integration beyond the chip: of an odd number of link updates the first is
+    made in place, so that the fused passes end in the caller's arrays.  Links of an accepted
+    trajectory and its energies against kicks and link updates made one by one (1e-13, as the
+    other gauge integration tests; relative 1e-13 of the energies, whose sums are of order V)."""
+    import torch
+    import qed2d
+    from qed2d import _lib
+    beta, eps = 5.0, 3e-4
+    prm = qed2d.LattParm((L1, L2), beta)
+    U = to_dev(hot_links(L1, L2, 31))
+    U1 = U.clone()
+    qed2d.seed(5)
+    info = qed2d.HMC_(U1, eps, ns, [], prm, None, counter=9,
+                      integrator=qed2d.OMF4() if integrator == "omf4" else qed2d.Leapfrog())
+    assert info.accepted and not qed2d.on_chip(prm, "gauge")
+    mom = qed2d.random_normal(2 * L1 * L2, 5, _lib.STREAM_MOMENTA, 9).reshape(2, L2, L1)
+    f1, f2 = torch.empty_like(mom), torch.empty_like(mom)
+    r1, r2, r3, r4 = 0.08398315262876693, 0.2539785108410595, 0.6822365335719091, -0.03230286765269967
+    r5, r6 = 0.5 - r1 - r3, 1.0 - 2.0 * (r2 + r4)
+    kicks, moves = ((r1, r3, r5, r5, r3, r1), (r2, r4, r6, r4, r2)) if integrator == "omf4" else ((0.5, 0.5), (1.0,))
+    for _ in range(ns):
+        for k, c in enumerate(kicks):
+            qed2d.krnl_force_(f1, f2, U, prm)
+            mom += c * eps * (f1 + f2)
+            if k < len(moves):
+                qed2d.updt_fld_(U, mom, eps * moves[k])
+    bound("gauge MD links, any number of passes", rel(to_host(U1), to_host(U)), 1e-13)
+    u1, u2 = U[0], U[1]
+    plaq = (u1 * torch.roll(u2, -1, 1) * torch.roll(u1, -1, 0).conj() * u2.conj()).real
+    hfin = float((mom ** 2).sum()) / 2 + beta * float((1 - plaq).sum())
+    bound("gauge MD final energy, any number of passes", abs(info.hfin - hfin) / hfin, 1e-13)
+
+
+def test_odd_steps_beyond_the_chip_copy_nothing_back():
+    """An OMF4 step on a lattice far beyond the caches, where bytes decide: one step moves 592
+    a site (a kick of 64, a separate update and kick of 144, four passes of 96), two move
+    1088: 0.544 of the time; with the result copied back (96 + 96 for the fifth pass) it
+    was 0.588.  The line is halfway."""
+    import torch
+    import qed2d
+    L = 4096
+    prm = qed2d.LattParm((L, L), 5.0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    U = torch.polar(torch.ones(2, L, L, dtype=torch.float64, device="cuda"),
+                    torch.randn(2, L, L, dtype=torch.float64, device="cuda", generator=g))
+    mom = torch.randn(2, L, L, dtype=torch.float64, device="cuda", generator=g)
+    took = {}
+    for ns in (1, 2):
+        ts = []
+        for _ in range(9):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            qed2d.OMF4_(mom, U, 1e-3, ns, prm, None)
+            b.record()
+            b.synchronize()
+            ts.append(a.elapsed_time(b))
+        took[ns] = min(ts[2:])
+    note("OMF4 steps at 4096^2, ms", took)
+    assert took[1] <= 0.566 * took[2], took
