@@ -1513,7 +1513,7 @@ static int multishift32_solve(Ctx& c, const double2* U, const double2* b, double
 }
 
 // The multishift solve with all its vectors on chip (resident_f64.cu): the library's
-// choice where they fit (about 190^2 with 12 shifts on 148 SMs).
+// choice where they fit (to 168^2 with 12 shifts on 148 SMs).
 static int multishift_resident(Ctx& c, const ResPlan& p, const double2* U, const double2* b, double2* const* x,
                                const double* mu2, int n, double am0, int maxiter, double eps) {
     ResShifts s{};

@@ -272,7 +272,8 @@ static int md_kick_rhmc(Ctx& c, double* mom, const double2* U, double2* X, const
 // integration holds.  Two OMF4 steps against the separate kernels: 768^2 185 -> 125 us,
 // 1024^2 231 -> 200, 1440^2 538 -> 379.  Passes change buffers, so of an odd number the
 // first is made by the separate kernels in place (144 B/site) instead of copying the
-// result back (96 + 96): one step at 1024 x 1032 took 153 us with copies, 139 separately.
+// result back (96 + 96): one step at 1024 x 1032 took 153 us with copies, 139 all
+// separately, 137 now.
 struct GaugePingPong {
     Ctx& c;
     double2* U[2];
